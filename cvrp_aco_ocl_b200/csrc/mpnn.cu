@@ -11,11 +11,28 @@
 //   u  = U + (1/k) sum_j g V_j;  h' = h + relu(u)
 // Head: z = relu(e W_h^T + b_h), logit s = z . w_o + b_o; weighted BCE loss.
 //
-// Edge kernels work on tiles of floor(128/k) whole nodes (their edges are one
-// contiguous row range), so the per-node sums need no atomics; the
-// contributions to a neighbour's row (dV, dC) are float atomics.  Weight
-// gradients accumulate in tensor memory across the tiles a persistent CTA
-// processes and are added to the gradient buffer once per CTA.
+// Common shape of the kernels: 256 threads work on a tile of up to 128 rows of
+// 64 channels.  Half-warp w (16 lanes, four channels a lane) owns rows 8w..8w+7,
+// so every global access is a whole 256-byte row.  BF16 operand tiles use the
+// 128-byte swizzle of umma.cuh, in which one staged copy serves as the
+// K-major operand of one product and the transposed (MN-major) operand of
+// another: no operand is staged twice.  The accumulator goes through a shared
+// FP32 tile (row stride 68) that takes the place of the operand tiles once the
+// product is done, which keeps a CTA at 44 KB and three CTAs on an SM.
+// Forward tiles hold whole nodes, so the per-node sums need no atomics.
+// Backward sums into dP are 16-byte vector reductions; weight gradients
+// accumulate in tensor memory over the tiles of a persistent CTA, bias
+// gradients in registers, and are added to the gradient buffer once per CTA.
+// Layer 0 makes its edge embedding from the edge feature on the fly (it is
+// never stored), and the backward of that layer sums the embedding's gradient
+// from its tiles.  The backward keeps the sign of q as one nibble a lane (16
+// bytes a row) in place of q itself.
+//
+// Measured on 32 graphs (9.2 k nodes, 185 k edges, k = 20), launch times under
+// ncu, before (one thread a row, an atomic a channel) and now, us: edge forward
+// 162 -> 55, head 1362 -> 36, edge backward 970 -> 97 (last layer 51), node
+// backward 82 -> 18, node GEMM 30 -> 7, embedding backward 419 -> none of its
+// own; the whole step 5.50 -> 0.545 ms.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -32,7 +49,10 @@ namespace {
 
 constexpr int H = 64;
 constexpr int FN = ACO_MPNN_NODE_FEATURES;
-constexpr int TPB = 128; // 4 warps: thread t owns TMEM lane t / tile row t
+constexpr int TPB = 256;
+constexpr int RT = 128; // rows of an edge tile
+constexpr int RPH = RT / (TPB / 16); // rows of a half-warp
+constexpr int MS = 68;  // row stride of the FP32 tile: 16-byte accesses by row and by TMEM lane are conflict-free
 
 // ---- packed parameter layout (same order as the oracle) --------------------
 struct ParamOffsets {
@@ -67,9 +87,10 @@ __host__ __device__ inline ParamOffsets param_offsets(int L)
 struct Workspace {
     int *status;
     float *loss;
-    float *h, *e, *P, *q, *u; // saved activations
-    float *s;                  // edge logits
-    float *dh, *de, *dP;       // backward
+    float *h, *e, *P, *u; // saved activations (e: layers 1..L, e0 is made from the edge feature)
+    uint8_t *qm;          // sign of q: bit i of byte 16 r + l is q > 0 at row r, channel 4 l + i
+    float *s;             // edge logits
+    float *dh, *de, *dP;  // backward
     size_t bytes;
 };
 
@@ -86,8 +107,8 @@ Workspace carve(void *base, int N, int k, int L)
         return o;
     };
     const size_t o_status = take(64), o_loss = take(64);
-    const size_t o_h = take(sizeof(float) * (L + 1) * N * H), o_e = take(sizeof(float) * (L + 1) * E * H);
-    const size_t o_P = take(sizeof(float) * L * N * 4 * H), o_q = take(sizeof(float) * L * E * H);
+    const size_t o_h = take(sizeof(float) * (L + 1) * N * H), o_e = take(sizeof(float) * L * E * H);
+    const size_t o_P = take(sizeof(float) * L * N * 4 * H), o_q = take(L * E * (H / 4));
     const size_t o_u = take(sizeof(float) * L * N * H), o_s = take(sizeof(float) * E);
     const size_t o_dh = take(sizeof(float) * N * H), o_de = take(sizeof(float) * E * H);
     const size_t o_dP = take(sizeof(float) * N * 4 * H);
@@ -99,7 +120,7 @@ Workspace carve(void *base, int N, int k, int L)
         w.h = (float *)(b + o_h);
         w.e = (float *)(b + o_e);
         w.P = (float *)(b + o_P);
-        w.q = (float *)(b + o_q);
+        w.qm = (uint8_t *)(b + o_q);
         w.u = (float *)(b + o_u);
         w.s = (float *)(b + o_s);
         w.dh = (float *)(b + o_dh);
@@ -112,51 +133,80 @@ Workspace carve(void *base, int N, int k, int L)
 // ---- device helpers ----------------------------------------------------------
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// rows [0, R) x K of a row-major fp32 source (row stride ld) -> K-major bf16 tile;
-// rows >= valid are zero.  K a multiple of 8.
-__device__ void stage_rows(uint8_t *tile, const float *src, size_t ld, int R, int K, int valid)
+__device__ __forceinline__ float4 ldg4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
+__device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+
+__device__ __forceinline__ void acc4(float4 &a, float4 b)
 {
-    const int q = K >> 2;
-    for (int idx = threadIdx.x; idx < R * q; idx += blockDim.x) {
-        const int r = idx / q, c = (idx - r * q) << 2;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < valid) v = *reinterpret_cast<const float4 *>(src + (size_t)r * ld + c);
-        const uint32_t lo = (uint32_t)umma::bf16_bits(v.x) | ((uint32_t)umma::bf16_bits(v.y) << 16);
-        const uint32_t hi = (uint32_t)umma::bf16_bits(v.z) | ((uint32_t)umma::bf16_bits(v.w) << 16);
-        *reinterpret_cast<uint2 *>(tile + umma::kmajor_offset(r, c, K)) = make_uint2(lo, hi);
+    a.x += b.x;
+    a.y += b.y;
+    a.z += b.z;
+    a.w += b.w;
+}
+
+// 16-byte vector reduction into global memory.
+__device__ __forceinline__ void red4(float *p, float4 v)
+{
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
+// The same into a caller's gradient, which need not be 16-byte aligned.
+__device__ __forceinline__ void add4(float *p, float4 v)
+{
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        red4(p, v);
+    } else {
+        atomicAdd(p, v.x);
+        atomicAdd(p + 1, v.y);
+        atomicAdd(p + 2, v.z);
+        atomicAdd(p + 3, v.w);
     }
 }
 
-// Transposed staging: tile(n, kk) = src[kk * ld + n] for n < Rn, kk < Kk;
-// source rows kk >= valid_k are zero.
-__device__ void stage_cols(uint8_t *tile, const float *src, size_t ld, int Rn, int Kk, int valid_k)
+// Channels 4l..4l+3 of row r into a 64-channel BF16 tile.
+__device__ __forceinline__ void put4(uint8_t *tile, int r, int l, float4 v)
 {
-    for (int idx = threadIdx.x; idx < Rn * Kk; idx += blockDim.x) {
-        const int kk = idx / Rn, n = idx - kk * Rn;
-        const float v = kk < valid_k ? src[(size_t)kk * ld + n] : 0.f;
-        *reinterpret_cast<uint16_t *>(tile + umma::kmajor_offset(n, kk, Kk)) = umma::bf16_bits(v);
+    const uint32_t lo = (uint32_t)umma::bf16_bits(v.x) | ((uint32_t)umma::bf16_bits(v.y) << 16);
+    const uint32_t hi = (uint32_t)umma::bf16_bits(v.z) | ((uint32_t)umma::bf16_bits(v.w) << 16);
+    *reinterpret_cast<uint2 *>(tile + umma::sw_offset(r, l >> 1) + ((l & 1) << 3)) = make_uint2(lo, hi);
+}
+
+// R rows of 64 channels (row stride ld) into a BF16 tile; rows >= valid are zero.
+__device__ __forceinline__ void stage_tile(uint8_t *tile, const float *src, size_t ld, int R, int valid)
+{
+    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
+#pragma unroll 4
+    for (int r = hw; r < R; r += TPB / 16) put4(tile, r, hl, r < valid ? ldg4(src + (size_t)r * ld + 4 * hl) : zero4());
+}
+
+// The 1024-byte aligned start of the dynamic shared memory (the swizzle's period).
+__device__ __forceinline__ uint8_t *tiles_base(uint8_t *sm) { return sm + ((1024u - (smem_u32(sm) & 1023u)) & 1023u); }
+
+// Products issued by thread 0 on 64-channel tiles (umma.cuh), K a multiple of 16:
+// D(128 x N) (+)= A B^T, each operand a tile read by rows (K = its 64 channels)
+// or transposed (K = K rows of it, M or N = its channels; a_lbo: byte
+// distance of the next 64 channels of a transposed A, 0: the same again).
+__device__ __forceinline__ void gemm_rows_cols(uint32_t d, const uint8_t *a, const uint8_t *b, bool b_transposed, int N)
+{
+    if (threadIdx.x == 0) {
+        const uint32_t id = umma::idesc_bf16(128, N, false, b_transposed);
+        const uint32_t aa = smem_u32(a), bb = smem_u32(b);
+        for (int s = 0; s < H / 16; s++)
+            umma::mma_bf16(d, umma::desc_k(aa, s), b_transposed ? umma::desc_mn(bb, s, 0) : umma::desc_k(bb, s), id, s > 0);
     }
 }
 
-// Zero rows [r0, R) of a K-major tile with K columns.
-__device__ void zero_rows(uint8_t *tile, int r0, int R, int K)
-{
-    const int q = K >> 2;
-    for (int idx = threadIdx.x; idx < (R - r0) * q; idx += blockDim.x) {
-        const int r = r0 + idx / q, c = (idx % q) << 2;
-        *reinterpret_cast<uint2 *>(tile + umma::kmajor_offset(r, c, K)) = make_uint2(0u, 0u);
-    }
-}
-
-// One GEMM D(128 x N) (+)= A(128 x K) B(N x K)^T issued by thread 0.
-__device__ __forceinline__ void gemm_issue(uint32_t tmem_d, const uint8_t *a, const uint8_t *b, int K, int N,
+__device__ __forceinline__ void gemm_outer(uint32_t d, const uint8_t *a, uint32_t a_lbo, const uint8_t *b, int K,
                                            bool accumulate)
 {
     if (threadIdx.x == 0) {
-        const uint32_t id = umma::idesc_bf16(128, N);
+        const uint32_t id = umma::idesc_bf16(128, H, true, true);
         const uint32_t aa = smem_u32(a), bb = smem_u32(b);
         for (int s = 0; s < (K >> 4); s++)
-            umma::mma_bf16(tmem_d, umma::smem_desc(aa, K, s), umma::smem_desc(bb, K, s), id, accumulate || s > 0);
+            umma::mma_bf16(d, umma::desc_mn(aa, s, a_lbo), umma::desc_mn(bb, s, 0), id, accumulate || s > 0);
     }
 }
 
@@ -206,155 +256,101 @@ __device__ void tmem_teardown(uint32_t base, uint32_t ncols)
     if (threadIdx.x < 32) umma::tmem_dealloc(base, ncols);
 }
 
-// Read this thread's 64 accumulator columns starting at column col0.
-__device__ __forceinline__ void tmem_row64(uint32_t base, int col0, float (&v)[64])
+// The 64 accumulator columns from col0 into the FP32 tile: warp w takes TMEM
+// lanes 32 (w mod 4) .. + 31 (tile rows) and columns 32 (w / 4) .. + 31.
+__device__ __forceinline__ void acc_to_tile(uint32_t base, int col0, float *ms)
 {
-    const int lane0 = (threadIdx.x >> 5) << 5;
+    const int w = threadIdx.x >> 5, lane0 = (w & 3) << 5, c0 = (w >> 2) << 5;
+    float v[32];
+    umma::tmem_ld32(umma::taddr(base, lane0, col0 + c0), v);
+    float *row = ms + (size_t)(lane0 + (threadIdx.x & 31)) * MS + c0;
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        float t[16];
-        umma::tmem_ld16(umma::taddr(base, lane0, col0 + 16 * c), t);
-#pragma unroll
-        for (int i = 0; i < 16; i++) v[16 * c + i] = t[i];
+    for (int i = 0; i < 32; i += 4) st4(row + i, make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+}
+
+// Per-thread sums of channels 4 hl .. + 3 added up over the CTA's half-warps and
+// into dst[0..63].  buf: 16 x 64 floats.
+__device__ __forceinline__ void add_channel_sums(float4 v, float *buf, float *dst)
+{
+    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
+    __syncthreads();
+    st4(buf + hw * H + 4 * hl, v);
+    __syncthreads();
+    if (threadIdx.x < H) {
+        float s = 0.f;
+        for (int i = 0; i < TPB / 16; i++) s += buf[i * H + threadIdx.x];
+        atomicAdd(dst + threadIdx.x, s);
     }
+}
+
+// Rows [0, 64) of the FP32 tile added into a 64 x 64 gradient.
+__device__ __forceinline__ void add_tile_rows(const float *ms, float *dst)
+{
+    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
+    for (int r = hw; r < H; r += TPB / 16) add4(dst + r * H + 4 * hl, ld4(ms + (size_t)r * MS + 4 * hl));
 }
 
 // ---- forward -----------------------------------------------------------------
-__global__ void embed_kernel(int N, int k, const float *prm, ParamOffsets o, const float *nf, const float *ef,
-                             float *h0, float *e0)
+__global__ void embed_nodes_kernel(int N, const float *prm, ParamOffsets o, const float *nf, float *h0)
 {
-    const size_t NH = (size_t)N * H, EH = (size_t)N * k * H;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < NH + EH;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        if (idx < NH) {
-            const size_t i = idx / H;
-            const int c = (int)(idx % H);
-            float acc = 0.f;
-            for (int f = 0; f < FN; f++) acc = __fmaf_rn(prm[o.W_n + c * FN + f], nf[i * FN + f], acc);
-            h0[idx] = acc + prm[o.b_n + c];
-        } else {
-            const size_t j = idx - NH, ei = j / H;
-            const int c = (int)(j % H);
-            e0[j] = __fmaf_rn(prm[o.W_e + c], ef[ei], prm[o.b_e + c]);
-        }
+    const size_t NH = (size_t)N * H;
+    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < NH; idx += (size_t)gridDim.x * blockDim.x) {
+        const size_t i = idx / H;
+        const int c = (int)(idx % H);
+        float acc = 0.f;
+        for (int f = 0; f < FN; f++) acc = __fmaf_rn(prm[o.W_n + c * FN + f], nf[i * FN + f], acc);
+        h0[idx] = acc + prm[o.b_n + c];
     }
 }
 
-// P = h W^T + b: tiles of 128 nodes, N = 256.
-struct NodeGemmSmem {
-    static constexpr size_t A = 0, B = A + 128 * H * 2, BYTES = B + 4 * H * H * 2;
+// The embedding of an edge feature on channels with weights w and biases b.
+__device__ __forceinline__ float4 embed4(float f, float4 w, float4 b)
+{
+    return make_float4(__fmaf_rn(w.x, f, b.x), __fmaf_rn(w.y, f, b.y), __fmaf_rn(w.z, f, b.z), __fmaf_rn(w.w, f, b.w));
+}
+
+// Shared memory of the edge kernels and the node GEMM: weights, then two
+// operand tiles whose place the FP32 tile takes after the product.
+struct TileSmem {
+    static constexpr size_t W = 0, A = W + H * H * 2, A2 = A + RT * H * 2, M = A, END = M + (size_t)RT * MS * 4,
+                            BYTES = END + 1024;
+    static_assert(A2 + RT * H * 2 <= END, "the FP32 tile covers both operand tiles");
 };
 
+// P = h W^T + b: a CTA takes 128 nodes x one 64-channel section of the 256
+// outputs (blockIdx.y), four times the CTAs of whole rows: 9.2 k nodes give 288.
 __global__ void __launch_bounds__(TPB) node_gemm_kernel(int N, const float *h, const float *W, const float *bias,
                                                         float *P, int *status)
 {
-    extern __shared__ __align__(1024) uint8_t sm[];
+    extern __shared__ uint8_t sm_raw[];
     __shared__ uint64_t bar;
     __shared__ uint32_t slot;
-    uint8_t *As = sm + NodeGemmSmem::A, *Bs = sm + NodeGemmSmem::B;
-    tmem_setup(&bar, &slot, 256);
-    const uint32_t tm = slot;
-    uint32_t phase = 0;
-    stage_rows(Bs, W, H, 4 * H, H, 4 * H);
-    const int tiles = (N + 127) / 128;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int r0 = t * 128, valid = min(128, N - r0);
-        stage_rows(As, h + (size_t)r0 * H, H, 128, H, valid);
-        operands_ready();
-        gemm_issue(tm, As, Bs, H, 4 * H, false);
-        if (!gemm_wait(&bar, phase, status)) break;
-        const int r = threadIdx.x, lane0 = (threadIdx.x >> 5) << 5;
-        for (int c = 0; c < 16; c++) {
-            float v[16];
-            umma::tmem_ld16(umma::taddr(tm, lane0, 16 * c), v);
-            if (r < valid) {
-                float *dst = P + (size_t)(r0 + r) * 4 * H + 16 * c;
-#pragma unroll
-                for (int i = 0; i < 16; i += 4)
-                    *reinterpret_cast<float4 *>(dst + i) =
-                        make_float4(v[i] + bias[16 * c + i], v[i + 1] + bias[16 * c + i + 1],
-                                    v[i + 2] + bias[16 * c + i + 2], v[i + 3] + bias[16 * c + i + 3]);
-            }
-        }
-        umma::fence_before();
-        __syncthreads();
-    }
-    tmem_teardown(tm, 256);
-}
-
-// Edge layer forward on tiles of npt = 128/k nodes.  M: the tile's 128 rows of
-// 64 fp32 values at row stride MS (the accumulator, then the gated messages),
-// padded so that the TMEM-lane-per-row writes fall in distinct banks.
-constexpr int MS = H + 1;
-struct EdgeFwdSmem {
-    static constexpr size_t A = 0, B = A + 128 * H * 2, M = B + H * H * 2, BYTES = M + 128 * MS * 4;
-};
-
-__global__ void __launch_bounds__(TPB) edge_fwd_kernel(int N, int k, const float *Wt, const float *a_bias,
-                                                       const float *e_in, const float *P, const float *h_in,
-                                                       const int *nbr, float *q_out, float *e_out, float *u_out,
-                                                       float *h_out, int *status)
-{
-    extern __shared__ __align__(1024) uint8_t sm[];
-    __shared__ uint64_t bar;
-    __shared__ uint32_t slot;
-    uint8_t *As = sm + EdgeFwdSmem::A, *Bs = sm + EdgeFwdSmem::B;
-    float *ms = reinterpret_cast<float *>(sm + EdgeFwdSmem::M);
+    uint8_t *sm = tiles_base(sm_raw);
+    uint8_t *Ws = sm + TileSmem::W, *As = sm + TileSmem::A;
+    float *ms = reinterpret_cast<float *>(sm + TileSmem::M);
     tmem_setup(&bar, &slot, 64);
     const uint32_t tm = slot;
     uint32_t phase = 0;
-    stage_rows(Bs, Wt, H, H, H, H); // A_l[o][i]: rows o, K = i
-    const int npt = 128 / k, tiles = (N + npt - 1) / npt;
+    const int sec = blockIdx.y * H, hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
+    stage_tile(Ws, W + (size_t)sec * H, H, H, H);
+    const float4 b4 = ldg4(bias + sec + 4 * hl);
+    const int tiles = (N + RT - 1) / RT;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int n0 = t * npt, nodes = min(npt, N - n0), rows = nodes * k;
-        const size_t e0 = (size_t)n0 * k;
-        stage_rows(As, e_in + e0 * H, H, 128, H, rows);
+        const int r0 = t * RT, valid = min(RT, N - r0);
+        stage_tile(As, h + (size_t)r0 * H, H, RT, valid);
         operands_ready();
-        gemm_issue(tm, As, Bs, H, H, false);
+        gemm_rows_cols(tm, As, Ws, false, H);
         if (!gemm_wait(&bar, phase, status)) break;
-        {   // the accumulator rows into shared memory (thread r holds TMEM lane r = row r)
-            const int r = threadIdx.x;
-            float d[64];
-            tmem_row64(tm, 0, d);
+        acc_to_tile(tm, 0, ms);
+        __syncthreads();
 #pragma unroll
-            for (int c = 0; c < H; c++) ms[r * MS + c] = d[c];
-        }
-        __syncthreads();
-        // epilogue by rows: a warp takes row r, lane l its channels 2l, 2l+1, so every
-        // global access of e, q and the P rows is one coalesced 256-byte row
-        {
-            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = 2 * lane;
-            const float2 ab = *reinterpret_cast<const float2 *>(a_bias + c);
-            for (int r = warp; r < rows; r += TPB / 32) {
-                const size_t ei = e0 + r;
-                const int src = n0 + r / k;
-                int j = nbr[ei];
-                if ((unsigned)j >= (unsigned)N) { // a neighbour id outside the batch: report, read node 0
-                    if (lane == 0) set_status(status, ACO_ERR_INVALID);
-                    j = 0;
-                }
-                const float *Pi = P + (size_t)src * 4 * H, *Pj = P + (size_t)j * 4 * H;
-                const float2 pi = *reinterpret_cast<const float2 *>(Pi + 2 * H + c);
-                const float2 pj = *reinterpret_cast<const float2 *>(Pj + 3 * H + c);
-                const float2 vj = *reinterpret_cast<const float2 *>(Pj + H + c);
-                const float2 ein = *reinterpret_cast<const float2 *>(e_in + ei * H + c);
-                float *mr = ms + r * MS + c;
-                const float q0 = mr[0] + ab.x + pi.x + pj.x, q1 = mr[1] + ab.y + pi.y + pj.y;
-                const float en0 = ein.x + fmaxf(q0, 0.f), en1 = ein.y + fmaxf(q1, 0.f);
-                *reinterpret_cast<float2 *>(q_out + ei * H + c) = make_float2(q0, q1);
-                *reinterpret_cast<float2 *>(e_out + ei * H + c) = make_float2(en0, en1);
-                mr[0] = sigmoidf_(en0) * vj.x; // the gated message replaces the accumulator
-                mr[1] = sigmoidf_(en1) * vj.y;
+        for (int s = 0; s < RPH; s++) {
+            const int r = hw * RPH + s;
+            if (r < valid) {
+                float4 v = ld4(ms + (size_t)r * MS + 4 * hl);
+                acc4(v, b4);
+                st4(P + (size_t)(r0 + r) * 4 * H + sec + 4 * hl, v);
             }
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < nodes * H; idx += blockDim.x) {
-            const int qn = idx / H, c = idx - qn * H, i = n0 + qn;
-            float acc = 0.f;
-            for (int j = 0; j < k; j++) acc += ms[(qn * k + j) * MS + c];
-            const float uv = P[(size_t)i * 4 * H + c] + acc / (float)k;
-            u_out[(size_t)i * H + c] = uv;
-            h_out[(size_t)i * H + c] = h_in[(size_t)i * H + c] + fmaxf(uv, 0.f);
         }
         umma::fence_before();
         __syncthreads();
@@ -362,316 +358,506 @@ __global__ void __launch_bounds__(TPB) edge_fwd_kernel(int N, int k, const float
     tmem_teardown(tm, 64);
 }
 
-// Head (tiles of 128 edges).  Inference: logits only.  Training: also the
-// weighted BCE loss, dL/ds, dz, de = dz W_h and the head's weight gradients.
-struct HeadSmem {
-    static constexpr size_t A = 0, B = A + 128 * H * 2, BT = B + H * H * 2, DZ = BT + H * H * 2,
-                            DZT = DZ + 128 * H * 2, ET = DZT + 128 * 128 * 2, RED = ET + H * 128 * 2,
-                            BYTES = RED + 4 * H * 4;
-};
-
-__global__ void __launch_bounds__(TPB) head_kernel(size_t E, const float *prm, ParamOffsets o, const float *eL,
-                                                   float *s_out, const float *labels, float pos_weight, float inv_E,
-                                                   float *de, float *grad, float *loss, int *status)
+// Edge layer forward on tiles of npt = 128/k nodes.  EMBED: layer 0, e_in is the
+// edge feature.  TRAIN: keep the sign of q and u for the backward.  What bounds
+// it: HBM (a row of e read, one written) once enough gathers are in flight;
+// the P rows come from L2.
+template <bool EMBED, bool TRAIN>
+__global__ void __launch_bounds__(TPB, 3) edge_fwd_kernel(int N, int k, const float *Wt, const float *a_bias,
+                                                          const float *e_in, const float *w_e, const float *b_e,
+                                                          const float *P, const float *h_in, const int *nbr,
+                                                          uint8_t *qm, float *e_out, float *u_out, float *h_out,
+                                                          int *status)
 {
-    extern __shared__ __align__(1024) uint8_t sm[];
+    extern __shared__ uint8_t sm_raw[];
     __shared__ uint64_t bar;
     __shared__ uint32_t slot;
-    const bool train = labels != nullptr;
-    uint8_t *As = sm + HeadSmem::A, *Bs = sm + HeadSmem::B, *BTs = sm + HeadSmem::BT, *DZs = sm + HeadSmem::DZ;
-    uint8_t *DZTs = sm + HeadSmem::DZT, *ETs = sm + HeadSmem::ET;
-    float *red = reinterpret_cast<float *>(sm + HeadSmem::RED); // b_h (64), w_o (64), b_o, loss
-    tmem_setup(&bar, &slot, 256);
-    const uint32_t tm = slot; // cols 0-63 z, 64-127 de, 128-191 dW_h
+    uint8_t *sm = tiles_base(sm_raw);
+    uint8_t *Ws = sm + TileSmem::W, *As = sm + TileSmem::A;
+    float *ms = reinterpret_cast<float *>(sm + TileSmem::M);
+    tmem_setup(&bar, &slot, 64);
+    const uint32_t tm = slot;
     uint32_t phase = 0;
-    const float *Wh = prm + o.W_h, *bh = prm + o.b_h, *wo = prm + o.w_o;
-    const float bo = prm[o.b_o];
-    stage_rows(Bs, Wh, H, H, H, H);      // W_h[o][i]
-    if (train) {
-        stage_cols(BTs, Wh, H, H, H, H); // tile(i, o) = W_h[o][i]
-        zero_rows(DZTs, H, 128, 128);    // rows o >= 64 of the transposed dz stay zero
-        for (int i = threadIdx.x; i < 4 * H; i += blockDim.x) red[i] = 0.f;
+    stage_tile(Ws, Wt, H, H, H); // A_l[o][i]: rows o, K = i
+    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15, c = 4 * hl;
+    const float4 ab = ldg4(a_bias + c);
+    float4 we = zero4(), be = zero4();
+    if (EMBED) {
+        we = ldg4(w_e + c);
+        be = ldg4(b_e + c);
     }
-    bool wg_started = false;
-    const size_t tiles = (E + 127) / 128;
-    for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const size_t e0 = t * 128;
-        const int rows = (int)min((size_t)128, E - e0);
-        stage_rows(As, eL + e0 * H, H, 128, H, rows);
-        if (train) stage_cols(ETs, eL + e0 * H, H, H, 128, rows); // tile(i, e) = eL[e][i]
-        operands_ready();
-        gemm_issue(tm, As, Bs, H, H, false);
-        if (!gemm_wait(&bar, phase, status)) break;
-        const int r = threadIdx.x;
-        float zp[64];
-        tmem_row64(tm, 0, zp);
-        float sv = bo;
-        for (int c = 0; c < H; c++) {
-            zp[c] += bh[c];
-            sv += fmaxf(zp[c], 0.f) * wo[c];
+    const int npt = RT / k, tiles = (N + npt - 1) / npt, q0 = hw * RPH / k, rem0 = hw * RPH - q0 * k;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int n0 = t * npt, nodes = min(npt, N - n0), rows = nodes * k;
+        const size_t e0 = (size_t)n0 * k;
+        float4 ein[RPH];
+        int jn[RPH];
+#pragma unroll
+        for (int s = 0; s < RPH; s++) {
+            const int r = hw * RPH + s;
+            ein[s] = zero4();
+            if (r < rows) ein[s] = EMBED ? embed4(__ldg(e_in + e0 + r), we, be) : ldg4(e_in + (e0 + r) * H + c);
         }
-        if (r < rows) s_out[e0 + r] = sv;
-        if (!train) {
+#pragma unroll
+        for (int s = 0; s < RPH; s++) {
+            const int r = hw * RPH + s;
+            put4(As, r, hl, ein[s]);
+            jn[s] = r < rows ? __ldg(nbr + e0 + r) : 0;
+        }
+        operands_ready();
+        gemm_rows_cols(tm, As, Ws, false, H);
+        if (!gemm_wait(&bar, phase, status)) break;
+        acc_to_tile(tm, 0, ms);
+        __syncthreads();
+        int src = n0 + q0, rem = rem0;
+#pragma unroll
+        for (int s = 0; s < RPH; s++) {
+            const int r = hw * RPH + s;
+            if (r < rows) {
+                const size_t ei = e0 + r;
+                int j = jn[s];
+                if ((unsigned)j >= (unsigned)N) { // a neighbour id outside the batch: report, read node 0
+                    if (hl == 0) set_status(status, ACO_ERR_INVALID);
+                    j = 0;
+                }
+                const float *Pj = P + (size_t)j * 4 * H + c;
+                const float4 pi = ldg4(P + (size_t)src * 4 * H + 2 * H + c), pj = ldg4(Pj + 3 * H), vj = ldg4(Pj + H);
+                float *mr = ms + (size_t)r * MS + c;
+                const float4 d = ld4(mr);
+                const float x0 = d.x + ab.x + pi.x + pj.x, x1 = d.y + ab.y + pi.y + pj.y;
+                const float x2 = d.z + ab.z + pi.z + pj.z, x3 = d.w + ab.w + pi.w + pj.w;
+                const float4 en = make_float4(ein[s].x + fmaxf(x0, 0.f), ein[s].y + fmaxf(x1, 0.f),
+                                              ein[s].z + fmaxf(x2, 0.f), ein[s].w + fmaxf(x3, 0.f));
+                st4(e_out + ei * H + c, en);
+                if (TRAIN)
+                    qm[ei * 16 + hl] = (uint8_t)((x0 > 0.f ? 1 : 0) | (x1 > 0.f ? 2 : 0) | (x2 > 0.f ? 4 : 0) |
+                                                 (x3 > 0.f ? 8 : 0));
+                // the gated message replaces the accumulator
+                st4(mr, make_float4(sigmoidf_(en.x) * vj.x, sigmoidf_(en.y) * vj.y, sigmoidf_(en.z) * vj.z,
+                                    sigmoidf_(en.w) * vj.w));
+            }
+            if (++rem == k) {
+                rem = 0;
+                src++;
+            }
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < nodes * H; idx += TPB) {
+            const int qn = idx / H, cc = idx - qn * H, i = n0 + qn;
+            float acc = 0.f;
+            for (int j = 0; j < k; j++) acc += ms[(size_t)(qn * k + j) * MS + cc];
+            const float uv = P[(size_t)i * 4 * H + cc] + acc / (float)k;
+            if (TRAIN) u_out[(size_t)i * H + cc] = uv;
+            h_out[(size_t)i * H + cc] = h_in[(size_t)i * H + cc] + fmaxf(uv, 0.f);
+        }
+        umma::fence_before();
+        __syncthreads();
+    }
+    tmem_teardown(tm, 64);
+}
+
+// Sum of each of a thread's 32 values over the warp's lanes: lane l ends with
+// the total of value l (31 shuffles, against 160 for 32 separate reductions).
+__device__ __forceinline__ float transpose_sum32(float (&v)[32])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = up ? v[i + o] : v[i], give = up ? v[i] : v[i + o];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0];
+}
+
+// Head (tiles of 128 edges).  Inference: logits only.  TRAIN: also the
+// weighted BCE loss, dL/ds, dz, de = dz W_h and the head's weight gradients.
+// Two threads a row (warps w and w + 4 take channels 0-31 and 32-63), column
+// sums of dz and ds z by a transposing warp reduction.
+template <bool TRAIN>
+__global__ void __launch_bounds__(TPB, 3) head_kernel(size_t E, const float *prm, ParamOffsets o, const float *eL,
+                                                      float *s_out, const float *labels, float pos_weight, float inv_E,
+                                                      float *de, float *grad, float *loss, int *status)
+{
+    extern __shared__ uint8_t sm_raw[];
+    __shared__ uint64_t bar;
+    __shared__ uint32_t slot;
+    __shared__ float part[RT], s_bh[H], s_wo[H];
+    uint8_t *sm = tiles_base(sm_raw);
+    uint8_t *Ws = sm + TileSmem::W, *Es = sm + TileSmem::A, *DZs = sm + TileSmem::A2;
+    float *ms = reinterpret_cast<float *>(sm + TileSmem::M);
+    constexpr uint32_t kCols = TRAIN ? 128 : 64; // cols 0-63 z, then de; 64-127 dW_h
+    if (threadIdx.x < H) {
+        s_bh[threadIdx.x] = prm[o.b_h + threadIdx.x];
+        s_wo[threadIdx.x] = prm[o.w_o + threadIdx.x];
+    }
+    tmem_setup(&bar, &slot, kCols);
+    const uint32_t tm = slot;
+    uint32_t phase = 0;
+    const float bo = prm[o.b_o];
+    stage_tile(Ws, prm + o.W_h, H, H, H); // W_h[o][i]
+    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, half = w >> 2, r = ((w & 3) << 5) + lane, c0 = half << 5;
+    float sum_bh = 0.f, sum_wo = 0.f, sum_bo = 0.f, sum_loss = 0.f; // channel c0 + lane; rows of this thread
+    bool wg_started = false;
+    const size_t tiles = (E + RT - 1) / RT;
+    for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const size_t e0 = t * RT;
+        const int rows = (int)min((size_t)RT, E - e0);
+        stage_tile(Es, eL + e0 * H, H, RT, rows);
+        operands_ready();
+        gemm_rows_cols(tm, Es, Ws, false, H);
+        if (!gemm_wait(&bar, phase, status)) break;
+        float zp[32];
+        umma::tmem_ld32(umma::taddr(tm, (w & 3) << 5, c0), zp);
+#pragma unroll
+        for (int i = 0; i < 32; i++) zp[i] += s_bh[c0 + i];
+        // the logit is summed channel by channel: the lower half's threads start it, the upper half's end it
+        float sv = bo;
+        if (half == 0) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) sv += fmaxf(zp[i], 0.f) * s_wo[i];
+            part[r] = sv;
+        }
+        __syncthreads();
+        if (half == 1) {
+            sv = part[r];
+#pragma unroll
+            for (int i = 0; i < 32; i++) sv += fmaxf(zp[i], 0.f) * s_wo[32 + i];
+            if (r < rows) s_out[e0 + r] = sv;
+        }
+        if (!TRAIN) {
             umma::fence_before();
             __syncthreads();
             continue;
         }
         float ds = 0.f;
-        if (r < rows) {
-            const float y = labels[e0 + r];
-            const float sg = sigmoidf_(sv);
-            // -(w y log sig(s) + (1-y) log(1-sig(s))), with log sig(s) = -softplus(-s)
-            const float sp_neg = fmaxf(-sv, 0.f) + log1pf(expf(-fabsf(sv)));
-            const float sp_pos = fmaxf(sv, 0.f) + log1pf(expf(-fabsf(sv)));
-            atomicAdd(&red[4 * H - 1], (pos_weight * y * sp_neg + (1.f - y) * sp_pos) * inv_E);
-            ds = (pos_weight * y * (sg - 1.f) + (1.f - y) * sg) * inv_E;
-            atomicAdd(&red[2 * H], ds);
-        }
-        for (int c = 0; c < H; c++) {
-            const float z = fmaxf(zp[c], 0.f);
-            const float dz = zp[c] > 0.f ? ds * wo[c] : 0.f;
+        if (half == 1) {
             if (r < rows) {
-                atomicAdd(&red[c], dz);
-                atomicAdd(&red[H + c], ds * z);
+                const float y = labels[e0 + r];
+                const float sg = sigmoidf_(sv);
+                // -(w y log sig(s) + (1-y) log(1-sig(s))), with log sig(s) = -softplus(-s)
+                const float sp_neg = fmaxf(-sv, 0.f) + log1pf(expf(-fabsf(sv)));
+                const float sp_pos = fmaxf(sv, 0.f) + log1pf(expf(-fabsf(sv)));
+                sum_loss += (pos_weight * y * sp_neg + (1.f - y) * sp_pos) * inv_E;
+                ds = (pos_weight * y * (sg - 1.f) + (1.f - y) * sg) * inv_E;
+                sum_bo += ds;
             }
-            *reinterpret_cast<uint16_t *>(DZs + umma::kmajor_offset(r, c, H)) = umma::bf16_bits(dz);
-            *reinterpret_cast<uint16_t *>(DZTs + umma::kmajor_offset(c, r, 128)) = umma::bf16_bits(dz);
+            part[r] = ds;
+        }
+        __syncthreads();
+        ds = part[r];
+        float tmp[32];
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+            const float z = fmaxf(zp[i], 0.f);
+            tmp[i] = ds * z;
+            zp[i] = zp[i] > 0.f ? ds * s_wo[c0 + i] : 0.f; // dz (rows past the end: ds = 0)
+        }
+        if (r >= rows) // keep whatever the padding rows hold out of the sums and products
+#pragma unroll
+            for (int i = 0; i < 32; i++) zp[i] = tmp[i] = 0.f;
+        sum_wo += transpose_sum32(tmp);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            uint32_t u[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                u[i] = (uint32_t)umma::bf16_bits(zp[8 * j + 2 * i]) | ((uint32_t)umma::bf16_bits(zp[8 * j + 2 * i + 1]) << 16);
+            *reinterpret_cast<uint4 *>(DZs + umma::sw_offset(r, (c0 >> 3) + j)) = make_uint4(u[0], u[1], u[2], u[3]);
         }
         operands_ready();
-        gemm_issue(tm + 64, DZs, BTs, H, H, false);         // de = dz W_h
-        gemm_issue(tm + 128, DZTs, ETs, 128, H, wg_started); // dW_h += dz^T eL
+        gemm_rows_cols(tm, DZs, Ws, true, H);           // de = dz W_h
+        gemm_outer(tm + 64, DZs, 0, Es, RT, wg_started); // dW_h += dz^T eL
         wg_started = true;
+        sum_bh += transpose_sum32(zp);
         if (!gemm_wait(&bar, phase, status)) break;
-        float dv[64];
-        tmem_row64(tm, 64, dv);
-        if (r < rows)
-            for (int c = 0; c < H; c += 4)
-                *reinterpret_cast<float4 *>(de + (e0 + r) * H + c) = make_float4(dv[c], dv[c + 1], dv[c + 2], dv[c + 3]);
+        acc_to_tile(tm, 0, ms);
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < RPH; s++) {
+            const int rr = hw * RPH + s;
+            if (rr < rows) st4(de + (e0 + rr) * H + 4 * hl, ld4(ms + (size_t)rr * MS + 4 * hl));
+        }
         umma::fence_before();
         __syncthreads();
     }
-    if (train) {
+    if (TRAIN) {
         __syncthreads();
+        umma::fence_after();
         if (wg_started) { // rows o < 64 of the accumulated dW_h (TMEM lanes 0-63)
-            float w[64];
-            tmem_row64(tm, 128, w);
-            if (threadIdx.x < H)
-                for (int c = 0; c < H; c++) atomicAdd(&grad[o.W_h + threadIdx.x * H + c], w[c]);
+            acc_to_tile(tm, 64, ms);
+            __syncthreads();
+            add_tile_rows(ms, grad + o.W_h);
         }
-        for (int i = threadIdx.x; i < H; i += blockDim.x) {
-            atomicAdd(&grad[o.b_h + i], red[i]);
-            atomicAdd(&grad[o.w_o + i], red[H + i]);
-        }
-        if (threadIdx.x == 0) {
-            atomicAdd(&grad[o.b_o], red[2 * H]);
-            atomicAdd(loss, red[4 * H - 1]);
+        atomicAdd(&grad[o.b_h + c0 + lane], sum_bh);
+        atomicAdd(&grad[o.w_o + c0 + lane], sum_wo);
+        if (half == 1) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                sum_bo += __shfl_xor_sync(0xffffffffu, sum_bo, off);
+                sum_loss += __shfl_xor_sync(0xffffffffu, sum_loss, off);
+            }
+            if (lane == 0) {
+                atomicAdd(&grad[o.b_o], sum_bo);
+                atomicAdd(loss, sum_loss);
+            }
         }
     }
-    tmem_teardown(tm, 256);
+    tmem_teardown(tm, kCols);
 }
 
 // ---- backward ------------------------------------------------------------------
-// Edge layer backward on node tiles.  dh = dL/dh', de = dL/de' (overwritten by
-// dL/de); dP receives du (owned), dV (atomic), dB (owned), dC (atomic).
-struct EdgeBwdSmem {
-    static constexpr size_t DQ = 0, BT = DQ + 128 * H * 2, DQT = BT + H * H * 2, ET = DQT + 128 * 128 * 2,
-                            DU = ET + H * 128 * 2, DQF = DU + 128 * H * 4, RED = DQF + 128 * H * 4,
-                            BYTES = RED + H * 4;
-};
-
-__global__ void __launch_bounds__(TPB) edge_bwd_kernel(int N, int k, const float *A_w, const float *P,
-                                                       const float *u, const float *q, const float *e_in,
-                                                       const float *e_out, const int *nbr, const float *dh, float *de,
-                                                       float *dP, float *gA, float *ga, int *status)
+// Edge layer backward on tiles of 128 edges.  dh = dL/dh', de = dL/de'
+// (overwritten by dL/de); dP receives du (owned), dV, dB and dC (vector
+// reductions into a zeroed buffer; a half-warp sums the rows of one node
+// before it adds them to dB).  LAST: the last layer, where dh = 0 and so du and
+// dV are zero.  EMBED: layer 0, whose e_in is made from the edge feature and
+// whose dL/de goes straight into the embedding's gradient (gwe, gbe).
+template <bool LAST, bool EMBED>
+__global__ void __launch_bounds__(TPB, 2) edge_bwd_kernel(size_t E, int N, int k, const float *A_w, const float *P,
+                                                          const float *u, const uint8_t *qm, const float *e_in,
+                                                          const float *w_e, const float *b_e, const float *e_out,
+                                                          const int *nbr, const float *dh, float *de, float *dP,
+                                                          float *gA, float *ga, float *gwe, float *gbe, int *status)
 {
-    extern __shared__ __align__(1024) uint8_t sm[];
+    extern __shared__ uint8_t sm_raw[];
     __shared__ uint64_t bar;
     __shared__ uint32_t slot;
-    uint8_t *DQs = sm + EdgeBwdSmem::DQ, *BTs = sm + EdgeBwdSmem::BT, *DQTs = sm + EdgeBwdSmem::DQT;
-    uint8_t *ETs = sm + EdgeBwdSmem::ET;
-    float *dus = reinterpret_cast<float *>(sm + EdgeBwdSmem::DU);  // npt x 64
-    float *dqf = reinterpret_cast<float *>(sm + EdgeBwdSmem::DQF); // 128 x 64
-    float *red = reinterpret_cast<float *>(sm + EdgeBwdSmem::RED); // grad of a
+    uint8_t *sm = tiles_base(sm_raw);
+    uint8_t *Ws = sm + TileSmem::W, *DQs = sm + TileSmem::A, *Es = sm + TileSmem::A2;
+    float *ms = reinterpret_cast<float *>(sm + TileSmem::M);
     tmem_setup(&bar, &slot, 128);
-    const uint32_t tm = slot; // cols 0-63 dgrad, 64-127 dA
+    const uint32_t tm = slot; // cols 0-63 dq A, 64-127 dA
     uint32_t phase = 0;
-    stage_cols(BTs, A_w, H, H, H, H); // tile(i, o) = A[o][i]
-    zero_rows(DQTs, H, 128, 128);
-    for (int i = threadIdx.x; i < H; i += blockDim.x) red[i] = 0.f;
+    stage_tile(Ws, A_w, H, H, H); // A[o][i]
+    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15, c = 4 * hl;
+    float4 we = zero4(), be = zero4(), sum_a = zero4(), sum_we = zero4(), sum_be = zero4();
+    if (EMBED) {
+        we = ldg4(w_e + c);
+        be = ldg4(b_e + c);
+    }
+    const float kf = (float)k;
     bool wg_started = false;
-    const int npt = 128 / k, tiles = (N + npt - 1) / npt;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int n0 = t * npt, nodes = min(npt, N - n0), rows = nodes * k;
-        const size_t e0 = (size_t)n0 * k;
-        for (int idx = threadIdx.x; idx < nodes * H; idx += blockDim.x) {
-            const int qn = idx / H, c = idx - qn * H, i = n0 + qn;
-            const float dv = u[(size_t)i * H + c] > 0.f ? dh[(size_t)i * H + c] : 0.f;
-            dus[qn * H + c] = dv;
-            dP[(size_t)i * 4 * H + c] = dv;
-        }
-        stage_cols(ETs, e_in + e0 * H, H, H, 128, rows); // tile(i, e) = e_in[e][i]
-        __syncthreads();
-        const int r = threadIdx.x;
-        if (r < rows) {
-            const size_t ei = e0 + r;
-            const int ql = r / k;
-            int j = nbr[ei];
-            if ((unsigned)j >= (unsigned)N) {
-                set_status(status, ACO_ERR_INVALID);
-                j = 0;
+    const size_t tiles = (E + RT - 1) / RT;
+    for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const size_t e0 = t * RT;
+        const int rows = (int)min((size_t)RT, E - e0);
+        int src = (int)((e0 + hw * RPH) / (size_t)k), rem = (int)((e0 + hw * RPH) - (size_t)src * k);
+        float4 dt[RPH], node = zero4();
+        float ef[RPH];
+#pragma unroll
+        for (int s = 0; s < RPH; s++) {
+            const int r = hw * RPH + s;
+            float4 dq = zero4(), ei4 = zero4();
+            dt[s] = zero4();
+            ef[s] = 0.f;
+            if (r < rows) {
+                const size_t ei = e0 + r;
+                int j = __ldg(nbr + ei);
+                if (EMBED) {
+                    ef[s] = __ldg(e_in + ei);
+                    ei4 = embed4(ef[s], we, be);
+                } else {
+                    ei4 = ldg4(e_in + ei * H + c);
+                }
+                const unsigned m = qm[ei * 16 + hl];
+                float4 d = ld4(de + ei * H + c);
+                if ((unsigned)j >= (unsigned)N) {
+                    if (hl == 0) set_status(status, ACO_ERR_INVALID);
+                    j = 0;
+                }
+                float *dPj = dP + (size_t)j * 4 * H + c;
+                if (!LAST) {
+                    const float4 eo = ldg4(e_out + ei * H + c), vj = ldg4(P + (size_t)j * 4 * H + H + c);
+                    const float4 uu = ldg4(u + (size_t)src * H + c), hh = ldg4(dh + (size_t)src * H + c);
+                    const float4 du = make_float4(uu.x > 0.f ? hh.x : 0.f, uu.y > 0.f ? hh.y : 0.f,
+                                                  uu.z > 0.f ? hh.z : 0.f, uu.w > 0.f ? hh.w : 0.f);
+                    if (rem == 0) st4(dP + (size_t)src * 4 * H + c, du);
+                    const float4 du_e = make_float4(du.x / kf, du.y / kf, du.z / kf, du.w / kf);
+                    const float g0 = sigmoidf_(eo.x), g1 = sigmoidf_(eo.y), g2 = sigmoidf_(eo.z), g3 = sigmoidf_(eo.w);
+                    red4(dPj + H, make_float4(du_e.x * g0, du_e.y * g1, du_e.z * g2, du_e.w * g3));
+                    d.x += du_e.x * vj.x * g0 * (1.f - g0);
+                    d.y += du_e.y * vj.y * g1 * (1.f - g1);
+                    d.z += du_e.z * vj.z * g2 * (1.f - g2);
+                    d.w += du_e.w * vj.w * g3 * (1.f - g3);
+                }
+                dt[s] = d; // the residual part; the product is added below
+                dq = make_float4(m & 1u ? d.x : 0.f, m & 2u ? d.y : 0.f, m & 4u ? d.z : 0.f, m & 8u ? d.w : 0.f);
+                red4(dPj + 3 * H, dq);
+                acc4(node, dq);
+                acc4(sum_a, dq);
+                if (rem == k - 1 || s == RPH - 1 || r == rows - 1) { // this node's rows here are done
+                    red4(dP + (size_t)src * 4 * H + 2 * H + c, node);
+                    node = zero4();
+                }
+                if (++rem == k) {
+                    rem = 0;
+                    src++;
+                }
             }
-            const float *Pj = P + (size_t)j * 4 * H;
-            for (int c = 0; c < H; c++) {
-                const float due = dus[ql * H + c] / (float)k;
-                const float g = sigmoidf_(e_out[ei * H + c]);
-                atomicAdd(&dP[(size_t)j * 4 * H + H + c], due * g);
-                const float dt = de[ei * H + c] + due * Pj[H + c] * g * (1.f - g);
-                const float dq = q[ei * H + c] > 0.f ? dt : 0.f;
-                de[ei * H + c] = dt; // the residual part; the GEMM part is added below
-                dqf[r * H + c] = dq;
-                atomicAdd(&dP[(size_t)j * 4 * H + 3 * H + c], dq);
-                *reinterpret_cast<uint16_t *>(DQs + umma::kmajor_offset(r, c, H)) = umma::bf16_bits(dq);
-                *reinterpret_cast<uint16_t *>(DQTs + umma::kmajor_offset(c, r, 128)) = umma::bf16_bits(dq);
-            }
-        } else {
-            for (int c = 0; c < H; c++) {
-                dqf[r * H + c] = 0.f;
-                *reinterpret_cast<uint16_t *>(DQs + umma::kmajor_offset(r, c, H)) = 0;
-                *reinterpret_cast<uint16_t *>(DQTs + umma::kmajor_offset(c, r, 128)) = 0;
-            }
+            put4(DQs, r, hl, dq);
+            put4(Es, r, hl, ei4);
         }
         operands_ready();
-        gemm_issue(tm, DQs, BTs, H, H, false);             // dq A
-        gemm_issue(tm + 64, DQTs, ETs, 128, H, wg_started); // dA += dq^T e_in
+        gemm_rows_cols(tm, DQs, Ws, true, H);           // dq A
+        gemm_outer(tm + 64, DQs, 0, Es, RT, wg_started); // dA += dq^T e_in
         wg_started = true;
         if (!gemm_wait(&bar, phase, status)) break;
-        float dv[64];
-        tmem_row64(tm, 0, dv);
-        if (r < rows) {
-            const size_t ei = e0 + r;
-            for (int c = 0; c < H; c++) de[ei * H + c] += dv[c];
-        }
-        for (int idx = threadIdx.x; idx < nodes * H; idx += blockDim.x) {
-            const int qn = idx / H, c = idx - qn * H;
-            float acc = 0.f;
-            for (int jj = 0; jj < k; jj++) acc += dqf[(qn * k + jj) * H + c];
-            dP[(size_t)(n0 + qn) * 4 * H + 2 * H + c] = acc;
-        }
-        for (int c = threadIdx.x; c < H; c += blockDim.x) {
-            float acc = 0.f;
-            for (int rr = 0; rr < rows; rr++) acc += dqf[rr * H + c];
-            red[c] += acc;
+        acc_to_tile(tm, 0, ms);
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < RPH; s++) {
+            const int r = hw * RPH + s;
+            if (r < rows) {
+                float4 d = ld4(ms + (size_t)r * MS + c);
+                d = make_float4(dt[s].x + d.x, dt[s].y + d.y, dt[s].z + d.z, dt[s].w + d.w);
+                if (EMBED) {
+                    acc4(sum_be, d);
+                    acc4(sum_we, make_float4(d.x * ef[s], d.y * ef[s], d.z * ef[s], d.w * ef[s]));
+                } else {
+                    st4(de + (e0 + r) * H + c, d);
+                }
+            }
         }
         umma::fence_before();
         __syncthreads();
     }
     __syncthreads();
+    umma::fence_after();
     if (wg_started) {
-        float w[64];
-        tmem_row64(tm, 64, w);
-        if (threadIdx.x < H)
-            for (int c = 0; c < H; c++) atomicAdd(&gA[threadIdx.x * H + c], w[c]);
+        acc_to_tile(tm, 64, ms);
+        __syncthreads();
+        add_tile_rows(ms, gA);
     }
-    for (int i = threadIdx.x; i < H; i += blockDim.x) atomicAdd(&ga[i], red[i]);
+    add_channel_sums(sum_a, ms, ga);
+    if (EMBED) {
+        add_channel_sums(sum_we, ms, gwe);
+        add_channel_sums(sum_be, ms, gbe);
+    }
     tmem_teardown(tm, 128);
 }
 
-// dh += dP W (K = 256), dW += dP^T h (two M = 128 halves), db += sum dP.
+// dh += dP W (K = 256), dW += dP^T h (two halves of 128 outputs), db += sum dP,
+// on tiles of 64 nodes (twice the CTAs of 128: 9.2 k nodes give 144).  The
+// accumulator of dP W has 128 rows; its upper 64 come from whatever follows
+// the operand's 64 rows in shared memory and are not read.  LAST: dh = 0 on
+// entry.  EMBED: layer 0, whose dL/dh goes into the node embedding's gradient.
 struct NodeBwdSmem {
-    static constexpr size_t A = 0, BT = A + 128 * 4 * H * 2, AT = BT + H * 4 * H * 2, HT = AT + 2 * 128 * 128 * 2,
-                            RED = HT + H * 128 * 2, BYTES = RED + 4 * H * 4;
+    static constexpr int NT = 64;
+    static constexpr size_t A = 0, W = A + 4 * NT * H * 2, HT = W + 4 * H * H * 2, M = HT + NT * H * 2,
+                            END = M + (size_t)RT * MS * 4, BYTES = END + 1024;
 };
 
+template <bool LAST, bool EMBED>
 __global__ void __launch_bounds__(TPB) node_bwd_kernel(int N, const float *W, const float *h_in, const float *dP,
-                                                       float *dh, float *gW, float *gb, int *status)
+                                                       float *dh, const float *nf, float *gW, float *gb, float *gwn,
+                                                       float *gbn, int *status)
 {
-    extern __shared__ __align__(1024) uint8_t sm[];
+    extern __shared__ uint8_t sm_raw[];
     __shared__ uint64_t bar;
     __shared__ uint32_t slot;
-    uint8_t *As = sm + NodeBwdSmem::A, *BTs = sm + NodeBwdSmem::BT, *ATs = sm + NodeBwdSmem::AT;
-    uint8_t *HTs = sm + NodeBwdSmem::HT;
-    float *red = reinterpret_cast<float *>(sm + NodeBwdSmem::RED);
+    constexpr int NT = NodeBwdSmem::NT, RH = NT / (TPB / 16);
+    constexpr uint32_t kAtom = NT * H * 2; // bytes of 64 channels of the dP tile
+    uint8_t *sm = tiles_base(sm_raw);
+    uint8_t *As = sm + NodeBwdSmem::A, *Ws = sm + NodeBwdSmem::W, *Hs = sm + NodeBwdSmem::HT;
+    float *ms = reinterpret_cast<float *>(sm + NodeBwdSmem::M);
     tmem_setup(&bar, &slot, 256);
     const uint32_t tm = slot; // 0-63 dgrad, 64-127 dW rows 0-127, 128-191 dW rows 128-255
     uint32_t phase = 0;
-    stage_cols(BTs, W, H, H, 4 * H, 4 * H); // tile(c, o) = W[o][c]
-    for (int i = threadIdx.x; i < 4 * H; i += blockDim.x) red[i] = 0.f;
+    stage_tile(Ws, W, H, 4 * H, 4 * H); // W[o][c], 256 rows
+    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15, c = 4 * hl;
+    const int sec = (threadIdx.x >> 4) & 3, rq = threadIdx.x >> 6; // staging: section and row group of the thread
+    float4 sum_b = zero4();
+    float4 sum_n[FN + 1];
+#pragma unroll
+    for (int f = 0; f <= FN; f++) sum_n[f] = zero4();
     bool wg_started = false;
-    const int tiles = (N + 127) / 128;
+    const int tiles = (N + NT - 1) / NT;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int r0 = t * 128, valid = min(128, N - r0);
-        stage_rows(As, dP + (size_t)r0 * 4 * H, 4 * H, 128, 4 * H, valid);
-        stage_cols(ATs, dP + (size_t)r0 * 4 * H, 4 * H, 128, 128, valid);                 // tile(o, i) = dP[i][o], o < 128
-        stage_cols(ATs + 128 * 128 * 2, dP + (size_t)r0 * 4 * H + 128, 4 * H, 128, 128, valid); // o in [128, 256)
-        stage_cols(HTs, h_in + (size_t)r0 * H, H, H, 128, valid);                       // tile(c, i) = h[i][c]
-        for (int oo = threadIdx.x; oo < 4 * H; oo += blockDim.x) {
-            float acc = 0.f;
-            for (int i = 0; i < valid; i++) acc += dP[(size_t)(r0 + i) * 4 * H + oo];
-            red[oo] += acc;
+        const int r0 = t * NT, valid = min(NT, N - r0);
+#pragma unroll 8
+        for (int r = rq; r < NT; r += 4) {
+            const float4 v = r < valid ? ldg4(dP + (size_t)(r0 + r) * 4 * H + sec * H + c) : zero4();
+            put4(As + sec * kAtom, r, hl, v);
+            acc4(sum_b, v);
         }
+        stage_tile(Hs, h_in + (size_t)r0 * H, H, NT, valid);
         operands_ready();
-        gemm_issue(tm, As, BTs, 4 * H, H, false);
-        gemm_issue(tm + 64, ATs, HTs, 128, H, wg_started);
-        gemm_issue(tm + 128, ATs + 128 * 128 * 2, HTs, 128, H, wg_started);
+        if (threadIdx.x == 0) { // dP W: K = 256 outputs, A by rows (four 64-channel sections), W transposed
+            const uint32_t id = umma::idesc_bf16(128, H, false, true);
+            const uint32_t aa = smem_u32(As), bb = smem_u32(Ws);
+            for (int s = 0; s < 4 * H / 16; s++)
+                umma::mma_bf16(tm, umma::desc_k(aa + (s >> 2) * kAtom, s & 3), umma::desc_mn(bb, s, 0), id, s > 0);
+        }
+        gemm_outer(tm + 64, As, kAtom, Hs, NT, wg_started);
+        gemm_outer(tm + 128, As + 2 * kAtom, kAtom, Hs, NT, wg_started);
         wg_started = true;
         if (!gemm_wait(&bar, phase, status)) break;
-        float dv[64];
-        tmem_row64(tm, 0, dv);
-        const int r = threadIdx.x;
-        if (r < valid)
-            for (int c = 0; c < H; c++) dh[(size_t)(r0 + r) * H + c] += dv[c];
+        acc_to_tile(tm, 0, ms);
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < RH; s++) {
+            const int r = hw * RH + s;
+            if (r < valid) {
+                float4 d = ld4(ms + (size_t)r * MS + c);
+                float *row = dh + (size_t)(r0 + r) * H + c;
+                if (!LAST) {
+                    const float4 o = ld4(row);
+                    d = make_float4(o.x + d.x, o.y + d.y, o.z + d.z, o.w + d.w);
+                }
+                if (EMBED) {
+                    const float *f5 = nf + (size_t)(r0 + r) * FN;
+#pragma unroll
+                    for (int f = 0; f < FN; f++) {
+                        const float x = __ldg(f5 + f);
+                        acc4(sum_n[f], make_float4(d.x * x, d.y * x, d.z * x, d.w * x));
+                    }
+                    acc4(sum_n[FN], d);
+                } else {
+                    st4(row, d);
+                }
+            }
+        }
         umma::fence_before();
         __syncthreads();
     }
     __syncthreads();
+    umma::fence_after();
     if (wg_started) {
-        float w0[64], w1[64];
-        tmem_row64(tm, 64, w0);
-        tmem_row64(tm, 128, w1);
-        const int o = threadIdx.x;
-        for (int c = 0; c < H; c++) {
-            atomicAdd(&gW[o * H + c], w0[c]);
-            atomicAdd(&gW[(128 + o) * H + c], w1[c]);
+        for (int half = 0; half < 2; half++) {
+            acc_to_tile(tm, 64 + 64 * half, ms);
+            __syncthreads();
+            for (int r = hw; r < RT; r += TPB / 16) add4(gW + (size_t)(half * RT + r) * H + c, ld4(ms + (size_t)r * MS + c));
+            __syncthreads();
         }
     }
-    for (int i = threadIdx.x; i < 4 * H; i += blockDim.x) atomicAdd(&gb[i], red[i]);
-    tmem_teardown(tm, 256);
-}
-
-// Input embeddings' gradients (CUDA cores: K = 5 and 1).
-__global__ void embed_bwd_kernel(int N, int k, ParamOffsets o, const float *nf, const float *ef, const float *dh0,
-                                 const float *de0, float *grad)
-{
-    // each block: one output channel c, all nodes / edges
-    const int c = blockIdx.x;
-    __shared__ float red[8][FN + 3];
-    float acc[FN + 3] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        const float d = dh0[(size_t)i * H + c];
-        for (int f = 0; f < FN; f++) acc[f] += d * nf[(size_t)i * FN + f];
-        acc[FN] += d;
-    }
-    const size_t E = (size_t)N * k;
-    for (size_t e = threadIdx.x; e < E; e += blockDim.x) {
-        const float d = de0[e * H + c];
-        acc[FN + 1] += d * ef[e];
-        acc[FN + 2] += d;
-    }
-    for (int f = 0; f < FN + 3; f++)
-        for (int off = 16; off > 0; off >>= 1) acc[f] += __shfl_xor_sync(0xffffffffu, acc[f], off);
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0)
-        for (int f = 0; f < FN + 3; f++) red[w][f] = acc[f];
+    // db: the four row groups of a section add up
+    st4(ms + (size_t)rq * 4 * H + sec * H + c, sum_b);
     __syncthreads();
-    if (threadIdx.x < FN + 3) {
-        float s = 0.f;
-        for (int ww = 0; ww < (int)(blockDim.x >> 5); ww++) s += red[ww][threadIdx.x];
-        const int f = threadIdx.x;
-        if (f < FN) grad[o.W_n + c * FN + f] = s;
-        else if (f == FN) grad[o.b_n + c] = s;
-        else if (f == FN + 1) grad[o.W_e + c] = s;
-        else grad[o.b_e + c] = s;
+    {
+        const int oo = threadIdx.x;
+        atomicAdd(&gb[oo], ((ms[oo] + ms[4 * H + oo]) + ms[8 * H + oo]) + ms[12 * H + oo]);
     }
+    if (EMBED) {
+        __syncthreads();
+#pragma unroll
+        for (int f = 0; f <= FN; f++) {
+            // W_n is 64 x FN: channel sums of feature f go FN floats apart
+            __syncthreads();
+            st4(ms + hw * H + c, sum_n[f]);
+            __syncthreads();
+            if (threadIdx.x < H) {
+                float s = 0.f;
+                for (int i = 0; i < TPB / 16; i++) s += ms[i * H + threadIdx.x];
+                atomicAdd(f < FN ? gwn + threadIdx.x * FN + f : gbn + threadIdx.x, s);
+            }
+        }
+    }
+    tmem_teardown(tm, 256);
 }
 
 __global__ void adam_kernel(int n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2,
@@ -711,27 +897,75 @@ bool args_ok(int N, int k, int L)
     return N >= 1 && k >= 1 && k <= 32 && L >= 1 && L <= 8 && (size_t)N * k < ((size_t)1 << 31);
 }
 
+// A persistent grid: at most as many CTAs as are resident at once (ctas per SM).
+unsigned grid_of(size_t tiles, int ctas) { return (unsigned)std::min(tiles, (size_t)sm_count() * ctas); }
+
+template <bool EMBED, bool TRAIN>
+cudaError_t launch_edge_fwd(int N, int k, const float *prm, const ParamOffsets &o, int l, const float *e_in,
+                            const float *h, const int *nbr, const float *P, const Workspace &w, cudaStream_t st)
+{
+    const size_t E = (size_t)N * k;
+    const cudaError_t e = set_smem(edge_fwd_kernel<EMBED, TRAIN>, TileSmem::BYTES);
+    if (e != cudaSuccess) return e;
+    const int npt = RT / k;
+    edge_fwd_kernel<EMBED, TRAIN><<<grid_of((N + npt - 1) / npt, 3), TPB, TileSmem::BYTES, st>>>(
+        N, k, prm + o.A[l], prm + o.a[l], e_in, prm + o.W_e, prm + o.b_e, P, h, nbr, w.qm + (size_t)l * E * 16,
+        w.e + (size_t)l * E * H, w.u + (size_t)l * N * H, w.h + (size_t)(l + 1) * N * H, w.status);
+    return cudaGetLastError();
+}
+
+template <bool TRAIN>
 int run_forward(int N, int k, int L, const float *prm, const float *nf, const float *ef, const int *nbr,
                 const Workspace &w, cudaStream_t st)
 {
     const ParamOffsets o = param_offsets(L);
     const size_t E = (size_t)N * k;
-    const int grid_sm = sm_count() * 2;
-    embed_kernel<<<std::min<size_t>(((size_t)N * H + E * H + 255) / 256, (size_t)grid_sm * 8), 256, 0, st>>>(
-        N, k, prm, o, nf, ef, w.h, w.e);
-    if (set_smem(node_gemm_kernel, NodeGemmSmem::BYTES) != cudaSuccess) return ACO_ERR_CUDA;
-    if (set_smem(edge_fwd_kernel, EdgeFwdSmem::BYTES) != cudaSuccess) return ACO_ERR_CUDA;
-    const int ntiles = (N + 127) / 128, npt = 128 / k, etiles = (N + npt - 1) / npt;
+    embed_nodes_kernel<<<grid_of(((size_t)N * H + 255) / 256, 8), 256, 0, st>>>(N, prm, o, nf, w.h);
+    if (set_smem(node_gemm_kernel, TileSmem::BYTES) != cudaSuccess) return ACO_ERR_CUDA;
+    const size_t ntiles = (N + RT - 1) / RT;
     for (int l = 0; l < L; l++) {
-        const float *h = w.h + (size_t)l * N * H, *e = w.e + (size_t)l * E * H;
+        const float *h = w.h + (size_t)l * N * H;
         float *P = w.P + (size_t)l * N * 4 * H;
-        node_gemm_kernel<<<std::min(ntiles, grid_sm), TPB, NodeGemmSmem::BYTES, st>>>(N, h, prm + o.W[l],
-                                                                                     prm + o.b[l], P, w.status);
-        edge_fwd_kernel<<<std::min(etiles, grid_sm), TPB, EdgeFwdSmem::BYTES, st>>>(
-            N, k, prm + o.A[l], prm + o.a[l], e, P, h, nbr, w.q + (size_t)l * E * H, w.e + (size_t)(l + 1) * E * H,
-            w.u + (size_t)l * N * H, w.h + (size_t)(l + 1) * N * H, w.status);
+        node_gemm_kernel<<<dim3(grid_of(ntiles, 1), 4), TPB, TileSmem::BYTES, st>>>(N, h, prm + o.W[l], prm + o.b[l], P,
+                                                                                   w.status);
+        const cudaError_t e = l == 0 ? launch_edge_fwd<true, TRAIN>(N, k, prm, o, l, ef, h, nbr, P, w, st)
+                                     : launch_edge_fwd<false, TRAIN>(N, k, prm, o, l, w.e + (size_t)(l - 1) * E * H, h,
+                                                                     nbr, P, w, st);
+        if (e != cudaSuccess) return ACO_ERR_CUDA;
     }
     return cudaGetLastError() == cudaSuccess ? ACO_OK : ACO_ERR_CUDA;
+}
+
+template <bool TRAIN>
+cudaError_t launch_head(size_t E, const float *prm, const ParamOffsets &o, const float *eL, float *scores,
+                        const float *labels, float pos_weight, float *de, float *grad, float *loss, int *status,
+                        cudaStream_t st)
+{
+    const cudaError_t e = set_smem(head_kernel<TRAIN>, TileSmem::BYTES);
+    if (e != cudaSuccess) return e;
+    head_kernel<TRAIN><<<grid_of((E + RT - 1) / RT, 3), TPB, TileSmem::BYTES, st>>>(
+        E, prm, o, eL, scores, labels, pos_weight, 1.0f / (float)E, de, grad, loss, status);
+    return cudaGetLastError();
+}
+
+template <bool LAST, bool EMBED>
+cudaError_t launch_layer_bwd(int N, int k, const float *prm, const ParamOffsets &o, int l, const float *nf,
+                             const float *ef, const int *nbr, const Workspace &w, float *grad, cudaStream_t st)
+{
+    const size_t E = (size_t)N * k;
+    cudaError_t e = cudaMemsetAsync(w.dP, 0, sizeof(float) * N * 4 * H, st);
+    if (e == cudaSuccess) e = set_smem(edge_bwd_kernel<LAST, EMBED>, TileSmem::BYTES);
+    if (e == cudaSuccess) e = set_smem(node_bwd_kernel<LAST, EMBED>, NodeBwdSmem::BYTES);
+    if (e != cudaSuccess) return e;
+    edge_bwd_kernel<LAST, EMBED><<<grid_of((E + RT - 1) / RT, 2), TPB, TileSmem::BYTES, st>>>(
+        E, N, k, prm + o.A[l], w.P + (size_t)l * N * 4 * H, w.u + (size_t)l * N * H, w.qm + (size_t)l * E * 16,
+        EMBED ? ef : w.e + (size_t)(l - 1) * E * H, prm + o.W_e, prm + o.b_e, w.e + (size_t)l * E * H, nbr, w.dh, w.de,
+        w.dP, grad + o.A[l], grad + o.a[l], grad + o.W_e, grad + o.b_e, w.status);
+    constexpr int NT = NodeBwdSmem::NT;
+    node_bwd_kernel<LAST, EMBED><<<grid_of((N + NT - 1) / NT, 1), TPB, NodeBwdSmem::BYTES, st>>>(
+        N, prm + o.W[l], w.h + (size_t)l * N * H, w.dP, w.dh, nf, grad + o.W[l], grad + o.b[l], grad + o.W_n,
+        grad + o.b_n, w.status);
+    return cudaGetLastError();
 }
 
 } // namespace
@@ -764,14 +998,13 @@ int aco_mpnn_forward(int n_nodes, int k, int layers, const float *params, const 
     if (ws_bytes < w.bytes) return ACO_ERR_CAPACITY;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(w.status, 0, 64, st) != cudaSuccess) return ACO_ERR_CUDA;
-    int rc = run_forward(n_nodes, k, layers, params, node_feat, edge_feat, nbr, w, st);
+    int rc = run_forward<false>(n_nodes, k, layers, params, node_feat, edge_feat, nbr, w, st);
     if (rc != ACO_OK) return rc;
-    const ParamOffsets o = param_offsets(layers);
     const size_t E = (size_t)n_nodes * k;
-    if (set_smem(head_kernel, HeadSmem::BYTES) != cudaSuccess) return ACO_ERR_CUDA;
-    head_kernel<<<(unsigned)std::min<size_t>((E + 127) / 128, (size_t)sm_count() * 2), TPB, HeadSmem::BYTES, st>>>(
-        E, params, o, w.e + (size_t)layers * E * H, scores, nullptr, 0.f, 0.f, nullptr, nullptr, nullptr, w.status);
-    return cudaGetLastError() == cudaSuccess ? ACO_OK : ACO_ERR_CUDA;
+    return launch_head<false>(E, params, param_offsets(layers), w.e + (size_t)(layers - 1) * E * H, scores, nullptr, 0.f,
+                              nullptr, nullptr, nullptr, w.status, st) == cudaSuccess
+               ? ACO_OK
+               : ACO_ERR_CUDA;
 }
 
 int aco_mpnn_grad(int n_nodes, int k, int layers, const float *params, const float *node_feat, const float *edge_feat,
@@ -786,31 +1019,24 @@ int aco_mpnn_grad(int n_nodes, int k, int layers, const float *params, const flo
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const ParamOffsets o = param_offsets(layers);
     const size_t E = (size_t)n_nodes * k;
-    const int N = n_nodes, L = layers, grid_sm = sm_count() * 2;
+    const int N = n_nodes, L = layers;
     if (cudaMemsetAsync(w.status, 0, 64, st) != cudaSuccess) return ACO_ERR_CUDA;
     if (cudaMemsetAsync(grad, 0, sizeof(float) * o.count, st) != cudaSuccess) return ACO_ERR_CUDA;
     if (cudaMemsetAsync(loss, 0, sizeof(float), st) != cudaSuccess) return ACO_ERR_CUDA;
-    if (cudaMemsetAsync(w.dh, 0, sizeof(float) * N * H, st) != cudaSuccess) return ACO_ERR_CUDA;
-    int rc = run_forward(N, k, L, params, node_feat, edge_feat, nbr, w, st);
+    int rc = run_forward<true>(N, k, L, params, node_feat, edge_feat, nbr, w, st);
     if (rc != ACO_OK) return rc;
-    if (set_smem(head_kernel, HeadSmem::BYTES) != cudaSuccess) return ACO_ERR_CUDA;
-    head_kernel<<<(unsigned)std::min<size_t>((E + 127) / 128, (size_t)grid_sm), TPB, HeadSmem::BYTES, st>>>(
-        E, params, o, w.e + (size_t)L * E * H, scores ? scores : w.s, labels, pos_weight, 1.0f / (float)E, w.de, grad,
-        loss, w.status);
-    if (set_smem(edge_bwd_kernel, EdgeBwdSmem::BYTES) != cudaSuccess) return ACO_ERR_CUDA;
-    if (set_smem(node_bwd_kernel, NodeBwdSmem::BYTES) != cudaSuccess) return ACO_ERR_CUDA;
-    const int ntiles = (N + 127) / 128, npt = 128 / k, etiles = (N + npt - 1) / npt;
+    if (launch_head<true>(E, params, o, w.e + (size_t)(L - 1) * E * H, scores ? scores : w.s, labels, pos_weight, w.de,
+                          grad, loss, w.status, st) != cudaSuccess)
+        return ACO_ERR_CUDA;
     for (int l = L - 1; l >= 0; l--) {
-        float *dP = w.dP;
-        if (cudaMemsetAsync(dP, 0, sizeof(float) * N * 4 * H, st) != cudaSuccess) return ACO_ERR_CUDA;
-        edge_bwd_kernel<<<std::min(etiles, grid_sm), TPB, EdgeBwdSmem::BYTES, st>>>(
-            N, k, params + o.A[l], w.P + (size_t)l * N * 4 * H, w.u + (size_t)l * N * H, w.q + (size_t)l * E * H,
-            w.e + (size_t)l * E * H, w.e + (size_t)(l + 1) * E * H, nbr, w.dh, w.de, dP, grad + o.A[l], grad + o.a[l],
-            w.status);
-        node_bwd_kernel<<<std::min(ntiles, grid_sm), TPB, NodeBwdSmem::BYTES, st>>>(
-            N, params + o.W[l], w.h + (size_t)l * N * H, dP, w.dh, grad + o.W[l], grad + o.b[l], w.status);
+        const bool last = l == L - 1, embed = l == 0;
+        const cudaError_t e =
+            last ? (embed ? launch_layer_bwd<true, true>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st)
+                          : launch_layer_bwd<true, false>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st))
+                 : (embed ? launch_layer_bwd<false, true>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st)
+                          : launch_layer_bwd<false, false>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st));
+        if (e != cudaSuccess) return ACO_ERR_CUDA;
     }
-    embed_bwd_kernel<<<H, 256, 0, st>>>(N, k, o, node_feat, edge_feat, w.dh, w.de, grad);
     return cudaGetLastError() == cudaSuccess ? ACO_OK : ACO_ERR_CUDA;
 }
 
