@@ -19,13 +19,15 @@ namespace aco {
 constexpr uint32_t kPM = 2147483647u; // Park-Miller modulus
 constexpr float kEps = 0.001f;        // EPSILON (utilities.h:19, kernel.cl:6)
 
-// a * b mod (2^31 - 1) for a, b < 2^31 - 1.
+// a * b mod (2^31 - 1) for a, b < 2^31 - 1.  Two folds of 31 bits leave a value in
+// [0, 2^31 - 1], and the modulus itself only for a nonzero product that is 0
+// modulo the prime, which nonzero a, b < 2^31 - 1 cannot give; so there is
+// nothing left to subtract.
 __device__ __forceinline__ uint32_t pm_mul(uint32_t a, uint32_t b)
 {
     const uint64_t p = (uint64_t)a * b;
-    uint32_t r = (uint32_t)(p & kPM) + (uint32_t)(p >> 31);
-    r = (r & kPM) + (r >> 31);
-    return r >= kPM ? r - kPM : r;
+    const uint32_t r = (uint32_t)(p & kPM) + (uint32_t)(p >> 31);
+    return (r & kPM) + (r >> 31);
 }
 
 // 16807^e mod (2^31 - 1): the jump of a Park-Miller state over e draws.

@@ -480,16 +480,28 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         max_routes = std::max<long long>(max_routes, ih.capacity > 0 ? dem / ih.capacity + 1 : 1);
         A_max = std::max(A_max, ih.A);
     }
-    if (!throughput) { // parity construct: warps per ant so that a thread owns <= 32 nodes of a row
+    if (!throughput) {
+        // Warps per ant.  A step costs each warp about 85 instructions plus 27 a node
+        // of its own, and the ant one barrier: few ants on an SM want the row spread,
+        // many want fewer warps.  Construct of one iteration, us, at 1 / 2 / 4 / 8 warps:
+        // 101 nodes 100 ants 28 / 35 / 32 / 34; 201 nodes 201 ants 74 / 65 / 63 / 73;
+        // 484 nodes 120 ants (route limit) 449 / 284 / 241 / 228, 484 ants 292 / 233 /
+        // 273 / 358; 801 nodes 200 ants - / 558 / 402 / 498, 800 ants - / 902 / 1177 / 1217.
         const InstHost &ih = inst[0];
-        int wpa = 1;
-        while (wpa < 8 && 32 * wpa * 32 < ih.n) wpa *= 2;
-        while (wpa < 8 && ih.n > 256 * wpa && 32 * wpa * 2 <= ih.nloc) wpa *= 2;
+        const int per_sm = (ih.A + sm_count - 1) / sm_count;
+        int wpa = 4;
+        if (ih.n <= 128) wpa = 1;
+        else if (per_sm > 3) wpa = ih.n <= 256 ? 1 : 2;
+        else if (per_sm <= 1 && ih.n > 256) wpa = 8;
+        while (wpa < 8 && 32 * wpa * 16 < ih.n) wpa *= 2; // 16 nodes a thread fit its registers
+        while (p.ants_per_block > 0 && wpa > 1 && p.ants_per_block * wpa > 16) wpa /= 2;
         wpa = std::min(wpa, ih.nloc / 32);
         if (p.warps_per_ant > 0) wpa = p.warps_per_ant;
         cp_wpa = wpa;
-        const int per_block = std::max(1, std::min(8, (ih.A + sm_count - 1) / sm_count));
-        cp_apc = p.ants_per_block > 0 ? p.ants_per_block : std::max(1, per_block / wpa);
+        // one CTA an SM with all of its ants (they share the staged matrix); short rows
+        // in fours, whose fewer CTAs start sooner (101 nodes: 27 us for 30)
+        const int per_block = std::max(ih.n <= 128 ? 4 : 1, std::min(8, per_sm));
+        cp_apc = p.ants_per_block > 0 ? p.ants_per_block : std::max(1, std::min(per_block, 16 / wpa));
         if (cp_apc * cp_wpa > 16) return ACO_ERR_INVALID; // 512 threads per CTA at most
         cp_stage = construct_parity_smem(ih.n, ih.nloc, ih.kmax, wpa, cp_apc, true, fin_any) <= kSmemBudget;
     } else {

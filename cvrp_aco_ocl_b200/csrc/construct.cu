@@ -222,6 +222,247 @@ __global__ void __launch_bounds__(512) construct_parity_kernel(ConstructArgs a)
         for (int l = t; l < nlanes; l += TPA) seeds[l] = (int)st[l];
 }
 
+// The same step with everything a thread needs about its nodes in registers, for
+// at most JM (16) nodes a thread; the kernel above is left with longer rows.
+// What bounds it is the latency of one step, so all that does not depend on the
+// step's row is taken off the chain:
+//   * every node keeps its own draw.  The draws of a lane are consecutive powers
+//     of 16807 times its state, so node i's number of the next step is this
+//     step's times 16807^(draws of its lane a step): one product a node and
+//     step, no lane state in shared memory.  It and ran01 + 0.001f are made one
+//     step ahead, under the latency of the row's loads.
+//   * demands and tie keys sit in registers; the tour goes to a shared buffer
+//     and its length is summed after the last step, in step order, from loads in
+//     flight together.
+// Lane states are written back from the lane's last node: its number is the
+// state after the step, so the one made ahead is divided by the lane's power.
+// Construct of one iteration, against the kernel above with its split: 201 nodes
+// 201 ants 298 -> 63 us, 484 nodes 120 ants with a route limit 1572 -> 228 us,
+// 51 nodes 50 ants 44 -> 20 us.
+struct ParityRegsLayout {
+    size_t bar, dem, red, tour, mat, bytes;
+};
+
+__host__ __device__ inline ParityRegsLayout parity_regs_layout(int n, int wpa, int apc, bool smat)
+{
+    const size_t n4 = (size_t)((n + 3) & ~3);
+    ParityRegsLayout L;
+    size_t o = 0;
+    L.bar = o; o = al128(o + 16);
+    L.dem = o; o = al128(o + n4 * 4);
+    L.red = o; o = al128(o + (size_t)apc * 2 * wpa * 8);
+    L.tour = o; o = al128(o + (size_t)apc * 2 * n * 2);
+    L.mat = o;
+    if (smat) o = al128(o + (size_t)n * n4 * 4);
+    L.bytes = o;
+    return L;
+}
+
+// ran01 + 0.001f (kernel.cl:50,353): the product with 2^-31 is exact, so one fused
+// operation rounds as the two do.
+__device__ __forceinline__ float ran01_shifted(uint32_t x)
+{
+    return __fmaf_rn(__int2float_rn((int)x), 4.656612873077392578125e-10f, 0.001f);
+}
+
+template <int WPA, int JM, bool FIN, bool SMAT>
+__global__ void __launch_bounds__(512) construct_parity_regs_kernel(ConstructArgs a)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int TPA = 32 * WPA;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int n = a.n, ld = a.ld, n4 = (n + 3) & ~3;
+    const int apc = blockDim.x / TPA;
+    const ParityRegsLayout L = parity_regs_layout(n, WPA, apc, SMAT);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L.bar);
+    int *s_dem = reinterpret_cast<int *>(smem + L.dem);
+    float *s_mat = reinterpret_cast<float *>(smem + L.mat);
+
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mbar_arrive_expect_tx(bar, (uint32_t)(n4 * 4) + (SMAT ? (uint32_t)(n * n4 * 4) : 0u));
+        tma_bulk_g2s(s_dem, a.demand, n4 * 4, bar);
+    }
+    if (SMAT)
+        for (int r = threadIdx.x; r < n; r += blockDim.x)
+            tma_bulk_g2s(s_mat + (size_t)r * n4, a.total + (size_t)r * ld, n4 * 4, bar);
+
+    const int slot = threadIdx.x / TPA, t = threadIdx.x - slot * TPA, lane = threadIdx.x & 31, wsl = t >> 5;
+    const int ant = blockIdx.x * apc + slot;
+    const bool live = ant < a.n_ants;
+    int *seeds = a.seeds + (size_t)(live ? ant : 0) * a.nloc;
+    const int lmask = a.nloc - 1;
+    // lanes below `more` have kmax nodes, the others one fewer (kmax 1: all of n)
+    const int more = n - (a.kmax - 1) * a.nloc;
+    const uint32_t adv_hi = a.adv[0], adv_lo = a.adv[a.nloc - 1];
+    // per node: draw of the coming step and its ran01 + 0.001f, demand, tie key
+    uint32_t y[JM], key[JM], adv[JM];
+    float r[JM], d0[FIN ? JM : 1];
+    int dem[JM];
+    uint32_t vis = 0u; // bit j: node visited (or past the row)
+#pragma unroll
+    for (int j = 0; j < JM; j++) {
+        const int i = t + TPA * j;
+        y[j] = 1u;
+        key[j] = 0u;
+        dem[j] = 0;
+        if (i < n && live) {
+            y[j] = pm_mul(pm_norm(__ldg(seeds + (i & lmask))), __ldg(a.jump + (i >> a.log2_nloc)));
+            key[j] = __ldg(a.tiekey + i);
+            dem[j] = __ldg(a.demand + i);
+            if (FIN) d0[j] = __ldg(a.dist + (size_t)i * ld); // column 0
+        }
+        adv[j] = (i & lmask) < more ? adv_hi : adv_lo;
+        if (i >= n || i == 0) vis |= 1u << j; // the depot starts visited (kernel.cl:431)
+        r[j] = ran01_shifted(y[j]);
+        // opaque from here on: a load may not be repeated in the loop to save its register
+        asm volatile("" : "+r"(key[j]), "+r"(dem[j]), "+r"(adv[j]));
+        if (FIN) asm volatile("" : "+f"(d0[j]));
+    }
+    const bool ok = mbar_wait(bar, 0, wait_polls(a.wait_limit));
+    if (__syncthreads_or(!ok)) { // give up, but let the copies in flight land first (default bound)
+        if (threadIdx.x == 0) set_status(a.status, ACO_ERR_TIMEOUT);
+        if (!ok) mbar_wait(bar, 0);
+        return;
+    }
+    if (!live) return;
+
+    int step = 0, vcnt = 1, load = 0, err = 0;
+    float rdist = 0.f, pend = 0.f; // FIN: route length before the last edge, that edge's length (or the reset)
+    bool ext = false;
+    uint16_t *tbuf = reinterpret_cast<uint16_t *>(smem + L.tour) + (size_t)slot * 2 * n;
+    if (t == 0) tbuf[0] = 0;
+    const float *base = SMAT ? s_mat : a.total;
+    const size_t stride = SMAT ? (size_t)n4 : (size_t)ld;
+
+    // the row of the coming step is loaded at the end of the step before it: across the
+    // loop's back edge the loads stay together.  Inside one iteration the compiler put
+    // them next to their uses, an L2 trip a node (484 nodes, 4 warps, route limit: 515 us
+    // for 241).
+    float p[JM], dd[FIN ? JM : 1];
+    const float *drow = a.dist;
+    auto load_row = [&](int row) {
+        const float *trow = base + (size_t)row * stride;
+        drow = a.dist + (size_t)row * ld;
+#pragma unroll
+        for (int j = 0; j < JM; j++) {
+            const int i = min(t + TPA * j, n - 1); // past the row: any node, its bit is set
+            p[j] = SMAT ? trow[i] : __ldg(trow + i);
+            if (FIN) dd[j] = __ldg(drow + i);
+        }
+    };
+    load_row(0);
+    while (vcnt < n) {
+        if (step >= a.T - 3) { // 2n-3 steps is the longest valid tour
+            err = ACO_ERR_STEP_LIMIT;
+            break;
+        }
+        // the last edge's length joins here: its load is in flight with the row's
+        if (FIN) rdist = ext ? __fadd_rn(rdist, __fadd_rn(pend, a.serv_time)) : 0.f;
+        // the next step's draws, under the latency of the loads
+        const int room = a.capacity - load;
+        float rc[JM];
+        uint32_t open = 0u;
+#pragma unroll
+        for (int j = 0; j < JM; j++) {
+            rc[j] = r[j];
+            y[j] = pm_mul(y[j], adv[j]);
+            r[j] = ran01_shifted(y[j]);
+            open |= (dem[j] <= room ? 1u : 0u) << j;
+        }
+        open &= ~vis;
+        // value bits over tie key: one 64-bit maximum is the tournament
+        unsigned long long best[JM];
+#pragma unroll
+        for (int j = 0; j < JM; j++) {
+            bool c = (open >> j) & 1u;
+            if (FIN) c = c & (__fadd_rn(__fadd_rn(rdist, __fadd_rn(dd[j], a.serv_time)), d0[j]) <= a.max_dist);
+            const float v = __fmul_rn(rc[j], __fmul_rn(p[j], 100.0f)); // (ran01 + 0.001f) * (total_info * 100)
+            best[j] = ((unsigned long long)(c ? __float_as_uint(v) : 0u) << 32) | key[j];
+        }
+#pragma unroll
+        for (int w = 1; w < JM; w *= 2)
+#pragma unroll
+            for (int j = 0; j + w < JM; j += 2 * w) best[j] = best[j + w] > best[j] ? best[j + w] : best[j];
+        const uint32_t bhi = (uint32_t)(best[0] >> 32), blo = (uint32_t)best[0];
+        uint32_t whi = __reduce_max_sync(FULL, bhi);
+        uint32_t wlo = __reduce_max_sync(FULL, bhi == whi ? blo : 0u);
+        if (WPA > 1) {
+            uint2 *red = reinterpret_cast<uint2 *>(smem + L.red) + (size_t)(slot * 2 + (step & 1)) * WPA;
+            if (lane == 0) red[wsl] = make_uint2(whi, wlo);
+            named_barrier(1 + slot, TPA);
+            const uint2 o = red[lane & (WPA - 1)];
+            whi = __reduce_max_sync(FULL, o.x);
+            wlo = __reduce_max_sync(FULL, o.x == whi ? o.y : 0u);
+        }
+        step++;
+        int nxt = 0;
+        ext = whi != 0u;
+        if (!ext) { // no candidate: back to the depot (kernel.cl:461-465)
+            load = 0;
+        } else {
+            nxt = (int)(wlo & 0xFFFFu);
+            load += s_dem[nxt];
+            if (FIN) pend = __ldg(drow + nxt);
+            vcnt++;
+            if ((nxt & (TPA - 1)) == t) vis |= 1u << (nxt / TPA);
+        }
+        if (t == 0) tbuf[step] = (uint16_t)nxt;
+        load_row(nxt);
+    }
+
+    int *tour = a.solutions + (size_t)ant * a.T;
+    if (err) {
+        if (t == 0) {
+            tour[a.T - 1] = 0;
+            a.lens[ant] = __int_as_float(0x7f800000);
+            set_status(a.status, err);
+        }
+    } else { // kernel.cl:482-488
+        const int size = step + 2;
+        if (t == 0) tbuf[step + 1] = 0;
+        if (WPA > 1) named_barrier(1 + slot, TPA);
+        else __syncwarp();
+        for (int q = t; q < size; q += TPA) tour[q] = tbuf[q];
+        if (wsl == 0) { // tour_dist: the edges in step order, four chunks of 32 in flight before their sums
+            float tdist = 0.f;
+            for (int b0 = 0; b0 < size - 1; b0 += 128) {
+                float e[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int q = b0 + 32 * c + lane;
+                    e[c] = q < size - 1 ? __ldg(a.dist + (size_t)tbuf[q] * ld + tbuf[q + 1]) : 0.f;
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int m = size - 1 - (b0 + 32 * c);
+#pragma unroll
+                    for (int k = 0; k < 32; k++) {
+                        const float x = __shfl_sync(FULL, e[c], k);
+                        if (k < m) tdist = __fadd_rn(tdist, x);
+                    }
+                }
+            }
+            if (lane == 0) {
+                tour[a.T - 1] = size;
+                a.lens[ant] = tdist;
+            }
+        }
+    }
+    if (step > 0) { // rnd_seeds[gid] = rnd_seed (kernel.cl:492) for every lane that drew
+        const uint32_t inv_hi = pm_pow16807((long long)kPM - 1 - a.kmax), inv_lo = pm_pow16807((long long)kPM - a.kmax);
+#pragma unroll
+        for (int j = 0; j < JM; j++) {
+            const int i = t + TPA * j;
+            if (i < n && i + a.nloc >= n) seeds[i & lmask] = (int)pm_mul(y[j], (i & lmask) < more ? inv_hi : inv_lo);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Throughput mode.  A persistent kernel: each CTA pulls work items (instance,
 // group of `apc` ants) from a device queue, stages the instance's demand,
@@ -1071,9 +1312,31 @@ __global__ void __launch_bounds__(512, 1) construct_nn_draw_kernel(const Constru
     construct_nn_body<FIN, 1>(args, items, n_items, queue, apc, lsw, lens_later != 0);
 }
 
+// Nodes a thread: up to 16 the register kernel, beyond it the shared-memory one.
+constexpr int kParityRegNodes = 16;
+
+template <int WPA, int JM, bool FIN, bool SMAT>
+cudaError_t launch_parity_regs(const ConstructArgs &a, int apc, cudaStream_t st)
+{
+    const size_t bytes = parity_regs_layout(a.n, WPA, apc, SMAT).bytes;
+    auto kern = construct_parity_regs_kernel<WPA, JM, FIN, SMAT>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    kern<<<(a.n_ants + apc - 1) / apc, apc * 32 * WPA, bytes, st>>>(a);
+    return cudaGetLastError();
+}
+
 template <int WPA, bool FIN, bool SMAT>
 cudaError_t launch_parity_t(const ConstructArgs &a, int apc, cudaStream_t st)
 {
+    const int J = (a.n + 32 * WPA - 1) / (32 * WPA);
+    if (J <= 1) return launch_parity_regs<WPA, 1, FIN, SMAT>(a, apc, st);
+    if (J <= 2) return launch_parity_regs<WPA, 2, FIN, SMAT>(a, apc, st);
+    if (J <= 3) return launch_parity_regs<WPA, 3, FIN, SMAT>(a, apc, st);
+    if (J <= 4) return launch_parity_regs<WPA, 4, FIN, SMAT>(a, apc, st);
+    if (J <= 6) return launch_parity_regs<WPA, 6, FIN, SMAT>(a, apc, st);
+    if (J <= 8) return launch_parity_regs<WPA, 8, FIN, SMAT>(a, apc, st);
+    if (J <= kParityRegNodes) return launch_parity_regs<WPA, kParityRegNodes, FIN, SMAT>(a, apc, st);
     const ParityLayout L = parity_layout(a.n, a.nloc, a.kmax, WPA, apc, SMAT);
     auto kern = construct_parity_kernel<WPA, FIN, SMAT>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes);
@@ -1095,6 +1358,7 @@ cudaError_t launch_parity_w(const ConstructArgs &a, int apc, bool smat, cudaStre
 
 size_t construct_parity_smem(int n, int nloc, int kmax, int wpa, int apc, bool stage_total, bool)
 {
+    if ((n + 32 * wpa - 1) / (32 * wpa) <= kParityRegNodes) return parity_regs_layout(n, wpa, apc, stage_total).bytes;
     return parity_layout(n, nloc, kmax, wpa, apc, stage_total).bytes;
 }
 
