@@ -149,8 +149,24 @@ int prep_instance(const InstanceSpec &sp, const aco_params &p, InstHost &ih)
         int depth = std::max(ih.nn_ls, ih.K);
         if (depth >= n) depth = n - 1;
         ih.depth = std::max(depth, 0);
+        // coordinates this small have finite distances, whatever the formula
+        for (int i = 0; i < n && ih.finite; i++) ih.finite = std::fabs(sp.x[i]) < 1e18f && std::fabs(sp.y[i]) < 1e18f;
     } else {
         ih.depth = compute_nn_lists(n, ih.dist.data(), ih.nn_ls, ih.K, ih.nn);
+        const float *d = ih.dist.data();
+        for (size_t e = 0; e < (size_t)n * n && ih.finite; e++) ih.finite = std::isfinite(d[e]);
+        for (int i = 0; i < n && ih.sym; i++)
+            for (int j = 0; j < i && ih.sym; j++) ih.sym = d[(size_t)i * n + j] == d[(size_t)j * n + i];
+        // the last listed distance of every node, and whether unlisted nodes are as far
+        ih.nnr.assign(n, make_float2(0.f, 0.f));
+        for (int i = 0; i < n && ih.nn_ls > 0; i++) {
+            const int *list = ih.nn.data() + (size_t)i * ih.depth;
+            const float last = d[(size_t)i * n + list[ih.nn_ls - 1]];
+            int all = 0, listed = 0;
+            for (int j = 1; j < n; j++) all += j != i && d[(size_t)i * n + j] == last;
+            for (int h = 0; h < ih.nn_ls; h++) listed += d[(size_t)i * n + list[h]] == last;
+            ih.nnr[i] = make_float2(last, all != listed ? 1.f : 0.f);
+        }
     }
     return ACO_OK;
 }
@@ -315,7 +331,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         return o;
     };
     struct Offs {
-        size_t dist, heur, tau, total, chc, dem, key, jump, adv, cand32, nn16, nnls, seeds, sol, elites, succ,
+        size_t dist, heur, tau, total, chc, dem, key, jump, adv, cand32, nn16, nnls, nnr, seeds, sol, elites, succ,
             dep, dtau, rec, nbsf, iter, xy;
     };
     std::vector<Offs> offs(count);
@@ -332,6 +348,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         o.cand32 = take((size_t)ih.n * ih.Kp * 4);
         o.nn16 = take((size_t)ih.n * ih.Kp * 2);
         o.nnls = take((size_t)ih.n * std::max(1, ih.nn_ls) * 4);
+        o.nnr = take((size_t)ih.n * sizeof(float2));
         o.seeds = take((size_t)ih.A * ih.nloc * 4);
         o.sol = take(((size_t)ih.T * (ih.A + 1) + 1) * 4);
         o.elites = take((size_t)ih.R * 4);
@@ -389,13 +406,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
             for (int i = 1; i < ih.n; i++) dem += ih.demand[i];
             const long long per = ih.capacity > 0 ? 2 * ((dem + ih.capacity - 1) / ih.capacity) + 16 : ih.n - 1;
             cap += (long long)ih.A * std::min<long long>(ih.n - 1, per);
-            if (!ih.device_prep) // coordinate formulas are symmetric; a given matrix is checked
-                for (int i = 0; i < ih.n && sym; i++)
-                    for (int j = 0; j < i; j++)
-                        if (ih.dist[(size_t)i * ih.n + j] != ih.dist[(size_t)j * ih.n + i]) {
-                            sym = false;
-                            break;
-                        }
+            sym = sym && ih.sym; // coordinate formulas are symmetric; a given matrix was checked
         }
         // measured: with few ants per SM the per-ant kernel is as fast (the slowest
         // route sets the time either way) and the list costs the construct a pass
@@ -427,6 +438,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         ih.key_d = (uint32_t *)(base + o.key); ih.jump_d = (uint32_t *)(base + o.jump);
         ih.adv_d = (uint32_t *)(base + o.adv); ih.cand32_d = (uint32_t *)(base + o.cand32);
         ih.nn16_d = (uint16_t *)(base + o.nn16); ih.nnls_d = (int *)(base + o.nnls);
+        ih.nnr_d = (float2 *)(base + o.nnr);
         ih.seeds_d = (int *)(base + o.seeds); ih.sol_d = (int *)(base + o.sol);
         ih.lens_d = (float *)(base + o_lens_all) + slot_base_h_[b]; ih.elites_d = (int *)(base + o.elites);
         ih.succ_d = (int *)(base + o.succ); ih.dep_d = (uint32_t *)(base + o.dep);
@@ -547,8 +559,12 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         };
         cn_lsw = 0;
         int n_max = 0;
-        for (const InstHost &ih : inst) n_max = std::max(n_max, ih.n);
-        if ((p.ls_flag & 1) && p.fuse_ls == 1 && n_max <= 1024) { // 2-opt fused into the construct
+        bool finite = true;
+        for (const InstHost &ih : inst) {
+            n_max = std::max(n_max, ih.n);
+            finite = finite && ih.finite;
+        }
+        if ((p.ls_flag & 1) && p.fuse_ls == 1 && n_max <= 1024 && finite) { // 2-opt fused into the construct
             // at most 4 constructing ants per CTA, the other warps (up to 16) improve
             // routes, so completed routes do not queue
             for (int apc = std::min(cn_apc, 4); apc >= 1 && cn_lsw == 0; apc--) {
@@ -696,7 +712,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         pa.n = n; pa.ld = ih.ld; pa.depth = ih.depth; pa.K = ih.K; pa.Kp = ih.Kp; pa.nn_ls = ih.nn_ls;
         pa.dist_type = ih.dist_type; pa.device_prep = ih.device_prep ? 1 : 0; pa.n_ants = ih.A;
         pa.x = ih.xy_d; pa.y = ih.xy_d ? ih.xy_d + ih.n4 : nullptr; pa.dist = ih.dist_d; pa.demand = ih.dem_d;
-        pa.nn16 = ih.nn16_d; pa.cand32 = ih.cand32_d; pa.nnls = ih.nnls_d; pa.seeds = ih.seeds_d;
+        pa.nn16 = ih.nn16_d; pa.cand32 = ih.cand32_d; pa.nnls = ih.nnls_d; pa.nnr = ih.nnr_d; pa.seeds = ih.seeds_d;
         if (ih.device_prep) {
             n_prep = std::max(n_prep, n);
         } else {
@@ -733,6 +749,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
             for (int i = 0; i < n; i++)
                 for (int j = 0; j < ih.nn_ls; j++) nnls[(size_t)i * ih.nn_ls + j] = ih.nn[(size_t)i * ih.depth + j];
             up(ih.nnls_d, nnls.data(), nnls.size() * 4);
+            up(ih.nnr_d, ih.nnr.data(), ih.nnr.size() * sizeof(float2));
         }
 
         ConstructArgs &c = cargs_h_[b];
@@ -742,7 +759,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         c.total = ih.total_d; c.dist = ih.dist_d; c.demand = ih.dem_d; c.tiekey = ih.key_d; c.jump = ih.jump_d;
         c.adv = ih.adv_d; c.nn16 = ih.nn16_d; c.cand32 = ih.cand32_d; c.chc = ih.chc_d; c.K = ih.K; c.Kp = ih.Kp;
         c.smat = ih.smat ? 1 : 0; c.packed = ih.packed ? 1 : 0; c.gtab = ih.gtab ? 1 : 0;
-        c.nn_list = ih.nnls_d; c.nn_ls = ih.nn_ls; c.pass_limit = p.ls_pass_limit; c.ant_base = ant_base[b];
+        c.nn_list = ih.nnls_d; c.nnr = ih.nnr_d; c.nn_ls = ih.nn_ls; c.pass_limit = p.ls_pass_limit; c.ant_base = ant_base[b];
         c.ls_best = p.ls_best;
         c.ls_needed = ls_needed_d_;
         c.route_desc = use_routes_ ? route_desc_d_ : nullptr;
@@ -757,6 +774,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         l = LocalSearchArgs{};
         l.n = n; l.ld = ih.ld; l.n_ants = ih.A; l.T = ih.T; l.nn_ls = ih.nn_ls; l.rmax = 32;
         l.pass_limit = p.ls_pass_limit; l.dist = ih.dist_d; l.nn_list = ih.nnls_d; l.solutions = ih.sol_d;
+        l.nnr = ih.nnr_d; l.sym = ih.sym ? 1 : 0; l.generic = ih.finite ? 0 : 1;
         l.best = p.ls_best;
         l.lens = ih.lens_d; l.status = status_d;
         StatsArgs &s = sargs[b];
@@ -799,6 +817,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
     for (InstHost &ih : inst) { // the host copies are no longer needed
         std::vector<int>().swap(ih.nn);
         std::vector<float>().swap(ih.dist);
+        std::vector<float2>().swap(ih.nnr);
         ih.x = ih.y = nullptr;
     }
     return sync_status();

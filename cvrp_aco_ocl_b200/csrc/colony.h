@@ -37,6 +37,9 @@ struct InstHost {
     uint64_t data_hash = 0;  // FNV-1a of the instance's data (checkpoint identity)
     uint64_t prior_hash = 0; // of the prior set by set_prior (0: none)
     bool smat = false, packed = false, gtab = false;
+    bool finite = true;                    // every distance is finite
+    bool sym = true;                       // and symmetric
+    std::vector<float2> nnr;               // host preparation: see LocalSearchArgs
     bool device_prep = false;              // distances and lists computed on the device
     const float *x = nullptr, *y = nullptr; // caller's coordinates (valid during create)
     int dist_type = 0;
@@ -50,6 +53,7 @@ struct InstHost {
     int *succ_d = nullptr, *nbsf_d = nullptr, *iter_d = nullptr;
     uint32_t *key_d = nullptr, *jump_d = nullptr, *adv_d = nullptr, *cand32_d = nullptr, *dep_d = nullptr;
     uint16_t *nn16_d = nullptr;
+    float2 *nnr_d = nullptr;
     float *xy_d = nullptr; // device preprocessing: coordinates (x, then y at n4)
     float *lens_d = nullptr, *dtau_d = nullptr;
     aco_record *rec_d = nullptr;

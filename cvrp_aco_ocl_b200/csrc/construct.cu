@@ -483,21 +483,20 @@ __global__ void __launch_bounds__(512) construct_parity_regs_kernel(ConstructArg
 //     step, in step order.
 // ---------------------------------------------------------------------------
 struct NNLayout {
-    size_t bar, dem, d0, cand, chc, vis, tour, mat, rid, li, dt, pend, cnt, q, ready, ls, ring, flag, bytes;
+    size_t bar, dem, d0, cand, chc, vis, tour, mat, dt, pend, cnt, q, ready, ls, ring, flag, bytes;
     int qcap;
 };
 
 // Helper-warp draws: steps per hand-over (the ring holds two such chunks per ant).
 constexpr int kDrawChunk = 16;
 
-// Shared memory of one 2-opt warp of the fused construct: distance tile,
-// in-route neighbour lists and counts, route node ids.
-constexpr size_t kLsWarpBytes = 32 * 32 * 4 + 32 * 32 + 32 + 64 + 32 * 32 * 2;
+// Shared memory of one 2-opt warp of the fused construct: distance tile, a byte a position.
+constexpr size_t kLsWarpBytes = 32 * 32 * 4 + 32;
 
 // gtab: the candidate table is read from global memory (L2) instead of being
 // staged (instances whose table does not fit next to the per-ant buffers).
-// lsw > 0: the fused 2-opt (lsw improving warps): per ant the route id and
-// local index of every node and the edge lengths, the route queue.
+// lsw > 0: the fused 2-opt (lsw improving warps): per ant the edge lengths, and
+// the route queue.
 __host__ __device__ inline NNLayout nn_layout(int n, int K, int Kp, int apc, bool smat, bool packed, bool gtab,
                                               int lsw = 0, bool draw = false)
 {
@@ -515,10 +514,8 @@ __host__ __device__ inline NNLayout nn_layout(int n, int K, int Kp, int apc, boo
     L.mat = o;
     if (smat) o = al128(o + (size_t)n * n4 * 4);
     L.qcap = apc * n + 64;
-    L.rid = L.li = L.dt = L.pend = L.cnt = L.q = L.ready = L.ls = o;
+    L.dt = L.pend = L.cnt = L.q = L.ready = L.ls = o;
     if (lsw > 0) {
-        L.rid = o; o = al128(o + (size_t)apc * n * 2);
-        L.li = o; o = al128(o + (size_t)apc * n);
         L.dt = o; o = al128(o + (size_t)apc * 2 * n * 4);
         L.pend = o; o = al128(o + (size_t)2 * apc * 4); // pending routes, deferred flag
         L.cnt = o; o = al128(o + 4 * 4);                // slots allocated, tickets, construct warps done
@@ -556,10 +553,7 @@ __device__ void fused_ls_warp(const ConstructArgs &a, unsigned char *smem, const
     const int *ready = reinterpret_cast<const int *>(smem + L.ready);
     unsigned char *w = smem + L.ls + (size_t)lsw_index * kLsWarpBytes;
     float *tile = reinterpret_cast<float *>(w);
-    uint8_t *lnn = w + 32 * 32 * 4;
-    uint8_t *lcnt = lnn + 32 * 32;
-    uint16_t *rnode = reinterpret_cast<uint16_t *>(lcnt + 32);
-    uint16_t *nnbuf = rnode + 32;
+    uint8_t *tpos = w + 32 * 32 * 4;
     int status = ACO_OK;
     for (;;) {
         int t = 0, state = 0; // state: 1 route ready, 2 nothing left, 3 timed out
@@ -584,44 +578,18 @@ __device__ void fused_ls_warp(const ConstructArgs &a, unsigned char *smem, const
         const int2 e = make_int2(qe[0], qe[1]);
         const int j = e.x & 0xff, r = e.x >> 8, rb = e.y & 0xffff, R = e.y >> 16;
         uint16_t *tb = reinterpret_cast<uint16_t *>(smem + L.tour) + (size_t)j * 2 * n;
-        const uint16_t *rid = reinterpret_cast<const uint16_t *>(smem + L.rid) + (size_t)j * n;
-        const uint8_t *li = reinterpret_cast<const uint8_t *>(smem + L.li) + (size_t)j * n;
         float *dt = reinterpret_cast<float *>(smem + L.dt) + (size_t)j * 2 * n;
         if (R > kRL) { // longer routes: the whole ant goes to the 2-opt kernel
             if (lane == 0) pend[apc + j] = 1;
         } else {
-            // route-local state, as the 2-opt kernel builds it (local_search.cu)
+            // as the 2-opt kernels (local_search.cu)
             const int v = lane < R ? (int)tb[rb + lane] : 0;
-            if (lane < R) rnode[lane] = (uint16_t)v;
-            __syncwarp();
-#pragma unroll 8
-            for (int x = lane; x < R * kRL; x += 32) {
-                const int k1 = x >> 5, k2 = x & 31;
-                tile[x] = k2 < R ? __ldg(a.dist + (size_t)rnode[k1] * a.ld + rnode[k2]) : 0.f;
-                nnbuf[x] = k2 < a.nn_ls ? (uint16_t)__ldg(a.nn_list + (size_t)rnode[k1] * a.nn_ls + k2) : 0;
-            }
-            __syncwarp();
-            for (int k = 0; k < R; k++) {
-                const int node = rnode[k];
-                int c = 0;
-                for (int h0 = 0; h0 < a.nn_ls && c < R - 1; h0 += 32) {
-                    const int h = h0 + lane;
-                    const int n2 = h >= a.nn_ls ? 0
-                                   : h0 == 0 ? (int)nnbuf[k * kRL + lane]
-                                             : __ldg(a.nn_list + (size_t)node * a.nn_ls + h);
-                    const bool in = h < a.nn_ls && n2 != 0 && rid[n2] == r;
-                    const unsigned m = __ballot_sync(kFullMask, in);
-                    const int slot = c + __popc(m & ((1u << lane) - 1u));
-                    if (in && slot < kRL) lnn[k * kRL + slot] = li[n2];
-                    c += __popc(m);
-                }
-                if (lane == 0) lcnt[k] = (uint8_t)(c < R - 1 ? c : R - 1);
-            }
-            __syncwarp();
-            int tq = lane < R ? lane : 0, pk = lane < R ? lane : 0;
+            const uint32_t nm = route_tile<8>(lane, R, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, tile);
+            int tq = lane < R ? lane : 0;
             float dq = lane < R ? tile[lane * kRL + (lane + 1 < R ? lane + 1 : 0)] : 0.f; // dist_tour_wrk
-            const int st = a.ls_best ? two_opt_route_best(lane, R, tile, lnn, tq, pk, dq, a.pass_limit)
-                                     : two_opt_route_regs(lane, R, r == 0, tile, lnn, lcnt, tq, pk, dq, a.pass_limit);
+            const int st = a.ls_best ? two_opt_route_best(lane, R, tile, tpos, tq, dq, a.pass_limit)
+                                     : two_opt_route_regs<false>(lane, R, r == 0, tile, nm, v, a.nn_list, a.nn_ls, tq,
+                                                                 dq, a.pass_limit);
             if (st != ACO_OK) status = st;
             const int node = __shfl_sync(kFullMask, v, tq);
             if (lane < R) {
@@ -934,8 +902,6 @@ __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int ap
     if (FIN)
         for (int i = threadIdx.x; i < n; i += blockDim.x) s_d0[i] = a.dist[(size_t)i * ld];
     if (LSF) { // fused 2-opt bookkeeping starts empty for this item
-        uint16_t *rid_all = reinterpret_cast<uint16_t *>(smem + L.rid);
-        for (int i = threadIdx.x; i < apc * n; i += blockDim.x) rid_all[i] = 0xFFFFu;
         int *ready_all = reinterpret_cast<int *>(smem + L.ready);
         for (int i = threadIdx.x; i < L.qcap; i += blockDim.x) ready_all[i] = 0;
         int *pend_all = reinterpret_cast<int *>(smem + L.pend);
@@ -988,10 +954,7 @@ __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int ap
     };
     if (warp < apc && ant < a.n_ants) {
         uint16_t *tbuf = s_tour + warp * 2 * n;
-        uint16_t *f_rid = reinterpret_cast<uint16_t *>(smem + L.rid) + (size_t)warp * n;
-        uint8_t *f_li = reinterpret_cast<uint8_t *>(smem + L.li) + (size_t)warp * n;
         int f_rb = 0, f_r = 0;
-        (void)f_rid; (void)f_li;
         uint32_t *vism = s_vis + warp * words;
         uint32_t vis = lane == 0 ? 1u : 0u; // register visited set (REGVIS): node 0 = lane 0, bit 0
         if (!REGVIS) {
@@ -1093,12 +1056,7 @@ __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int ap
             if (!DRAW && nxt != 0 && nd == mind) mcnt--; // one customer of the smallest demand fewer
             if (lane == 0) tbuf[step] = (uint16_t)nxt;
             if (LSF) {
-                if (nxt != 0) {
-                    if (lane == 0) {
-                        f_rid[nxt] = (uint16_t)f_r;
-                        f_li[nxt] = (uint8_t)(step - f_rb < 256 ? step - f_rb : 0);
-                    }
-                } else { // back at the depot: the route [f_rb, step) is complete
+                if (nxt == 0) { // back at the depot: the route [f_rb, step) is complete
                     publish(f_r, f_rb, step - f_rb);
                     f_r++;
                     f_rb = step;

@@ -45,6 +45,7 @@ struct ConstructArgs {
     // fused 2-opt (throughput construct with improving warps): the 2-opt lists, the
     // pass limit, and per global ant whether the 2-opt kernel still has to run
     const int *nn_list;    // n x nn_ls
+    const float2 *nnr;     // n: see LocalSearchArgs
     int nn_ls, pass_limit, ant_base;
     int ls_best;           // the fused 2-opt improves best-first (aco_params.ls_best)
     uint8_t *ls_needed;    // total ants of the colony
@@ -72,6 +73,9 @@ struct LocalSearchArgs {
     int best;              // 1: best-improvement 2-opt for routes of at most 32 nodes (aco_params.ls_best)
     const float *dist;     // n x ld
     const int *nn_list;    // n x nn_ls
+    const float2 *nnr;     // n: distance of the list's last entry; 1 if unlisted nodes are as far, else 0
+    int sym;               // symmetric distances
+    int generic;           // distances that are not all finite: every route takes the list-scanning paths
     int *solutions;
     float *lens;
     int *status;
@@ -235,6 +239,7 @@ struct PrepArgs {
     uint16_t *nn16;   // n x Kp: first K of the list, padded with node 0
     uint32_t *cand32; // n x Kp: the same with the demand in the high half
     int *nnls;        // n x nn_ls: the 2-opt list
+    float2 *nnr;      // n: the 2-opt list's last distance (LocalSearchArgs)
     int *seeds;       // n_ants x nloc
 };
 // Every instance of a batch in one launch per step (global row g: row g -

@@ -18,17 +18,10 @@
 // local_search_kernel: CTAs of 1-8 ants whose warps pull the routes of all of
 // them from a shared counter, longest first; route_opt_kernel: a persistent
 // grid over the construct's list of every ant's routes (see below).  A route of
-// at most 32 nodes (depot included) runs entirely in one warp's registers: lane q
-// holds the local node at route position q, its edge length, and the position
-// of local node q; the don't-look bits are one warp-uniform mask; the route's
-// distance sub-matrix is a 32x32 shared tile; and every node's neighbour list
-// is pre-filtered to the neighbours inside the route, in list order.  The scan
-// of kernel.cl:180-230 only ever stops on an in-route entry (others `continue`),
-// so the filtered list visits exactly the entries that decide the outcome: the
-// first that ends the scan (radius test fails) or improves, found with ballot +
-// find-first-set.  A move reverses a position range with shuffles.  Longer
-// routes take the generic path over shared-memory arrays and the L2-resident
-// distance matrix.
+// at most 32 nodes (depot included) runs entirely in one warp's registers
+// (two_opt.cuh); longer ones, and all routes of an instance whose distances are
+// not all finite, take the list-scanning paths over shared-memory arrays and the
+// L2-resident distance matrix.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -69,8 +62,8 @@ __host__ __device__ inline LsAnt ls_ant_layout(int n)
     return L;
 }
 
-// per warp: distance tile, in-route neighbour lists (local indices), list counts
-constexpr size_t kLsWarp = kRL * kRL * 4 + kRL * kRL + kRL;
+// per warp: distance tile, a byte a position (best improvement)
+constexpr size_t kLsWarp = kRL * kRL * 4 + kRL;
 constexpr int kLsRows = 8; // tile rows loaded per round
 constexpr int kMaxLsAnts = 8;
 constexpr int kLsOrder = 128; // routes of a CTA ordered longest first when at most this many
@@ -307,8 +300,7 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
     const LsAnt AL = ls_ant_layout(n_max);
     unsigned char *wbase = smem + (size_t)apc * AL.bytes + (size_t)warp * kLsWarp;
     float *tile = reinterpret_cast<float *>(wbase);
-    uint8_t *lnn = wbase + kRL * kRL * 4;
-    uint8_t *lcnt = lnn + kRL * kRL;
+    uint8_t *tpos = wbase + kRL * kRL * 4;
     auto ant_ptr = [&](int j, size_t off) { return smem + (size_t)j * AL.bytes + off; };
     __shared__ int s_group;
     const int listed = list ? min(list_ctr[0], total_ants) : 0;
@@ -448,60 +440,23 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
         float *dt = reinterpret_cast<float *>(ant_ptr(j, AL.dt));
         const int rb = rstart[r], re = rstart[r + 1] - 1, R = re - rb + 1;
         int st = ACO_OK;
-        if (R <= kRL && s_only[j] == 1) {
+        const bool small = R <= kRL && (a.best || !a.generic); // best improvement reads no list
+        if (small && s_only[j] == 1) {
             // routes of at most 32 nodes improved already (fused construct or
             // route-level kernel); only the longer ones of this ant are left
             // here.  Their edge lengths still enter the tour length.
             for (int p = rb + lane; p <= re; p += 32) dt[p] = __ldg(a.dist + (size_t)tour[p] * a.ld + tour[p + 1]);
-        } else if (R <= kRL) {
-            // route-local state: the distance tile (row k1 = distances from route
-            // node k1, lane k2 its column) and every route node's neighbour list
-            // filtered to the route, in list order.  Lane q holds route node q; row
-            // nodes come by shuffle, so the loads of a round of kLsRows rows depend
-            // on nothing in shared memory and are all in flight together.
+        } else if (small) {
+            // lane q holds route node q
             const int v = lane < R ? (int)tour[rb + lane] : 0;
-            for (int k0 = 0; k0 < R; k0 += kLsRows) {
-                float d[kLsRows];
-                int nb[kLsRows];
-#pragma unroll
-                for (int u = 0; u < kLsRows; u++) {
-                    const int k1 = k0 + u;
-                    const int node1 = __shfl_sync(FULL, v, k1 & 31);
-                    d[u] = (k1 < R && lane < R) ? __ldg(a.dist + (size_t)node1 * a.ld + v) : 0.f;
-                    nb[u] = (k1 < R && lane < a.nn_ls) ? __ldg(a.nn_list + (size_t)node1 * a.nn_ls + lane) : 0;
-                }
-#pragma unroll
-                for (int u = 0; u < kLsRows; u++) {
-                    const int k1 = k0 + u;
-                    if (k1 >= R) break; // warp-uniform
-                    tile[k1 * kRL + lane] = d[u];
-                    const int n2 = nb[u];
-                    const bool in = n2 != 0 && rid[n2] == r;
-                    const unsigned m = __ballot_sync(FULL, in);
-                    const int slot = __popc(m & ((1u << lane) - 1u));
-                    if (in && slot < kRL) lnn[k1 * kRL + slot] = li[n2];
-                    int cnt = __popc(m);
-                    // lists deeper than 32: the rest while the route may still gain entries
-                    const int node1 = __shfl_sync(FULL, v, k1 & 31);
-                    for (int h0 = 32; h0 < a.nn_ls && cnt < R - 1; h0 += 32) {
-                        const int h = h0 + lane;
-                        const int n3 = h < a.nn_ls ? __ldg(a.nn_list + (size_t)node1 * a.nn_ls + h) : 0;
-                        const bool in3 = n3 != 0 && rid[n3] == r;
-                        const unsigned m3 = __ballot_sync(FULL, in3);
-                        const int slot3 = cnt + __popc(m3 & ((1u << lane) - 1u));
-                        if (in3 && slot3 < kRL) lnn[k1 * kRL + slot3] = li[n3];
-                        cnt += __popc(m3);
-                    }
-                    if (lane == 0) lcnt[k1] = (uint8_t)(cnt < R - 1 ? cnt : R - 1);
-                }
-            }
-            __syncwarp();
+            const uint32_t nm = route_tile<kLsRows>(lane, R, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, tile);
             int tq = lane < R ? lane : 0;
-            int pk = lane < R ? lane : 0;
             // edge lengths: position q -> q+1, the last one back to the next depot (node 0 = local 0)
             float dq = lane < R ? tile[lane * kRL + (lane + 1 < R ? lane + 1 : 0)] : 0.f;
-            st = a.best ? two_opt_route_best(lane, R, tile, lnn, tq, pk, dq, a.pass_limit)
-                        : two_opt_route_regs(lane, R, r == 0, tile, lnn, lcnt, tq, pk, dq, a.pass_limit);
+            st = a.best  ? two_opt_route_best(lane, R, tile, tpos, tq, dq, a.pass_limit)
+                 : a.sym ? two_opt_route_regs<true>(lane, R, r == 0, tile, nm, v, a.nn_list, a.nn_ls, tq, dq, a.pass_limit)
+                         : two_opt_route_regs<false>(lane, R, r == 0, tile, nm, v, a.nn_list, a.nn_ls, tq, dq,
+                                                     a.pass_limit);
             const int node = __shfl_sync(FULL, v, tq);
             if (lane < R) {
                 tour[rb + lane] = (uint16_t)node;
@@ -572,16 +527,16 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
 // most 255 nodes) is one entry of the list the construct kernel wrote, and the
 // warps of a persistent grid take entries from a counter, so the routes of
 // one ant spread over all SMs instead of queueing in one CTA.  A route needs
-// no state of its ant beyond its own nodes: its membership test is a per-warp
-// node -> local index map in shared memory, set for the route and cleared
-// after it.  Routes of at most 32 nodes run in registers (two_opt.cuh), longer
-// ones through two_opt_route_local.  The warp that improves an ant's last listed route sums the ant's
+// no state of its ant beyond its own nodes.  Routes of at most 32 nodes run in
+// registers (two_opt.cuh), longer ones through two_opt_route_local, whose
+// membership test is a per-warp node -> local index map in shared memory, set for
+// the route and cleared after it.  The warp that improves an ant's last listed route sums the ant's
 // tour length (kernel.cl:534-538) from the distances of its final tour edges,
 // which equal the 2-opt's edge lengths for a symmetric matrix (the only case
 // this kernel is used for); ants flagged for the per-ant kernel get their
 // length there.
 // ---------------------------------------------------------------------------
-constexpr int kRouteRows = 4; // tile rows loaded per round (register budget of two CTAs per SM)
+constexpr int kRouteRows = 8; // tile rows loaded per round
 
 // Routes of 33..255 nodes in the route-level kernel: kernel.cl:126-277 with
 // the route's state in the warp's shared memory (the area of the register
@@ -777,7 +732,7 @@ __device__ int two_opt_route_local(int lane, int R, const float *dist, int ld, c
 
 __host__ __device__ inline size_t route_warp_bytes(int n_max)
 {
-    return kRL * kRL * 4 + kRL * kRL + kRL + al16((size_t)n_max);
+    return kRL * kRL * 4 + kRL + al16((size_t)n_max);
 }
 
 __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs *args, const int *ant_inst,
@@ -788,9 +743,8 @@ __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *wbase = smem + (size_t)warp * route_warp_bytes(n_max);
     float *tile = reinterpret_cast<float *>(wbase);
-    uint8_t *lnn = wbase + kRL * kRL * 4;
-    uint8_t *lcnt = lnn + kRL * kRL;
-    uint8_t *loc = lcnt + kRL; // node -> local index (0: not in the route)
+    uint8_t *tpos = wbase + kRL * kRL * 4;
+    uint8_t *loc = tpos + kRL; // node -> local index (0: not in the route; longer routes only)
     for (int i = lane; i < n_max; i += 32) loc[i] = 0;
     __syncwarp();
     const int total = min(ctr[0], cap);
@@ -805,7 +759,7 @@ __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs
         const int b = __ldg(ant_inst + g), ant = g - __ldg(ant_base + b);
         const LocalSearchArgs a = args[b];
         int *gt = a.solutions + (size_t)ant * a.T;
-        if (R > kRL) { // 33..255 nodes: the route-local generic path in the warp's tile area
+        if (R > kRL || (a.generic && !a.best)) { // the route-local generic path in the warp's tile area
             uint16_t *nodes = reinterpret_cast<uint16_t *>(wbase);
             uint8_t *tk = wbase + 512, *pk = tk + 256, *dlb = pk + 256;
             float *dq = reinterpret_cast<float *>(wbase + 1280);
@@ -828,52 +782,16 @@ __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs
             __syncwarp();
         } else {
         const int v = lane < R ? gt[rb + lane] : 0;
-        if (lane >= 1 && lane < R) loc[v] = (uint8_t)lane; // customers only (kernel.cl:293-300)
-        __syncwarp();
-        for (int k0 = 0; k0 < R; k0 += kRouteRows) {
-            float dd[kRouteRows];
-            int nb[kRouteRows];
-#pragma unroll
-            for (int u = 0; u < kRouteRows; u++) {
-                const int k1 = k0 + u;
-                const int node1 = __shfl_sync(FULL, v, k1 & 31);
-                dd[u] = (k1 < R && lane < R) ? __ldg(a.dist + (size_t)node1 * a.ld + v) : 0.f;
-                nb[u] = (k1 < R && lane < a.nn_ls) ? __ldg(a.nn_list + (size_t)node1 * a.nn_ls + lane) : 0;
-            }
-#pragma unroll
-            for (int u = 0; u < kRouteRows; u++) {
-                const int k1 = k0 + u;
-                if (k1 >= R) break; // warp-uniform
-                tile[k1 * kRL + lane] = dd[u];
-                const int n2 = nb[u];
-                const int l2 = n2 != 0 ? loc[n2] : 0;
-                const unsigned m = __ballot_sync(FULL, l2 != 0);
-                const int slot = __popc(m & ((1u << lane) - 1u));
-                if (l2 != 0 && slot < kRL) lnn[k1 * kRL + slot] = (uint8_t)l2;
-                int cnt = __popc(m);
-                const int node1 = __shfl_sync(FULL, v, k1 & 31);
-                for (int h0 = 32; h0 < a.nn_ls && cnt < R - 1; h0 += 32) { // lists deeper than 32
-                    const int h = h0 + lane;
-                    const int n3 = h < a.nn_ls ? __ldg(a.nn_list + (size_t)node1 * a.nn_ls + h) : 0;
-                    const int l3 = n3 != 0 ? loc[n3] : 0;
-                    const unsigned m3 = __ballot_sync(FULL, l3 != 0);
-                    const int slot3 = cnt + __popc(m3 & ((1u << lane) - 1u));
-                    if (l3 != 0 && slot3 < kRL) lnn[k1 * kRL + slot3] = (uint8_t)l3;
-                    cnt += __popc(m3);
-                }
-                if (lane == 0) lcnt[k1] = (uint8_t)(cnt < R - 1 ? cnt : R - 1);
-            }
-        }
-        __syncwarp();
+        const uint32_t nm = route_tile<kRouteRows>(lane, R, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, tile);
         // edge lengths: position q -> q+1, the last one back to the next depot (node 0 = local 0)
-        int tq = lane < R ? lane : 0, pk = lane < R ? lane : 0;
+        int tq = lane < R ? lane : 0;
         float dq = lane < R ? tile[lane * kRL + (lane + 1 < R ? lane + 1 : 0)] : 0.f;
-        const int st = a.best ? two_opt_route_best(lane, R, tile, lnn, tq, pk, dq, a.pass_limit)
-                              : two_opt_route_regs(lane, R, rb == 0, tile, lnn, lcnt, tq, pk, dq, a.pass_limit);
+        const int st = a.best ? two_opt_route_best(lane, R, tile, tpos, tq, dq, a.pass_limit)
+                              : two_opt_route_regs<true>(lane, R, rb == 0, tile, nm, v, a.nn_list, a.nn_ls, tq, dq,
+                                                         a.pass_limit);
         if (st != ACO_OK && lane == 0) set_status(a.status, st);
         const int node = __shfl_sync(FULL, v, tq);
         if (lane < R) __stcs(gt + rb + lane, node); // evict first: not read again before the statistics
-        if (lane >= 1 && lane < R) loc[v] = 0;
         __syncwarp();
         }
         __threadfence();

@@ -210,6 +210,15 @@ __global__ void lists_rows_kernel(const PrepArgs *pa, const int *row_base, const
             a.cand32[(size_t)i * a.Kp + j] = (uint32_t)c | ((uint32_t)(a.demand[c] & 0xFFFF) << 16);
         }
         for (int j = lane; j < a.nn_ls; j += 32) a.nnls[(size_t)i * a.nn_ls + j] = idx[j];
+        if (a.nn_ls > 0) { // the list's last distance, and whether unlisted nodes are as far
+            const float *row = a.dist + (size_t)i * a.ld;
+            const float last = row[idx[a.nn_ls - 1]];
+            int more = 0; // nodes at that distance, less the listed ones
+            for (int k = lane; k < n; k += 32) more += k != 0 && k != i && row[k] == last;
+            for (int j = lane; j < a.nn_ls; j += 32) more -= row[idx[j]] == last;
+            more = __reduce_add_sync(0xffffffffu, more);
+            if (lane == 0) a.nnr[i] = make_float2(last, more != 0 ? 1.f : 0.f);
+        }
         __syncwarp(); // the row's buffers are reused by the warp's next row
     }
 }

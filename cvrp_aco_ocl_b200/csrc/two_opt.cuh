@@ -1,14 +1,28 @@
 // two_opt.cuh -- the register path of the route 2-opt (first improvement in
 // sequence order with don't-look bits, kernel.cl:126-277) for routes of at most
-// 32 nodes, shared by the 2-opt kernel and the construct kernel that improves
+// 32 nodes, shared by the 2-opt kernels and the construct kernel that improves
 // routes while later ones are still being built.
 //
-// Lane q holds the local node at route position q (tq), the length of the edge
-// leaving position q (dq, dist_tour_wrk) and the position of local node q (pk);
-// the don't-look bits are one warp-uniform mask; `tile` is the route's 32x32
-// distance sub-matrix; lnn / lcnt are every local node's neighbour list
-// filtered to the route, in list order.  The scan only stops on in-route
-// entries, so the filtered lists decide exactly as the full ones.
+// Lane p holds everything about route position p: the local node there (tq), its
+// neighbours on the tour, the length of the edge leaving it (dq, dist_tour_wrk)
+// and the mask of the route nodes on its neighbour list.  An examination takes
+// the examined position's words by shuffle, and every lane evaluates its own
+// node as the move partner from its own registers and three entries of `tile`,
+// the route's 32x32 distance sub-matrix.
+//
+// The lists are sorted by distance, so the reference's scan (stop at the first
+// entry past the radius or improving) finds a move exactly when some listed
+// route node inside the radius improves, and takes the nearest of them; equal
+// distances are settled by the list itself.  No list is read otherwise: a node
+// is listed exactly when it is no farther than the list's last entry, whose
+// distance is kept per node (nnr), except where the list ends inside a group of
+// equal distances (flagged there, looked up).  Instances with distances that
+// are not finite do not come here.
+//
+// Warp instructions: about 45 an examination and 45 a move (90 and 75 with the
+// lists filtered into shared memory and the partner's words fetched by shuffle),
+// 10 a row to build the tile (60 with the list filtering).  512 instances, 2.9 M
+// routes of 14 nodes: 9.81 -> 6.58 ms; 201 ants with full lists: 74 -> 28 us.
 #pragma once
 
 #include <cstdint>
@@ -22,158 +36,147 @@ constexpr int kRL = 32; // largest route (nodes, depot included) of the register
 
 constexpr unsigned kFullMask = 0xffffffffu;
 
-// The 2-opt move that replaces edges (h1,h2) and (h3,h4) by (h1,h3) and (h2,h4)
-// (kernel.cl:235-270) on the lane-per-position state: the positions between
-// the two edges are reversed and dist_tour_wrk follows them.
-__device__ __forceinline__ void route_exchange(int lane, const float *tile, int h1, int h2, int h3, int h4, int &tq,
-                                               int &pk, float &dq)
+// The distance tile of a route and, as the return value of lane k, the mask of
+// the route's customers on the neighbour list of route node k (its own bit and
+// the depot's are never set).  Lane q < R holds route node q's global id (v); a
+// round of ROWS rows has its loads in flight together.
+template <int ROWS>
+__device__ __forceinline__ uint32_t route_tile(int lane, int R, int v, const float *dist, int ld, const float2 *nnr,
+                                               const int *nn, int nn_ls, float *tile)
 {
-    const unsigned FULLM = 0xffffffffu;
-    int p1 = __shfl_sync(FULLM, pk, h1), p3 = __shfl_sync(FULLM, pk, h3);
-    if (p3 < p1) {
-        int t = h1; h1 = h3; h3 = t;
-        t = h2; h2 = h4; h4 = t;
-        t = p1; p1 = p3; p3 = t;
+    const uint32_t cust = (R >= 32 ? kFullMask : (1u << R) - 1u) & ~1u;
+    float2 last = make_float2(-__int_as_float(0x7f800000), 0.f); // the list's last distance; 1: others share it
+    if (lane < R && nn_ls > 0) last = __ldg(nnr + v);
+    uint32_t nm = 0u;
+    for (int k0 = 0; k0 < R; k0 += ROWS) {
+        float d[ROWS];
+#pragma unroll
+        for (int u = 0; u < ROWS; u++) {
+            const int node1 = __shfl_sync(kFullMask, v, (k0 + u) & 31);
+            d[u] = (k0 + u < R && lane < R) ? __ldg(dist + (size_t)node1 * ld + v) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < ROWS; u++) {
+            const int k1 = k0 + u;
+            if (k1 >= R) break; // warp-uniform
+            tile[k1 * kRL + lane] = d[u];
+            const uint32_t m = __ballot_sync(kFullMask, d[u] <= __shfl_sync(kFullMask, last.x, k1));
+            if (lane == k1) nm = m & cust & ~(1u << k1);
+        }
     }
-    const int i = p1, jj = p3, a = __shfl_sync(FULLM, pk, h2);
-    const float d13 = tile[h1 * kRL + h3], d24 = tile[h2 * kRL + h4];
-    // dist_tour_wrk: [i] = d(h1,h3), [jj] = d(h2,h4), (i, jj) reversed
-    const float dsrc = __shfl_sync(FULLM, dq, (lane > i && lane < jj) ? i + jj - lane : lane);
-    if (lane == jj) dq = d24; // written after [i], as kernel.cl:249-250
-    else if (lane == i) dq = d13;
-    else if (lane > i && lane < jj) dq = dsrc;
-    // tour positions [a, jj] reversed; positions of the moved nodes mirrored
-    const int tsrc = __shfl_sync(FULLM, tq, (lane >= a && lane <= jj) ? a + jj - lane : lane);
-    if (lane >= a && lane <= jj) tq = tsrc;
-    if (pk >= a && pk <= jj) pk = a + jj - pk;
+    // lists that end inside a group of equal distances: look those route nodes up
+    for (uint32_t amb = __ballot_sync(kFullMask, lane < R && last.y != 0.f); amb; amb &= amb - 1u) {
+        const int k1 = __ffs(amb) - 1;
+        const float thr = __shfl_sync(kFullMask, last.x, k1);
+        const int *list = nn + (size_t)__shfl_sync(kFullMask, v, k1) * nn_ls;
+        for (uint32_t at = __ballot_sync(kFullMask, tile[k1 * kRL + lane] == thr) & cust & ~(1u << k1); at;
+             at &= at - 1u) {
+            const int b = __ffs(at) - 1, node = __shfl_sync(kFullMask, v, b);
+            bool hit = false;
+            for (int h = lane; h < nn_ls; h += 32) hit = hit || __ldg(list + h) == node;
+            if (!__any_sync(kFullMask, hit) && lane == k1) nm &= ~(1u << b);
+        }
+    }
+    __syncwarp();
+    return nm;
+}
+
+// The lane of `mv` (improving partners) the scan reaches first: the smallest
+// distance, equal ones in list order.  gnode: the lane's global node.
+__device__ __noinline__ int first_listed(uint32_t mv, int lane, float d12, int gnode, const int *list, int nn_ls)
+{
+    const uint32_t b = __float_as_uint(__fadd_rn(d12, 0.f)); // -0 as +0
+    const uint32_t ord = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    const bool in = (mv >> lane) & 1u;
+    const uint32_t lo = __reduce_min_sync(kFullMask, in ? ord : 0xffffffffu);
+    const uint32_t tied = __ballot_sync(kFullMask, in && ord == lo);
+    if (tied & (tied - 1u))
+        for (int h = 0; h < nn_ls; h++) {
+            const uint32_t m = __ballot_sync(kFullMask, ((tied >> lane) & 1u) && __ldg(list + h) == gnode);
+            if (m) return __ffs(m) - 1;
+        }
+    return __ffs(tied) - 1;
 }
 
 // ---------------------------------------------------------------------------
-// Register path: routes of at most 32 nodes.
+// Register path: routes of at most 32 nodes.  tq, dq: on entry lane p's local
+// node p and edge length, on return the improved route's; nm: lane k's mask
+// (route_tile); v: lane k's global node.  SYM: the distances are symmetric, so
+// an edge's length is its dist_tour_wrk entry (otherwise the tile's).
 // ---------------------------------------------------------------------------
-__device__ int two_opt_route_regs(int lane, int R, bool first_route, const float *tile, const uint8_t *lnn,
-                                  const uint8_t *lcnt, int &tq, int &pk, float &dq, int pass_limit)
+template <bool SYM>
+__device__ int two_opt_route_regs(int lane, int R, bool first_route, const float *tile, uint32_t nm, int v,
+                                  const int *nn, int nn_ls, int &tq, float &dq, int pass_limit)
 {
-    // lane q: tq = local node at position q, dq = dist_tour_wrk of position q;
-    // lane k: pk = position of local node k.  Local node 0 is the depot at position 0.
-    //
-    // The scan visits positions q1 = 0, 1, ..., R-1 and skips a node whose
-    // don't-look bit is set.  `open` holds one bit per position whose node's bit
-    // is clear, rebuilt whenever a move changes the tour or the bits, so the next
-    // position to examine is a bit operation away.  For each examined node the
-    // successor and the predecessor searches (kernel.cl:180-198, 202-230) are
-    // evaluated together; the predecessor result is used only when the successor
-    // search finds no move, as in the sequential code.
-    const unsigned FULLM = 0xffffffffu;
-    const unsigned rmask = R >= 32 ? FULLM : ((1u << R) - 1u);
-    // lane k, by local node: the nodes after and before it on the tour, and the
-    // dist_tour_wrk entries at its position and the one before (position 0: its
-    // own), rebuilt after every move
-    int nsucc, npred;
-    float dout, din;
-    auto by_node = [&]() {
-        nsucc = __shfl_sync(FULLM, tq, pk + 1 < R ? pk + 1 : 0);
-        npred = __shfl_sync(FULLM, tq, pk > 0 ? pk - 1 : R - 1);
-        dout = __shfl_sync(FULLM, dq, pk);
-        din = __shfl_sync(FULLM, dq, pk > 0 ? pk - 1 : 0);
+    // `open`: bit p set while the don't-look bit of position p's node is clear; a
+    // move carries it along with the positions it reverses
+    uint32_t open = (R >= 32 ? kFullMask : (1u << R) - 1u) & ~(first_route ? 0u : 1u);
+    if (!open) return ACO_OK;
+    const int pn = lane + 1 < R ? lane + 1 : 0, pp = lane > 0 ? lane - 1 : R - 1; // next and previous position
+    int ts, tp;   // the local nodes there
+    float dqp;    // dist_tour_wrk of the previous position
+    uint32_t word; // tq | ts << 8 | tp << 16
+    auto neighbours = [&]() {
+        ts = __shfl_sync(kFullMask, tq, pn);
+        tp = __shfl_sync(kFullMask, tq, pp);
+        dqp = __shfl_sync(kFullMask, dq, pp);
+        word = (uint32_t)tq | ((uint32_t)ts << 8) | ((uint32_t)tp << 16);
     };
-    by_node();
-    uint32_t dlb = first_route ? 0u : 1u; // bit k: don't-look bit of local node k
-    int passes = 0;
-    bool imp = true;
-    // the first half of an examination: node k1 at position q, its tour
-    // neighbours, its filtered list entry for this lane and the radii.  It
-    // depends only on q and the tour, so the next open position's is loaded
-    // while the current examination's ballots resolve (used when no move
-    // happens, which is the common case; recomputed after a move).
-    struct Head {
-        int k1, ks1, kp1, k2;
-        bool act;
-        float d12, rs, rp;
-    };
-    auto head = [&](int q) {
-        Head h;
-        h.k1 = __shfl_sync(FULLM, tq, q);
-        h.ks1 = __shfl_sync(FULLM, tq, q + 1 < R ? q + 1 : 0);
-        h.kp1 = __shfl_sync(FULLM, tq, q > 0 ? q - 1 : R - 1);
-        h.act = lane < (int)lcnt[h.k1];
-        h.k2 = h.act ? lnn[h.k1 * kRL + lane] : 0;
-        h.d12 = tile[h.k1 * kRL + h.k2];
-        h.rs = tile[h.k1 * kRL + h.ks1]; // successor radius
-        h.rp = tile[h.kp1 * kRL + h.k1]; // predecessor radius
-        return h;
-    };
-    while (imp) {
-        if (pass_limit > 0 && passes >= pass_limit) return ACO_ERR_LS_LIMIT;
-        passes++;
-        imp = false;
-        uint32_t open = __ballot_sync(FULLM, lane < R && !((dlb >> tq) & 1u)) & rmask;
-        if (!open) break;
-        int q1 = __ffs(open) - 1;
-        Head h = head(q1);
-        for (;;) {
-            const int k1 = h.k1, ks1 = h.ks1, kp1 = h.kp1, k2 = h.k2;
-            const bool act = h.act;
-            const float d12 = h.d12, rs = h.rs, rp = h.rp;
-            // k2's neighbours on the tour and edge lengths, one shuffle level from k2
-            const int ks2 = __shfl_sync(FULLM, nsucc, k2);
-            const int kpp2 = __shfl_sync(FULLM, npred, k2);
-            const float dq2 = __shfl_sync(FULLM, dout, k2);
-            const float dqp2 = __shfl_sync(FULLM, din, k2);
-            const bool sc = act && __fsub_rn(rs, d12) > kEps;
-            const bool pc = act && __fsub_rn(rp, d12) > kEps;
-            bool sok = false, pok = false;
-            if (sc) {
-                const float g = __fsub_rn(__fadd_rn(__fadd_rn(-rs, d12), tile[ks1 * kRL + ks2]), dq2);
-                sok = g < -kEps;
-            }
-            if (pc && !(kpp2 == k1 || kp1 == k2)) {
-                const float g = __fsub_rn(__fadd_rn(__fadd_rn(-rp, d12), tile[kp1 * kRL + kpp2]), dqp2);
-                pok = g < -kEps;
-            }
-            // the scan stops at the first lane whose entry ends it: past the radius, or
-            // an improving move (kernel.cl:180-198, 202-230); found = that lane moves
-            const unsigned sstop = __ballot_sync(FULLM, act && (!sc || sok));
-            const unsigned pstop = __ballot_sync(FULLM, act && (!pc || pok));
-            const unsigned smove = __ballot_sync(FULLM, sok), pmove = __ballot_sync(FULLM, pok);
-            // the next open position if this examination makes no move, and its head
-            const uint32_t rest = open & ~((2u << q1) - 1u); // positions > q1 (2u << 31 wraps to 0: none)
-            const int qn = __ffs(rest) - 1;                   // -1 when none (the head is then unused)
-            const Head hn = head(qn);
-            const bool sfound = (sstop & (0u - sstop) & smove) != 0u; // the lowest stop is a move
-            const bool pfound = (pstop & (0u - pstop) & pmove) != 0u;
-            int h1, h2, h3, h4;
-            if (sfound) {
-                const int sf = __ffs(sstop) - 1;
-                h1 = k1;
-                h2 = ks1;
-                h3 = __shfl_sync(FULLM, k2, sf);
-                h4 = __shfl_sync(FULLM, ks2, sf);
-            } else if (pfound) {
-                const int pf = __ffs(pstop) - 1;
-                h1 = kp1;
-                h2 = k1;
-                h3 = __shfl_sync(FULLM, kpp2, pf);
-                h4 = __shfl_sync(FULLM, k2, pf);
-            } else {
-                dlb |= 1u << k1; // kernel.cl:232
-                open &= ~(1u << q1);
-                if (!rest) break;
-                q1 = qn;
-                h = hn;
-                continue;
-            }
-            // exchange (kernel.cl:235-270)
+    neighbours();
+    int passes = 1;
+    bool imp = false;
+    int q1 = __ffs(open) - 1;
+    for (;;) {
+        const uint32_t w1 = __shfl_sync(kFullMask, word, q1), m1 = __shfl_sync(kFullMask, nm, q1);
+        const int k1 = w1 & 0xff, ks1 = (w1 >> 8) & 0xff, kp1 = w1 >> 16;
+        const float d12 = tile[k1 * kRL + tq], xs = tile[ks1 * kRL + ts], xp = tile[kp1 * kRL + tp];
+        // radii: the examined node's two tour edges
+        const float rs = SYM ? __shfl_sync(kFullMask, dq, q1) : tile[k1 * kRL + ks1];
+        const float rp = SYM ? __shfl_sync(kFullMask, dqp, q1) : tile[kp1 * kRL + k1];
+        const bool act = (m1 >> tq) & 1u;
+        // successor and predecessor searches (kernel.cl:180-198, 202-230); -r + d is -(r - d)
+        const float us = __fsub_rn(rs, d12), up = __fsub_rn(rp, d12);
+        const float gs = __fsub_rn(__fsub_rn(xs, us), dq), gp = __fsub_rn(__fsub_rn(xp, up), dqp);
+        const uint32_t smove = __ballot_sync(kFullMask, act & (us > kEps) & (gs < -kEps));
+        const uint32_t pmove =
+            __ballot_sync(kFullMask, act & (up > kEps) & (tp != k1) & (tq != kp1) & (gp < -kEps));
+        const uint32_t later = 0xfffffffeu << q1; // positions after q1
+        uint32_t next;
+        if ((smove | pmove) == 0u) {
+            open &= ~(1u << q1); // kernel.cl:232
+            next = open & later;
+        } else { // the predecessor's result counts only when the successor search finds no move
             imp = true;
-            dlb &= ~((1u << h1) | (1u << h2) | (1u << h3) | (1u << h4));
-            route_exchange(lane, tile, h1, h2, h3, h4, tq, pk, dq);
-            by_node();
-            open = __ballot_sync(FULLM, lane < R && !((dlb >> tq) & 1u)) & rmask; // the tour and bits changed
-            const uint32_t ahead = open & ~((2u << q1) - 1u); // the scan goes on after q1
-            if (!ahead) break;
-            q1 = __ffs(ahead) - 1;
-            h = head(q1);
+            const uint32_t mv = smove ? smove : pmove;
+            int f = __ffs(mv) - 1;
+            if (mv & (mv - 1u))
+                f = first_listed(mv, lane, d12, __shfl_sync(kFullMask, v, tq),
+                                 nn + (size_t)__shfl_sync(kFullMask, v, k1) * nn_ls, nn_ls);
+            // exchange (kernel.cl:235-270): the edges leaving positions i < j make way for
+            // (i, j) and (i + 1, j + 1); positions i + 1 .. j are reversed
+            const int pa = smove ? q1 : (q1 > 0 ? q1 - 1 : R - 1), pb = smove ? f : f - 1;
+            const int i = min(pa, pb), j = max(pa, pb), jn = j + 1 < R ? j + 1 : 0;
+            const uint32_t wi = __shfl_sync(kFullMask, word, i), wj = __shfl_sync(kFullMask, word, j);
+            const float d13 = tile[(wi & 0xff) * kRL + (wj & 0xff)];
+            const float d24 = tile[((wi >> 8) & 0xff) * kRL + ((wj >> 8) & 0xff)];
+            const bool in = lane > i && lane <= j;
+            const int src = in ? i + 1 + j - lane : lane;
+            tq = __shfl_sync(kFullMask, tq, src);
+            nm = __shfl_sync(kFullMask, nm, src);
+            const float dr = __shfl_sync(kFullMask, dq, in && lane < j ? i + j - lane : lane);
+            dq = lane == j ? d24 : lane == i ? d13 : dr;
+            open = __ballot_sync(kFullMask, (open >> src) & 1u) | (1u << i) | (2u << i) | (1u << j) | (1u << jn);
+            neighbours();
+            next = open & later;
         }
+        if (next == 0u) { // end of the pass
+            if (!imp || open == 0u) break;
+            if (pass_limit > 0 && passes >= pass_limit) return ACO_ERR_LS_LIMIT;
+            passes++;
+            imp = false;
+            next = open;
+        }
+        q1 = __ffs(next) - 1;
     }
     return ACO_OK;
 }
@@ -188,8 +191,7 @@ __device__ int two_opt_route_regs(int lane, int R, bool first_route, const float
 // bytes of the warp's shared memory for the local node at every position.  At
 // most move_limit moves (then ACO_ERR_LS_LIMIT).
 // ---------------------------------------------------------------------------
-__device__ int two_opt_route_best(int lane, int R, const float *tile, uint8_t *tpos, int &tq, int &pk, float &dq,
-                                  int move_limit)
+__device__ int two_opt_route_best(int lane, int R, const float *tile, uint8_t *tpos, int &tq, float &dq, int move_limit)
 {
     const unsigned FULLM = 0xffffffffu;
     for (int moves = 0;; moves++) {
@@ -229,7 +231,6 @@ __device__ int two_opt_route_best(int lane, int R, const float *tile, uint8_t *t
         else if (lane > i && lane < jj) dq = dsrc;
         const int tsrc = __shfl_sync(FULLM, tq, (lane >= a && lane <= jj) ? a + jj - lane : lane);
         if (lane >= a && lane <= jj) tq = tsrc;
-        if (pk >= a && pk <= jj) pk = a + jj - pk;
     }
     return ACO_OK;
 }
