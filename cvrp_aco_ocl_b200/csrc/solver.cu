@@ -851,7 +851,9 @@ void *aco_batch_get_stream(aco_batch *b) { return b ? (void *)b->c.st : nullptr;
 namespace {
 
 // Per-kernel times (ms per iteration) of one configuration on a fresh colony.
-int time_config(const InstanceSpec *specs, int count, const aco_params &p, int iters, float *ph4)
+// parity_shape (optional): the parity construct's {ants per CTA, warps per ant} it ran with.
+int time_config(const InstanceSpec *specs, int count, const aco_params &p, int iters, float *ph4,
+                int *parity_shape = nullptr)
 {
     Colony c;
     int rc = c.create(specs, count, p);
@@ -861,6 +863,10 @@ int time_config(const InstanceSpec *specs, int count, const aco_params &p, int i
     if (rc == ACO_OK) rc = c.time_phases(iters, ph4);
     if (rc != ACO_OK) return rc;
     for (int k = 0; k < 4; k++) ph4[k] /= (float)iters;
+    if (parity_shape) {
+        parity_shape[0] = c.cp_apc;
+        parity_shape[1] = c.cp_wpa;
+    }
     return ACO_OK;
 }
 
@@ -878,9 +884,14 @@ int autotune(const InstanceSpec *specs, int count, const aco_params &p0, int ite
     float best_ph[4] = {0, 0, 0, 0};
     float best_c = INFINITY;
     bool any = false;
-    if (time_config(specs, count, p0, iters, best_ph) == ACO_OK) {
+    int shape[2];
+    if (time_config(specs, count, p0, iters, best_ph, shape) == ACO_OK) {
         best_c = best_ph[0] * kMargin;
         any = true;
+        if (!thr) { // the model's own shape is an answer too: set where it was left to it
+            best.ants_per_block = shape[0];
+            best.warps_per_ant = shape[1];
+        }
     }
     // construct: ants per CTA x (warps per ant | matrix staging x (helper draw warps |
     // CTAs per SM))
