@@ -5,25 +5,29 @@
 // Who needs it: hosts whose own memory manager owns every byte of device memory
 // and forbids libraries from calling cudaMalloc (fixed memory budgets, pooled
 // allocators), and loops that cannot afford the device-wide synchronisation that
-// cudaMalloc / cudaFree imply.  Such a caller passes its own device buffers for
-// the inputs and outputs; the only other memory this entry point touches is the
-// fixed scratch array below, which lives in the library image and is reserved on
-// every GPU that loads the library until the process exits.
+// cudaMalloc / cudaFree imply.  Such a caller passes its own device buffers; the
+// update touches no other device memory, so calls on different streams and
+// threads do not meet.
 //
 // Limits: n <= kMaxNodes (4096) nodes and ras_ranks <= kMaxRanks (8); larger
-// problems are rejected with ACO_ERR_CAPACITY.  All calls share the one scratch
-// array (it keeps the last call's contents; each call re-initialises what it
-// reads), so calls that overlap on the GPU -- on different streams, or from
-// different threads -- race and must be serialised by the caller.
+// problems are rejected with ACO_ERR_CAPACITY.
+//
+// One launch.  A CTA owns a block of matrix rows and finds for itself what its
+// rows receive: it selects the elites from the lengths, walks the elite tours (a
+// few times 2n ints, from L2) and keeps the edges that leave its rows in shared
+// memory, then streams the rows.  Before, one CTA wrote deposit lists for a
+// second launch to read.  What bounds it: the instructions of one CTA's phases
+// (37 k a CTA at half the issue slots) and the chain of dependent reads between
+// them (lengths, tour sizes, tours; the rows' first part is loaded ahead); 16 MB at
+// the copy bandwidth would take 2.5 us.  n = 1001, 256 ants: 28.7 -> 12.3 us a call.
 //
 // The elite tours come from the caller's buffers, so they are checked before
-// any scratch write: an elite whose tour size lies outside [2, 2n-1] or that
-// holds a node id outside [0, n) deposits nothing, and its elites_out entry
+// they are used as indices: an elite whose tour size lies outside [2, 2n-1] or
+// that holds a node id outside [0, n) deposits nothing, and its elites_out entry
 // reads ACO_ERR_INVALID instead of the ant id.
-#include <cuda.h>
 #include <cuda_runtime.h>
 
-#include <mutex>
+#include <atomic>
 
 #include "../../include/cvrp_aco.h"
 #include "aco_device.cuh"
@@ -33,24 +37,10 @@ namespace {
 
 constexpr int kMaxNodes = 4096;
 constexpr int kMaxRanks = 8;
-
-struct NoAllocScratch {
-    int succ[kMaxRanks * kMaxNodes]; // successor of customer i in elite r's tour, -1 if none
-    uint32_t depmask[kMaxNodes];     // bit r: elite r's tour goes depot -> i
-    float d_tau[kMaxRanks];          // (ras_ranks - r) / length of elite r
-    int elites[kMaxRanks];           // elite ant ids, [0] = best-so-far slot
-};
-
-// The scratch: 148 KB of device memory in the library image, no allocation.
-static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
-
-// Device address of g_noalloc_scratch per device, looked up once per device and
-// context: a context that is destroyed and created again (cudaDeviceReset) may
-// load the module at another address, so the cached address is keyed on the
-// context it was looked up in.
-std::mutex g_scratch_mu;
-NoAllocScratch *g_scratch_ptr[64] = {};
-CUcontext g_scratch_ctx[64] = {};
+constexpr int kThreads = 1024;
+constexpr int kLens = 2048;  // lengths kept in shared memory (more are read again in every round)
+constexpr int kRowsMax = 32; // rows of a CTA
+constexpr int kU = 4;        // columns of a lane in a chunk of 32 kU
 
 __device__ __forceinline__ unsigned long long block_min_key(unsigned long long v, unsigned long long *red)
 {
@@ -61,8 +51,7 @@ __device__ __forceinline__ unsigned long long block_min_key(unsigned long long v
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    const int nw = (blockDim.x + 31) >> 5;
-    v = (int)(threadIdx.x & 31) < nw ? red[threadIdx.x & 31] : ~0ull;
+    v = red[threadIdx.x & 31];
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
         v = w < v ? w : v;
@@ -70,94 +59,155 @@ __device__ __forceinline__ unsigned long long block_min_key(unsigned long long v
     return v;
 }
 
-// Elites (kernel.cl:717-741) and the per-node deposit lists, written into the
-// scratch.  One CTA.
-__global__ void __launch_bounds__(1024) noalloc_deposit_list_kernel(NoAllocScratch *sc, int n, int n_ants,
-                                                                     int ras_ranks, const int *solutions,
-                                                                     const float *lens, int *elites_out)
+// Rows [blockIdx.x * rows, + rows).  eta^beta is recomputed from the distance
+// (kernel.cl:782-789).
+template <bool PLAIN>
+__global__ void __launch_bounds__(kThreads) noalloc_update_kernel(int n, int ld, int n_ants, int R, int rows, float evap,
+                                                                  float alpha, int alpha_int, float beta, int beta_int,
+                                                                  float *tau, float *total, const float *dist,
+                                                                  const int *solutions, const float *lens,
+                                                                  int *elites_out)
 {
+    static_assert(kThreads == 1024, "block_min_key reads 32 warps' minima");
     __shared__ unsigned long long red[32];
-    __shared__ int s_knocked[kMaxRanks];
-    const int A = n_ants, T = 2 * n, tid = threadIdx.x, bs = blockDim.x;
-    if (tid == 0) sc->elites[0] = A;
-    for (int r = 1; r < ras_ranks; r++) {
-        unsigned long long m = ~0ull;
-        for (int k = tid; k < A; k += bs) {
-            bool out = false;
-            for (int q = 1; q < r; q++) out = out || (s_knocked[q] == k);
-            const float v = out ? __int_as_float(0x7f800000) : lens[k];
-            const unsigned long long key = ((unsigned long long)__float_as_uint(v) << 32) | (unsigned)k;
-            m = key < m ? key : m;
+    __shared__ float s_len[kLens], s_amt[kMaxRanks];
+    __shared__ int s_elite[kMaxRanks], s_size[kMaxRanks], s_bad[kMaxRanks];
+    __shared__ int s_succ[kMaxRanks][kRowsMax]; // successor of the CTA's customers in elite r's tour, -1 if none
+    __shared__ uint32_t s_dep[kMaxNodes];       // row 0's CTA: bit r, elite r's tour goes depot -> column
+    const int A = n_ants, T = 2 * n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i0 = blockIdx.x * rows, i1 = min(n, i0 + rows);
+    // chunks of 32 kU columns over the CTA's rows; the warp's first is loaded ahead
+    const int per_row = (n + 32 * kU - 1) / (32 * kU), chunks = (i1 - i0) * per_row;
+    float t[kU], d[kU];
+    auto load = [&](int c) {
+        const int i = i0 + c / per_row, j0 = (c % per_row) * 32 * kU + lane;
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const int j = j0 + 32 * u;
+            t[u] = j < n ? tau[(size_t)i * ld + j] : 0.f;
+            d[u] = j < n ? dist[(size_t)i * ld + j] : 0.f;
         }
-        m = block_min_key(m, red);
-        if (tid == 0) {
-            const int target = (int)(m & 0xffffffffu);
-            s_knocked[r] = target;
-            sc->elites[r] = target;
+    };
+    if (warp < chunks) load(warp);
+
+    // elites (kernel.cl:717-741): the best-so-far slot, then rounds of "first
+    // minimum, knocked out to +inf"
+    const float inf = __int_as_float(0x7f800000);
+    for (int k = tid; k < A && k < kLens; k += kThreads) s_len[k] = lens[k];
+    for (int e = tid; e < kMaxRanks * kRowsMax; e += kThreads) s_succ[0][e] = -1;
+    if (i0 == 0)
+        for (int j = tid; j < n; j += kThreads) s_dep[j] = 0u;
+    if (tid < kMaxRanks) s_bad[tid] = 0;
+    if (tid == 0) s_elite[0] = A;
+    __syncthreads();
+    if (A <= kLens) { // one warp runs the rounds, without block barriers
+        if (warp == 0) {
+            for (int r = 1; r < R; r++) {
+                uint32_t lo = 0xffffffffu, at = 0xffffffffu;
+                for (int k = lane; k < A; k += 32) {
+                    const uint32_t b = __float_as_uint(s_len[k]);
+                    at = b < lo ? (uint32_t)k : at;
+                    lo = b < lo ? b : lo;
+                }
+                const uint32_t least = __reduce_min_sync(0xffffffffu, lo);
+                const int target = (int)__reduce_min_sync(0xffffffffu, lo == least ? at : 0xffffffffu);
+                if (lane == 0) {
+                    s_elite[r] = target;
+                    s_len[target] = inf;
+                }
+                __syncwarp();
+            }
         }
         __syncthreads();
+    } else {
+        for (int r = 1; r < R; r++) {
+            unsigned long long m = ~0ull;
+            for (int k = tid; k < A; k += kThreads) {
+                float v = k < kLens ? s_len[k] : lens[k];
+                if (k >= kLens)
+                    for (int q = 1; q < r; q++) v = s_elite[q] == k ? inf : v;
+                const unsigned long long key = ((unsigned long long)__float_as_uint(v) << 32) | (unsigned)k;
+                m = key < m ? key : m;
+            }
+            m = block_min_key(m, red);
+            if (tid == 0) {
+                const int target = (int)(m & 0xffffffffu);
+                s_elite[r] = target;
+                if (target < kLens) s_len[target] = inf;
+            }
+            __syncthreads();
+        }
     }
-    for (int e = tid; e < ras_ranks * n; e += bs) sc->succ[e] = -1; // clear what the last call left
-    for (int e = tid; e < n; e += bs) sc->depmask[e] = 0u;
-    // Check every elite tour before it is read as indices: size in [2, T-1],
-    // every node id in [0, n).  A failing elite deposits nothing (d_tau = 0 and
-    // no list entries) and is reported as ACO_ERR_INVALID.
-    __shared__ int s_bad[kMaxRanks];
-    if (tid < ras_ranks) s_bad[tid] = 0;
+    if (tid < R) {
+        const int e = s_elite[tid], size = solutions[(size_t)T * e + T - 1];
+        const bool bad = size < 2 || size > T - 1;
+        s_size[tid] = bad ? 0 : size;
+        s_bad[tid] = bad ? 1 : 0;
+        s_amt[tid] = __fdiv_rn((float)(R - tid), lens[e]);
+    }
     __syncthreads();
-    for (int r = 0; r < ras_ranks; r++) {
-        const int *tour = solutions + (size_t)T * sc->elites[r];
-        const int size = tour[T - 1];
-        if (size < 2 || size > T - 1) {
-            if (tid == 0) s_bad[r] = 1;
-            continue;
-        }
-        for (int k = tid; k < size; k += bs) {
-            const int u = tour[k];
-            if (u < 0 || u >= n) s_bad[r] = 1;
+    // every node of the elite tours checked, the edges that leave this CTA's rows
+    // kept: the warps are dealt out over the elites, four nodes a lane in flight
+    {
+        const int per = kThreads / 32 / R, r = warp / per; // warps of an elite (at least 4)
+        const int size = r < R ? s_size[r] : 0, step = per * 32;
+        const int *tour = solutions + (size_t)T * (r < R ? s_elite[r] : A);
+        for (int k0 = (warp - r * per) * 32 + lane; k0 < size; k0 += 4 * step) {
+            int uu[4], vv[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int k = k0 + q * step;
+                uu[q] = k < size ? __ldg(tour + k) : 0;
+                vv[q] = k + 1 < size ? __ldg(tour + k + 1) : -1;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if ((unsigned)uu[q] >= (unsigned)n) s_bad[r] = 1;
+                if (uu[q] < i0 || uu[q] >= i1 || (unsigned)vv[q] >= (unsigned)n) continue;
+                if (uu[q] == 0) atomicOr(&s_dep[vv[q]], 1u << r);
+                else s_succ[r][uu[q] - i0] = vv[q];
+            }
         }
     }
     __syncthreads();
-    if (tid < ras_ranks) {
-        const bool bad = s_bad[tid] != 0;
-        sc->d_tau[tid] = bad ? 0.0f : __fdiv_rn((float)(ras_ranks - tid), lens[sc->elites[tid]]);
-        if (elites_out) elites_out[tid] = bad ? ACO_ERR_INVALID : sc->elites[tid];
-    }
-    for (int r = 0; r < ras_ranks; r++) {
-        if (s_bad[r]) continue;
-        const int *tour = solutions + (size_t)T * sc->elites[r];
-        const int size = tour[T - 1];
-        for (int k = tid; k < size - 1; k += bs) {
-            const int u = tour[k], v = tour[k + 1];
-            if (u != 0) sc->succ[(size_t)r * n + u] = v;
-            else atomicOr(&sc->depmask[v], 1u << r);
-        }
-    }
-}
+    if (blockIdx.x == 0 && tid < R && elites_out) elites_out[tid] = s_bad[tid] ? ACO_ERR_INVALID : s_elite[tid];
+    uint32_t good = 0u;
+    for (int r = 0; r < R; r++) good |= (s_bad[r] ? 0u : 1u) << r;
 
-// Evaporation + deposit (elite order) + total_info, one element per thread, any
-// row pitch; eta^beta is recomputed from the distance (kernel.cl:782-789).
-__global__ void __launch_bounds__(256) noalloc_pass_kernel(const NoAllocScratch *sc, int n, int ld, int ras_ranks,
-                                                            float evap, float alpha, int alpha_int, float beta,
-                                                            int beta_int, float *tau, float *total,
-                                                            const float *dist)
-{
-    const size_t count = (size_t)n * n;
-    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < count; g += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(g / (size_t)n), j = (int)(g - (size_t)i * n);
-        const size_t off = (size_t)i * ld + j;
-        float v = __fmul_rn(evap, tau[off]);
+    // evaporation + deposit (elite order) + total_info
+    for (int c = warp; c < chunks; c += kThreads / 32) {
+        if (c != warp) load(c);
+        const int i = i0 + c / per_row, j0 = (c % per_row) * 32 * kU + lane;
+        const size_t off = (size_t)i * ld;
+        float v[kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++) v[u] = __fmul_rn(evap, t[u]);
         if (i != 0) {
-            for (int r = 0; r < ras_ranks; r++)
-                if (sc->succ[(size_t)r * n + i] == j) v = __fadd_rn(v, sc->d_tau[r]);
+            for (int r = 0; r < R; r++) {
+                const unsigned at = (unsigned)(s_succ[r][i - i0] - (j0 - lane)); // place in the chunk
+                if (at >= 32u * kU || !((good >> r) & 1u)) continue;             // warp-uniform
+                if ((at & 31u) == (unsigned)lane) {
+                    const float amt = s_amt[r];
+#pragma unroll
+                    for (int u = 0; u < kU; u++) v[u] = (at >> 5) == (unsigned)u ? __fadd_rn(v[u], amt) : v[u];
+                }
+            }
         } else {
-            const uint32_t m = sc->depmask[j];
-            for (int r = 0; r < ras_ranks; r++)
-                if ((m >> r) & 1u) v = __fadd_rn(v, sc->d_tau[r]);
+#pragma unroll
+            for (int u = 0; u < kU; u++)
+                for (uint32_t m = j0 + 32 * u < n ? s_dep[j0 + 32 * u] & good : 0u; m; m &= m - 1u)
+                    v[u] = __fadd_rn(v[u], s_amt[__ffs(m) - 1]);
         }
-        const float eta = __fdiv_rn(1.0f, __fadd_rn(dist[off], 0.1f));
-        tau[off] = v;
-        total[off] = __fmul_rn(pow_rule(v, alpha, alpha_int), pow_rule(eta, beta, beta_int));
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const int j = j0 + 32 * u;
+            if (j >= n) continue;
+            const float eta = __fdiv_rn(1.0f, __fadd_rn(d[u], 0.1f));
+            tau[off + j] = v[u];
+            // the defaults alpha 1, beta 2 without pow_rule's loops (the same products)
+            total[off + j] = PLAIN ? __fmul_rn(v[u], __fmul_rn(eta, eta))
+                                   : __fmul_rn(pow_rule(v[u], alpha, alpha_int), pow_rule(eta, beta, beta_int));
+        }
     }
 }
 
@@ -167,43 +217,18 @@ int exp_int(float e)
     return -1;
 }
 
-// Set-up, once per device and context, with that device current: the device
-// address of the scratch array (its host-side name is only a stand-in, not a
-// device address).  The current context comes from the driver's
-// cuCtxGetCurrent, reached through cudaGetDriverEntryPoint so the library
-// needs no link against libcuda.
-using CtxGetCurrentFn = CUresult (*)(CUcontext *);
-
-CtxGetCurrentFn ctx_get_current()
+// Multiprocessors of the current device, asked once per device.
+int multiprocessors()
 {
-    static CtxGetCurrentFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<CtxGetCurrentFn>(p);
-    }();
-    return fn;
-}
-
-int scratch_address(NoAllocScratch **out)
-{
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ACO_ERR_CUDA;
-    const CtxGetCurrentFn get = ctx_get_current();
-    CUcontext ctx = nullptr; // null until the runtime has made the device's primary context current
-    if (!get || get(&ctx) != CUDA_SUCCESS) return ACO_ERR_CUDA;
-    std::lock_guard<std::mutex> lock(g_scratch_mu);
-    if (ctx == nullptr || !g_scratch_ptr[dev] || g_scratch_ctx[dev] != ctx) {
-        void *p = nullptr; // the lookup also initialises the primary context when needed
-        if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || p == nullptr) return ACO_ERR_CUDA;
-        if (ctx == nullptr && (get(&ctx) != CUDA_SUCCESS || ctx == nullptr)) return ACO_ERR_CUDA;
-        g_scratch_ptr[dev] = static_cast<NoAllocScratch *>(p);
-        g_scratch_ctx[dev] = ctx;
+    static std::atomic<int> known[64];
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    v = known[dev].load(std::memory_order_relaxed);
+    if (v == 0) {
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+        known[dev].store(v, std::memory_order_relaxed);
     }
-    *out = g_scratch_ptr[dev];
-    return ACO_OK;
+    return v;
 }
 
 } // namespace
@@ -217,17 +242,16 @@ extern "C" int aco_pheromone_update_noalloc(int n, int ld, int n_ants, int ras_r
     if (n < 2 || ld < n || n_ants < 1 || ras_ranks < 1 || !tau || !total_info || !dist || !solutions || !lens)
         return ACO_ERR_INVALID;
     if (!(rho > 0.0f && rho <= 1.0f)) return ACO_ERR_INVALID;
-    if (n > kMaxNodes || ras_ranks > kMaxRanks) return ACO_ERR_CAPACITY; // beyond the fixed scratch array
-    NoAllocScratch *sc = nullptr;
-    const int rc = scratch_address(&sc);
-    if (rc != ACO_OK) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    noalloc_deposit_list_kernel<<<1, 1024, 0, st>>>(sc, n, n_ants, ras_ranks, solutions, lens, elites_out);
-    if (cudaGetLastError() != cudaSuccess) return ACO_ERR_CUDA;
-    const size_t count = (size_t)n * n;
-    const int blocks = (int)((count + 255) / 256 < 2048 ? (count + 255) / 256 : 2048);
-    noalloc_pass_kernel<<<blocks, 256, 0, st>>>(sc, n, ld, ras_ranks, 1.0f - rho, alpha, exp_int(alpha), beta,
-                                                exp_int(beta), tau, total_info, dist);
+    if (n > kMaxNodes || ras_ranks > kMaxRanks) return ACO_ERR_CAPACITY; // beyond a CTA's shared memory
+    const int sm = multiprocessors();
+    if (sm < 1) return ACO_ERR_CUDA;
+    int rows = (n + sm - 1) / sm; // one CTA an SM
+    if (rows > kRowsMax) rows = kRowsMax;
+    const int ai = exp_int(alpha), bi = exp_int(beta);
+    auto kern = ai == 1 && bi == 2 ? noalloc_update_kernel<true> : noalloc_update_kernel<false>;
+    kern<<<(n + rows - 1) / rows, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        n, ld, n_ants, ras_ranks, rows, 1.0f - rho, alpha, ai, beta, bi, tau, total_info, dist, solutions, lens,
+        elites_out);
     if (cudaGetLastError() != cudaSuccess) return ACO_ERR_CUDA;
     return ACO_OK;
 }

@@ -402,11 +402,8 @@ int aco_batch_get_bsf_records(aco_batch *b, int idx, aco_record *out, int cap, i
  * The elite tours are checked before they are used as indices: an elite whose
  * size is outside [2, 2n-1] or that holds a node id outside [0, n) deposits
  * nothing, and its elites_out entry reads ACO_ERR_INVALID instead of its ant id.
- * Scratch is a fixed 148 KB array inside the library (kept by every GPU that
- * loads it until exit): n <= 4096 and ras_ranks <= 8, else ACO_ERR_CAPACITY.
- * The first call on a device (and again after its context is recreated) looks
- * up that array's device address; make it before any stream capture.  Calls
- * share the array, so calls that overlap on the GPU race.  Allocates nothing,
+ * Limits: n <= 4096 and ras_ranks <= 8, else ACO_ERR_CAPACITY.  Uses no device
+ * memory but the caller's; calls on different buffers may overlap.  Allocates nothing,
  * frees nothing. */
 int aco_pheromone_update_noalloc(int n, int ld, int n_ants, int ras_ranks, float rho, float alpha, float beta,
                                  float *tau, float *total_info, const float *dist, const int *solutions,
