@@ -389,7 +389,6 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
     // construct work items {instance, first ant}, larger instances first
     // (set after cn_apc is known; sized for apc = 1)
     const size_t o_items = take((size_t)total_ants * sizeof(int2));
-    const size_t o_sw_items = take((size_t)total_ants * sizeof(int2));
     const size_t o_ns_items = take((size_t)total_ants * sizeof(int2));
     const size_t o_ls_needed = take((size_t)total_ants);
     // route list of the route-level 2-opt: throughput mode with 2-opt, instances
@@ -471,7 +470,6 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
     uargs_d_ = (UpdateArgs *)(base + o_uargs);
     PrepArgs *pargs_d = (PrepArgs *)(base + o_pargs);
     items_d_ = (int2 *)(base + o_items);
-    sw_items_d_ = (int2 *)(base + o_sw_items);
     ns_items_d_ = (int2 *)(base + o_ns_items);
     ls_needed_d_ = (uint8_t *)(base + o_ls_needed);
     route_desc_d_ = (int2 *)(base + o_rdesc);
@@ -630,15 +628,13 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         }
         if (best_cost < 0 && (p.ls_flag & 1)) return ACO_ERR_INVALID; // the caller's shape does not fit
     }
-    if (p.ls_flag & 2) { // swap stage: as many ants per CTA as their shared arrays allow, up to 8
-        int n_max = 0, ld_of_max = 32;
-        for (const InstHost &ih : inst)
-            if (ih.n > n_max) { n_max = ih.n; ld_of_max = ih.ld; }
-        sw_apc = 8;
-        while (sw_apc > 1 && swap_smem(n_max, ld_of_max, sw_apc) > kSmemBudget) sw_apc--;
-        sw_smem = 0;
-        for (const InstHost &ih : inst) sw_smem = std::max(sw_smem, swap_smem(ih.n, ih.ld, sw_apc));
+    if (p.ls_flag & 2) { // swap stage: one CTA per ant
+        sw_smem = swap_smem(ls_nmax);
         if (sw_smem > kSmemBudget) return ACO_ERR_INVALID; // the tour arrays of one ant do not fit
+        // few ants: latency, so more positions at once (302 nodes, 128 ants: 482 / 368 / 323 us of
+        // 2-opt and swap at 2 / 4 / 8 warps); many: what is examined past an exchange is wasted
+        // (8192 ants of 128 instances: 8.9 / 5.7 / 6.9 ms)
+        sw_warps = total_ants <= 4 * sm_count ? 8 : 4;
     }
     if (p.ns_rounds > 0) { // random-descent stage: up to 8 ants per CTA
         int n_max = 0;
@@ -653,7 +649,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
 
     // ---- host tables and uploads
     std::vector<int> ant_inst(total_ants), ant_base(count + 1), row_base(count + 1), row_inst(total_rows);
-    std::vector<int2> items, swi, nsi;
+    std::vector<int2> items, nsi;
     {
         int a0 = 0, r0 = 0;
         for (int b = 0; b < count; b++) {
@@ -672,9 +668,6 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         for (int b : order)
             for (int a0 = 0; a0 < inst[b].A; a0 += cn_apc) items.push_back(make_int2(b, a0));
         n_items = (int)items.size();
-        for (int b = 0; b < count; b++)
-            for (int a0 = 0; a0 < inst[b].A; a0 += sw_apc) swi.push_back(make_int2(b, a0));
-        sw_items = (int)swi.size();
         for (int b = 0; b < count; b++)
             for (int a0 = 0; a0 < inst[b].A; a0 += ns_apc) nsi.push_back(make_int2(b, a0));
         ns_items = (int)nsi.size();
@@ -761,6 +754,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         c.smat = ih.smat ? 1 : 0; c.packed = ih.packed ? 1 : 0; c.gtab = ih.gtab ? 1 : 0;
         c.nn_list = ih.nnls_d; c.nnr = ih.nnr_d; c.nn_ls = ih.nn_ls; c.pass_limit = p.ls_pass_limit; c.ant_base = ant_base[b];
         c.ls_best = p.ls_best;
+        c.sym = ih.sym ? 1 : 0;
         c.ls_needed = ls_needed_d_;
         c.route_desc = use_routes_ ? route_desc_d_ : nullptr;
         c.route_ctr = route_ctr_d_;
@@ -804,7 +798,6 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
     const int wl = std::max(0, p.wait_limit);
     up(wait_d, &wl, 4);
     up(items_d_, items.data(), items.size() * sizeof(int2));
-    up(sw_items_d_, swi.data(), swi.size() * sizeof(int2));
     up(ns_items_d_, nsi.data(), nsi.size() * sizeof(int2));
     up(pargs_d, pargs.data(), sizeof(PrepArgs) * count);
     ok = ok && stage.flush(res->pool, sm_count, st) == cudaSuccess;
@@ -1072,7 +1065,8 @@ int Colony::local_search()
                            last_fused_ || routes ? ls_needed_d_ : nullptr, routes ? ls_list_d_ : nullptr,
                            routes ? ls_list_ctr_d_ : nullptr, sm_count));
     last_fused_ = false;
-    if (p.ls_flag & 2) CK(launch_swap(cargs_d_, sw_items_d_, sw_items, sw_apc, sw_smem, kSwapLimitPerNode, st));
+    if (p.ls_flag & 2) 
+        CK(launch_swap(cargs_d_, ant_inst_d_, ant_base_d_, total_ants, sw_warps, sw_smem, kSwapLimitPerNode, st));
     return ACO_OK;
 }
 

@@ -122,7 +122,7 @@ public:
     StatsArgs stats_one_{};     // a single instance's statistics arguments, passed by value
     size_t cn_smem = 0;
     int ls_warps = 1, ls_apc = 1, ls_nmax = 0; // 2-opt: warps and ants per CTA, largest instance
-    int sw_apc = 1, sw_items = 0; // swap stage: ants per CTA, work items
+    int sw_warps = 8;             // swap stage: warps of an ant's CTA
     size_t sw_smem = 0;
     int ns_apc = 1, ns_items = 0; // random-descent stage
     size_t ns_smem_ = 0;
@@ -139,7 +139,7 @@ private:
     void *arena_ = nullptr;
     bool pooled_ = false; // arena from the device's memory pool (freed stream-ordered)
     unsigned long long *t0_d_ = nullptr;
-    int2 *items_d_ = nullptr, *sw_items_d_ = nullptr, *ns_items_d_ = nullptr;
+    int2 *items_d_ = nullptr, *ns_items_d_ = nullptr;
     uint8_t *ls_needed_d_ = nullptr;
     // route-level 2-opt (throughput mode, symmetric distances): the construct's
     // route list, its counters and the listed routes left per ant

@@ -48,6 +48,7 @@ struct ConstructArgs {
     const float2 *nnr;     // n: see LocalSearchArgs
     int nn_ls, pass_limit, ant_base;
     int ls_best;           // the fused 2-opt improves best-first (aco_params.ls_best)
+    int sym;               // symmetric distances (swap stage)
     uint8_t *ls_needed;    // total ants of the colony
     // route list for the route-level 2-opt (null: not used): every route of at
     // most 255 nodes as {global ant, first position | nodes << 16}; route_ctr[0]
@@ -209,11 +210,12 @@ cudaError_t launch_validate(const ConstructArgs *d_args, int n_inst, int max_slo
 cudaError_t launch_gather_best(const ConstructArgs *d_args, int n_inst, const int *d_tour_base, int *tours,
                                int *sizes, float *lens, cudaStream_t st);
 
-// Inter-route swap stage (swap.cu): one CTA per item {instance, first ant}
-// with `apc` ants (one warp each).
-size_t swap_smem(int n, int ld, int apc);
-cudaError_t launch_swap(const ConstructArgs *d_args, const int2 *d_items, int n_items, int apc, size_t smem,
-                        int max_swaps_per_node, cudaStream_t st);
+// Inter-route swap stage (swap.cu): one CTA of `warps` (at most 8) warps per ant
+// of the colony; smem: swap_smem of its largest instance.  max_swaps_per_node * n
+// accepted swaps end it with ACO_ERR_LS_LIMIT.
+size_t swap_smem(int n);
+cudaError_t launch_swap(const ConstructArgs *d_args, const int *d_ant_inst, const int *d_ant_base, int total_ants,
+                        int warps, size_t smem, int max_swaps_per_node, cudaStream_t st);
 
 // Random-descent stage (ns.cu): one CTA per item {instance, first ant} with
 // `apc` ants, `rounds` neighbourhood-move proposals per ant.

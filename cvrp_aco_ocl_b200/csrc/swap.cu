@@ -4,15 +4,19 @@
 //
 // The reference scans positions i < j in order and applies the first exchange
 // of two customers whose gain is below -EPSILON and that keeps both routes
-// within capacity and max_distance, then resumes the scan at the same i.  One
-// warp per ant: for position i the lanes evaluate 32 candidate positions j at
-// a time and a ballot picks the lowest qualifying one, which is the one the
-// sequential scan would take.  Depot positions never move (only customers are
-// exchanged), so each position's route index is fixed for the whole stage.
-// Every float expression keeps the reference's evaluation order.
+// within capacity and max_distance, then resumes the scan at the same i.  Depot
+// positions never move (only customers are exchanged), so each position's route
+// index is fixed for the whole stage.  Every float expression keeps the
+// reference's evaluation order.
 //
-// One CTA per construct work item (instance, first ant): its ants share the
-// instance, whose distance matrix is staged in shared memory when it fits.
+// One CTA per ant.  Its warps examine consecutive positions i at once, each
+// scanning j in order, 64 candidates a round; the lowest i that found an
+// exchange is the one the sequential scan would reach first (the positions
+// before it have none), it is applied, and the scan resumes there.  Distances
+// of tour edges are kept per position, so a candidate costs four independent
+// reads of the matrix, three rows of it when it is symmetric.  What bounds it is
+// the latency of those reads times the rounds: 302 nodes, 128 ants, 1.01 ms with
+// a warp an ant and eight ants a CTA -> 0.28 ms.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -25,135 +29,181 @@ namespace aco {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
+constexpr int kMaxWarps = 8;
 
-// Per-warp shared arrays: tour (T ints), route index of every position (T
-// ints), route loads and lengths (n each).
-__host__ __device__ inline size_t swap_warp_bytes(int n) { return (size_t)(2 * 2 * n + 2 * n) * 4; }
+// Shared arrays of the ant: edge length at every position, route loads and
+// lengths, tour, route index of every position.
+struct SwapLayout {
+    size_t edge, load, dist, tour, rpos, bytes;
+};
 
-__host__ __device__ inline bool swap_stage_matrix(int n, int ld, int apc)
+__host__ __device__ inline SwapLayout swap_layout(int n)
 {
-    return (size_t)n * ld * 4 + (size_t)apc * swap_warp_bytes(n) <= (size_t)200 * 1024;
+    SwapLayout L;
+    size_t o = 0;
+    L.edge = o; o += (size_t)2 * n * 4;
+    L.load = o; o += (size_t)n * 4;
+    L.dist = o; o += (size_t)n * 4;
+    L.tour = o; o += (size_t)2 * n * 2;
+    L.rpos = o; o += (size_t)2 * n * 2;
+    L.bytes = (o + 15) & ~(size_t)15;
+    return L;
 }
 
-template <bool SMAT>
-__device__ void swap_ant(const ConstructArgs &a, int ant, const float *D, int ldd, int *tour, int *rpos, int *rload,
-                         float *rdist, int max_swaps)
+// One candidate exchange of positions i and j: the four new edges and both
+// routes' loads and lengths after it.
+struct Swap {
+    bool ok;
+    float a, b, c, d; // D(p1, n2), D(n2, s1), D(p2, n1), D(n1, s2)
+    int load1, load2;
+    float dist1, dist2;
+};
+
+__global__ void __launch_bounds__(kMaxWarps * 32) swap_kernel(const ConstructArgs *args, const int *ant_inst,
+                                                              const int *ant_base, int max_swaps_per_node)
 {
-    const int lane = threadIdx.x & 31, n = a.n, T = a.T;
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ int s_found[kMaxWarps];
+    const int inst = __ldg(ant_inst + blockIdx.x), ant = blockIdx.x - __ldg(ant_base + inst);
+    const ConstructArgs &a = args[inst];
+    const int n = a.n, ld = a.ld, T = a.T, capacity = a.capacity;
+    const float max_dist = a.max_dist, serv = a.serv_time;
+    const float *D = a.dist;
+    const int *demand = a.demand;
+    const bool symmetric = a.sym != 0;
+    const SwapLayout L = swap_layout(n);
+    float *edge = reinterpret_cast<float *>(sm + L.edge), *rdist = reinterpret_cast<float *>(sm + L.dist);
+    int *rload = reinterpret_cast<int *>(sm + L.load);
+    uint16_t *tour = reinterpret_cast<uint16_t *>(sm + L.tour), *rpos = reinterpret_cast<uint16_t *>(sm + L.rpos);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
     int *gt = a.solutions + (size_t)ant * T;
     const int size = gt[T - 1];
     if (size < 2) return; // a failed construction: nothing to do (its status is already set)
-    for (int p = lane; p < size; p += 32) tour[p] = gt[p];
-    __syncwarp();
-    // route index of every position (depots at or before it, counted from position 1)
-    int base = 0;
-    for (int p0 = 0; p0 < size; p0 += 32) {
-        const int p = p0 + lane;
-        const bool dep = p >= 1 && p < size && tour[p] == 0;
-        const unsigned m = __ballot_sync(FULL, dep);
-        if (p < size) rpos[p] = base + __popc(m & ((1u << lane) - 1u));
-        base += __popc(m);
-    }
-    __syncwarp();
-    // route loads and lengths (localSearch.cpp:322-341): one lane per route
-    // walks it; the route of a depot position p >= 1 ends there
-    for (int p0 = 1; p0 < size; p0 += 32) {
-        const int p = p0 + lane;
-        if (p < size && tour[p] == 0) {
-            const int k = rpos[p];
-            int beg = p - 1;
-            while (beg > 0 && tour[beg] != 0) beg--;
-            int load = 0;
-            float dd = 0.f;
-            for (int q = beg + 1; q <= p; q++) {
-                load += a.demand[tour[q]];
-                dd = __fadd_rn(dd, D[(size_t)tour[q - 1] * ldd + tour[q]]);
-            }
-            rload[k] = load;
-            rdist[k] = __fadd_rn(dd, __fmul_rn(a.serv_time, (float)(p - beg - 1)));
+    for (int p = threadIdx.x; p < size; p += blockDim.x) tour[p] = (uint16_t)gt[p];
+    __syncthreads();
+    for (int p = threadIdx.x; p < size - 1; p += blockDim.x) edge[p] = __ldg(D + (size_t)tour[p] * ld + tour[p + 1]);
+    if (warp == 0) { // route index of every position (depots at or before it, counted from position 1)
+        int base = 0;
+        for (int p0 = 0; p0 < size; p0 += 32) {
+            const int p = p0 + lane;
+            const unsigned m = __ballot_sync(FULL, p >= 1 && p < size && tour[p] == 0);
+            if (p < size) rpos[p] = (uint16_t)(base + __popc(m & ((1u << lane) - 1u)));
+            base += __popc(m);
         }
     }
-    __syncwarp();
+    __syncthreads();
+    // route loads and lengths (localSearch.cpp:322-341): one thread per route
+    // walks it; the route of a depot position p >= 1 ends there
+    for (int p = 1 + threadIdx.x; p < size; p += blockDim.x) {
+        if (tour[p] != 0) continue;
+        int beg = p - 1;
+        while (beg > 0 && tour[beg] != 0) beg--;
+        int load = 0;
+        float dd = 0.f;
+        for (int q = beg + 1; q <= p; q++) {
+            load += __ldg(demand + tour[q]);
+            dd = __fadd_rn(dd, edge[q - 1]);
+        }
+        const int k = rpos[p];
+        rload[k] = load;
+        rdist[k] = __fadd_rn(dd, __fmul_rn(serv, (float)(p - beg - 1)));
+    }
+    __syncthreads();
+
+    const int max_swaps = max_swaps_per_node * n;
     int swaps = 0;
     bool over = false;
-    for (int i = 1; i < size && !over;) {
-        const int n1 = tour[i];
-        if (n1 == 0) {
-            i++;
-            continue;
-        }
-        const int p_n1 = tour[i - 1], s_n1 = tour[i + 1], p1 = rpos[i];
-        const float d_pn1_n1 = D[(size_t)p_n1 * ldd + n1], d_n1_sn1 = D[(size_t)n1 * ldd + s_n1];
-        bool moved = false;
-        for (int j0 = i + 1; j0 < size; j0 += 32) {
-            const int j = j0 + lane;
-            int n2 = 0;
-            bool cand = false;
-            int load1 = 0, load2 = 0;
-            float dist1 = 0.f, dist2 = 0.f;
-            if (j < size) n2 = tour[j];
-            if (j < size && n2 != 0) {
-                const int p_n2 = tour[j - 1], s_n2 = tour[j + 1], p2 = rpos[j];
-                const float d_pn1_n2 = D[(size_t)p_n1 * ldd + n2], d_n1_sn2 = D[(size_t)n1 * ldd + s_n2];
-                const float d_n2_sn2 = D[(size_t)n2 * ldd + s_n2];
+    for (int i0 = 1; i0 < size && !over;) {
+        const int i = i0 + warp, n1 = i < size ? tour[i] : 0;
+        int hit_j = 0, hit_n2 = 0, hit_lane = 0;
+        Swap hit;
+        if (n1 != 0) {
+            const int p1 = tour[i - 1], s1 = tour[i + 1], r1 = rpos[i], dem1 = __ldg(demand + n1), load_1 = rload[r1];
+            const float d_p1_n1 = edge[i - 1], d_n1_s1 = edge[i], dist_1 = rdist[r1];
+            const float *row_p1 = D + (size_t)p1 * ld, *row_n1 = D + (size_t)n1 * ld, *row_s1 = D + (size_t)s1 * ld;
+            auto eval = [&](int j, int &n2) {
+                Swap s;
+                n2 = j < size ? tour[j] : 0;
+                s.ok = n2 != 0;
+                const int jc = s.ok ? j : i + 1; // an in-range position for the reads
+                const int x = tour[jc], p2 = tour[jc - 1], s2 = jc + 1 < size ? tour[jc + 1] : 0, r2 = rpos[jc];
+                s.a = __ldg(row_p1 + x);
+                s.d = __ldg(row_n1 + s2);
+                s.b = symmetric ? __ldg(row_s1 + x) : __ldg(D + (size_t)x * ld + s1);
+                s.c = symmetric ? __ldg(row_n1 + p2) : __ldg(D + (size_t)p2 * ld + n1);
+                const int dem2 = __ldg(demand + x);
+                const float d_p2_n2 = edge[jc - 1], d_n2_s2 = jc < size - 1 ? edge[jc] : 0.f;
                 float gain;
-                float d_pn2_n2 = 0.f, d_n2_sn1 = 0.f, d_pn2_n1 = 0.f;
                 if (j == i + 1) {
-                    gain = __fadd_rn(-__fadd_rn(d_pn1_n1, d_n2_sn2), __fadd_rn(d_pn1_n2, d_n1_sn2));
+                    gain = __fadd_rn(-__fadd_rn(d_p1_n1, d_n2_s2), __fadd_rn(s.a, s.d));
                 } else {
-                    d_pn2_n2 = D[(size_t)p_n2 * ldd + n2];
-                    d_n2_sn1 = D[(size_t)n2 * ldd + s_n1];
-                    d_pn2_n1 = D[(size_t)p_n2 * ldd + n1];
-                    const float rem = __fadd_rn(__fadd_rn(__fadd_rn(d_pn1_n1, d_n1_sn1), d_pn2_n2), d_n2_sn2);
-                    const float add = __fadd_rn(__fadd_rn(__fadd_rn(d_pn1_n2, d_n2_sn1), d_pn2_n1), d_n1_sn2);
+                    const float rem = __fadd_rn(__fadd_rn(__fadd_rn(d_p1_n1, d_n1_s1), d_p2_n2), d_n2_s2);
+                    const float add = __fadd_rn(__fadd_rn(__fadd_rn(s.a, s.b), s.c), s.d);
                     gain = __fadd_rn(-rem, add);
                 }
-                if (gain < -kEps) {
-                    if (p1 != p2) {
-                        load1 = rload[p1] - a.demand[n1] + a.demand[n2];
-                        load2 = rload[p2] - a.demand[n2] + a.demand[n1];
-                        dist1 = __fadd_rn(__fsub_rn(rdist[p1], __fadd_rn(d_pn1_n1, d_n1_sn1)),
-                                          __fadd_rn(d_pn1_n2, d_n2_sn1));
-                        dist2 = __fadd_rn(__fsub_rn(rdist[p2], __fadd_rn(d_pn2_n2, d_n2_sn2)),
-                                          __fadd_rn(d_pn2_n1, d_n1_sn2));
-                        cand = !((load1 > a.capacity || load2 > a.capacity) || (dist1 > a.max_dist || dist2 > a.max_dist));
-                    } else {
-                        load1 = load2 = rload[p1];
-                        dist1 = dist2 = __fadd_rn(rdist[p1], gain);
-                        cand = true;
-                    }
+                if (r1 != r2) {
+                    s.load1 = load_1 - dem1 + dem2;
+                    s.load2 = rload[r2] - dem2 + dem1;
+                    s.dist1 = __fadd_rn(__fsub_rn(dist_1, __fadd_rn(d_p1_n1, d_n1_s1)), __fadd_rn(s.a, s.b));
+                    s.dist2 = __fadd_rn(__fsub_rn(rdist[r2], __fadd_rn(d_p2_n2, d_n2_s2)), __fadd_rn(s.c, s.d));
+                    s.ok = s.ok && gain < -kEps &&
+                           !((s.load1 > capacity || s.load2 > capacity) || (s.dist1 > max_dist || s.dist2 > max_dist));
+                } else {
+                    s.load1 = s.load2 = load_1;
+                    s.dist1 = s.dist2 = __fadd_rn(dist_1, gain);
+                    s.ok = s.ok && gain < -kEps;
                 }
-            }
-            const unsigned m = __ballot_sync(FULL, cand);
-            if (m) {
-                const int src = __ffs(m) - 1;
-                const int jj = __shfl_sync(FULL, j, src), nn2 = __shfl_sync(FULL, n2, src);
-                const int l1 = __shfl_sync(FULL, load1, src), l2 = __shfl_sync(FULL, load2, src);
-                const float e1 = __shfl_sync(FULL, dist1, src), e2 = __shfl_sync(FULL, dist2, src);
-                if (lane == 0) {
-                    const int p2 = rpos[jj];
-                    tour[i] = nn2;
-                    tour[jj] = n1;
-                    rload[p1] = l1;
-                    rload[p2] = l2;
-                    rdist[p1] = e1;
-                    rdist[p2] = e2;
+                return s;
+            };
+            for (int j0 = i + 1; j0 < size; j0 += 64) { // two groups of 32 with their reads in flight together
+                int x0, x1;
+                const Swap c0 = eval(j0 + lane, x0), c1 = eval(j0 + 32 + lane, x1);
+                const unsigned m0 = __ballot_sync(FULL, c0.ok), m1 = __ballot_sync(FULL, c1.ok);
+                if (m0 | m1) {
+                    hit = m0 ? c0 : c1;
+                    hit_lane = __ffs(m0 ? m0 : m1) - 1;
+                    hit_j = j0 + (m0 ? 0 : 32) + hit_lane;
+                    hit_n2 = m0 ? x0 : x1; // this lane's; the hit lane's is the one applied
+                    break;
                 }
-                __syncwarp();
-                moved = true;
-                if (++swaps > max_swaps) over = true;
-                break;
             }
         }
-        if (!moved) i++; // an accepted swap re-examines position i (the reference's i--)
+        if (lane == 0) s_found[warp] = hit_j;
+        __syncthreads();
+        const unsigned any = __ballot_sync(FULL, lane < W && s_found[lane & (kMaxWarps - 1)] != 0);
+        if (any) {
+            const int w = __ffs(any) - 1;
+            if (warp == w && lane == hit_lane) {
+                const int r1 = rpos[i], r2 = rpos[hit_j];
+                tour[i] = (uint16_t)hit_n2;
+                tour[hit_j] = (uint16_t)n1;
+                rload[r1] = hit.load1;
+                rload[r2] = hit.load2;
+                rdist[r1] = hit.dist1;
+                rdist[r2] = hit.dist2;
+                edge[i - 1] = hit.a;
+                edge[hit_j] = hit.d;
+                if (hit_j == i + 1) {
+                    edge[i] = __ldg(D + (size_t)hit_n2 * ld + n1);
+                } else {
+                    edge[i] = hit.b;
+                    edge[hit_j - 1] = hit.c;
+                }
+            }
+            i0 += w; // an accepted swap re-examines its position (the reference's i--)
+            over = ++swaps > max_swaps;
+        } else {
+            i0 += W;
+        }
+        __syncthreads();
     }
-    if (over && lane == 0) set_status(a.status, ACO_ERR_LS_LIMIT);
-    for (int p = lane; p < size; p += 32) gt[p] = tour[p];
+    if (over && threadIdx.x == 0) set_status(a.status, ACO_ERR_LS_LIMIT);
+    for (int p = threadIdx.x; p < size; p += blockDim.x) gt[p] = tour[p];
+    if (warp != 0) return;
     // compute_tour_length: fp32 sum of the edges in position order
     float len = 0.f;
     for (int b0 = 0; b0 < size - 1; b0 += 32) {
-        const int p = b0 + lane;
-        const float e = p < size - 1 ? D[(size_t)tour[p] * ldd + tour[p + 1]] : 0.f;
+        const float e = b0 + lane < size - 1 ? edge[b0 + lane] : 0.f;
         const int m = size - 1 - b0 < 32 ? size - 1 - b0 : 32;
 #pragma unroll
         for (int k = 0; k < 32; k++) {
@@ -162,52 +212,18 @@ __device__ void swap_ant(const ConstructArgs &a, int ant, const float *D, int ld
         }
     }
     if (lane == 0) a.lens[ant] = len;
-    (void)n;
-}
-
-__global__ void __launch_bounds__(512) swap_kernel(const ConstructArgs *args, const int2 *items, int apc,
-                                                   int max_swaps_per_node)
-{
-    extern __shared__ __align__(16) unsigned char sm[];
-    const int2 it = items[blockIdx.x];
-    const ConstructArgs a = args[it.x];
-    const int n = a.n, warp = threadIdx.x >> 5;
-    const bool stage = swap_stage_matrix(n, a.ld, apc);
-    const float *D = a.dist;
-    int ldd = a.ld;
-    size_t off = 0;
-    if (stage) { // whole matrix, rows of n (only the first n columns are read)
-        float *sd = reinterpret_cast<float *>(sm);
-        for (int e = threadIdx.x; e < n * n; e += blockDim.x) sd[e] = a.dist[(size_t)(e / n) * a.ld + (e % n)];
-        D = sd;
-        ldd = n;
-        off = ((size_t)n * n * 4 + 15) & ~(size_t)15;
-        __syncthreads();
-    }
-    const int ant = it.y + warp;
-    if (warp >= apc || ant >= a.n_ants) return;
-    int *w = reinterpret_cast<int *>(sm + off + (size_t)warp * swap_warp_bytes(n));
-    int *tour = w, *rpos = w + 2 * n, *rload = w + 4 * n;
-    float *rdist = reinterpret_cast<float *>(w + 5 * n);
-    const int limit = max_swaps_per_node * n;
-    if (stage) swap_ant<true>(a, ant, D, ldd, tour, rpos, rload, rdist, limit);
-    else swap_ant<false>(a, ant, D, ldd, tour, rpos, rload, rdist, limit);
 }
 
 } // namespace
 
-size_t swap_smem(int n, int ld, int apc)
-{
-    return (swap_stage_matrix(n, ld, apc) ? (((size_t)n * n * 4 + 15) & ~(size_t)15) : 0) +
-           (size_t)apc * swap_warp_bytes(n);
-}
+size_t swap_smem(int n) { return swap_layout(n).bytes; }
 
-cudaError_t launch_swap(const ConstructArgs *d_args, const int2 *d_items, int n_items, int apc, size_t smem,
-                        int max_swaps_per_node, cudaStream_t st)
+cudaError_t launch_swap(const ConstructArgs *d_args, const int *d_ant_inst, const int *d_ant_base, int total_ants,
+                        int warps, size_t smem, int max_swaps_per_node, cudaStream_t st)
 {
     const cudaError_t e = cudaFuncSetAttribute(swap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    swap_kernel<<<n_items, apc * 32, smem, st>>>(d_args, d_items, apc, max_swaps_per_node);
+    swap_kernel<<<total_ants, warps * 32, smem, st>>>(d_args, d_ant_inst, d_ant_base, max_swaps_per_node);
     return cudaGetLastError();
 }
 
