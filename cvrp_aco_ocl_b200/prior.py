@@ -1,9 +1,9 @@
 """Learned sampling prior: an edge-scoring message-passing network whose output
 multiplies eta^beta in the ant colony's choice weights.
 
-* ``build_graph``: the k-nearest-customer graph of an instance (the
-  reference's neighbour-list rule, cvrp_ocl/vrpHelper.cpp:188-236) with node
-  features (x, y, demand/capacity, is_depot, distance to the depot) and edge
+* ``build_graph`` (on the device: ``GraphBatch.from_problem``): the
+  k-nearest-customer graph of an instance (the reference's neighbour-list rule,
+  cvrp_ocl/vrpHelper.cpp:188-236) with node features (x, y, demand/capacity, is_depot, distance to the depot) and edge
   feature distance, all lengths divided by the bounding box's longer side.
 * ``EdgeScorer``: parameters on the device; forward, gradient and Adam steps
   are the hand-written kernels of csrc/mpnn.cu (tcgen05 BF16 products, FP32
@@ -35,6 +35,8 @@ DEFAULT_GAMMA = 2.0  # prior exponent: the best final lengths of the 0.5 / 1 / 2
 DEFAULT_WEIGHTS = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data", "edge_prior_k20_l3.npz")
 HIDDEN = 64
 NODE_FEATURES = 5
+DEVICE_LIST_NODES = 25600  # rows of the device's list kernel fit shared memory up to here
+GEO = 2  # instances.GEO
 
 
 @dataclasses.dataclass
@@ -59,18 +61,24 @@ def build_graph(problem, k: int = K_GRAPH, keep_dist: bool = True) -> Graph:
     y = np.asarray(problem.y, np.float32)
     dist = problem.distance if problem.distance is not None else compute_distances(x, y, problem.dis_type)
     nn = compute_nn_lists(dist, k, k)[:, :k]
-    xmin, ymin = float(x.min()), float(y.min())
-    s = max(float(x.max()) - xmin, float(y.max()) - ymin)
-    s = s if s > 0 else 1.0
-    nf = np.zeros((n, NODE_FEATURES), np.float32)
-    nf[:, 0] = (x - xmin) / s
-    nf[:, 1] = (y - ymin) / s
-    nf[:, 2] = np.asarray(problem.demand, np.float32) / float(problem.vehicle_capacity)
-    nf[0, 3] = 1.0
+    nf, s = _node_features(problem, x, y)
     nf[:, 4] = dist[:, 0] / s
     rows = np.repeat(np.arange(n), k)
     ef = (dist[rows, nn.ravel()] / s).astype(np.float32)
     return Graph(n, k, nf, ef, nn.ravel().astype(np.int32), dist if keep_dist else None)
+
+
+def _node_features(problem, x: np.ndarray, y: np.ndarray) -> Tuple[np.ndarray, float]:
+    """Node features without the distance to the depot (column 4), and the length unit."""
+    xmin, ymin = float(x.min()), float(y.min())
+    s = max(float(x.max()) - xmin, float(y.max()) - ymin)
+    s = s if s > 0 else 1.0
+    nf = np.zeros((x.shape[0], NODE_FEATURES), np.float32)
+    nf[:, 0] = (x - xmin) / s
+    nf[:, 1] = (y - ymin) / s
+    nf[:, 2] = np.asarray(problem.demand, np.float32) / float(problem.vehicle_capacity)
+    nf[0, 3] = 1.0
+    return nf, s
 
 
 def route_labels(g: Graph, tour) -> np.ndarray:
@@ -102,6 +110,48 @@ class GraphBatch:
         self.labels = None
         if labels is not None:
             self.labels = torch.from_numpy(np.concatenate(labels).astype(np.float32)).to(dev)
+
+    @classmethod
+    def from_problem(cls, problem, k: int = K_GRAPH, device: int = 0) -> Tuple["GraphBatch", np.ndarray]:
+        """One instance's graph built on the device (``build_graph``'s, bit for bit) and its
+        neighbour ids on the host.  Distances and lists take the device entry points (1001
+        nodes: 7.2 ms on one host core, 0.3 ms here); GEO distances, whose bits depend on the
+        math library, come from the host."""
+        import torch
+
+        from .aco import compute_distances
+
+        x = np.ascontiguousarray(problem.x, np.float32)
+        y = np.ascontiguousarray(problem.y, np.float32)
+        n = x.shape[0]
+        if n - 2 < k:
+            raise ValueError(f"graph degree {k} needs at least {k + 2} nodes, the instance has {n}")
+        nf, s = _node_features(problem, x, y)
+        dev = torch.device("cuda", device)
+        with torch.cuda.device(dev):
+            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+            given = problem.distance
+            if given is None and problem.dis_type == GEO:
+                given = compute_distances(x, y, problem.dis_type)
+            if given is not None:
+                dist = torch.from_numpy(np.ascontiguousarray(given, np.float32)).to(dev)
+            else:
+                xy = torch.from_numpy(np.stack([x, y])).to(dev)
+                dist = torch.empty((n, n), dtype=torch.float32, device=dev)
+                check(lib().aco_compute_distances_device(n, xy[0].data_ptr(), xy[1].data_ptr(), int(problem.dis_type),
+                                                         dist.data_ptr(), n, stream), "aco_compute_distances_device")
+            nbr = torch.empty((n, k), dtype=torch.int32, device=dev)
+            depth = ctypes.c_int()
+            check(lib().aco_compute_nn_lists_device(n, dist.data_ptr(), n, k, k, nbr.data_ptr(), ctypes.byref(depth),
+                                                    stream), "aco_compute_nn_lists_device")
+            unit = torch.tensor(s, dtype=torch.float32, device=dev)  # a tensor: divided, not multiplied by 1/s
+            b = cls.__new__(cls)
+            b.k, b.n_nodes, b.offsets, b.labels = k, n, np.array([0, n]), None
+            b.node_feat = torch.from_numpy(nf).to(dev)
+            b.node_feat[:, 4] = dist[:, 0] / unit
+            b.edge_feat = (torch.gather(dist, 1, nbr.to(torch.int64)) / unit).reshape(-1)
+            b.nbr = nbr.reshape(-1)
+            return b, b.nbr.cpu().numpy()
 
     @property
     def n_edges(self) -> int:
@@ -229,9 +279,14 @@ class EdgeScorer:
     # -- prior for the colony
     def prior(self, problem, gamma: float = DEFAULT_GAMMA, floor: float = 1e-3, k: int = K_GRAPH,
               graph: Optional[Graph] = None) -> np.ndarray:
-        g = graph or build_graph(problem, k)
-        s = self.scores(GraphBatch([g], device=self.device)).cpu().numpy()
-        return prior_matrix(g, s, gamma, floor)
+        given = problem.distance
+        if graph is None and problem.num_node <= DEVICE_LIST_NODES and (given is None or given.dtype == np.float32):
+            batch, nbr = GraphBatch.from_problem(problem, k, self.device)
+            graph = Graph(problem.num_node, k, None, None, nbr, None)  # what prior_matrix reads
+        else:
+            graph = graph or build_graph(problem, k, keep_dist=False)
+            batch = GraphBatch([graph], device=self.device)
+        return prior_matrix(graph, self.scores(batch).cpu().numpy(), gamma, floor)
 
 
 def json_dumps(d) -> str:
