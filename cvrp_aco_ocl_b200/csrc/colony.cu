@@ -331,10 +331,12 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         return o;
     };
     struct Offs {
-        size_t dist, heur, tau, total, chc, dem, key, jump, adv, cand32, nn16, nnls, nnr, seeds, sol, elites, succ,
+        size_t dist, heur, tau, total, chc, dem, demr, perm, rank, key, jump, adv, cand32, nn16, nnr16, order, cdist, nnls, nnr, seeds, sol, elites, succ,
             dep, dtau, rec, nbsf, iter, xy;
     };
     std::vector<Offs> offs(count);
+    bool limited = false; // one instance with a route length limit: all take the kernel that reads cdist
+    for (const InstHost &ih : inst) limited = limited || !std::isinf(ih.max_dist);
     for (int b = 0; b < count; b++) {
         const InstHost &ih = inst[b];
         const size_t nl = (size_t)ih.n * ih.ld * 4;
@@ -347,6 +349,12 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         o.adv = take((size_t)ih.nloc * 4);
         o.cand32 = take((size_t)ih.n * ih.Kp * 4);
         o.nn16 = take((size_t)ih.n * ih.Kp * 2);
+        o.nnr16 = take((size_t)ih.n * ih.Kp * 2);
+        o.cdist = limited ? take((size_t)ih.n * ih.Kp * 4) : 0;
+        o.demr = take((size_t)ih.n4 * 4);
+        o.perm = take(((size_t)ih.n * 2 + 15) & ~(size_t)15);
+        o.rank = take((size_t)ih.n * 2);
+        o.order = ih.K > 0 && ih.n <= kOrderNodes ? take(((size_t)ih.n * 2 + 15) & ~(size_t)15) : 0;
         o.nnls = take((size_t)ih.n * std::max(1, ih.nn_ls) * 4);
         o.nnr = take((size_t)ih.n * sizeof(float2));
         o.seeds = take((size_t)ih.A * ih.nloc * 4);
@@ -437,6 +445,10 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         ih.key_d = (uint32_t *)(base + o.key); ih.jump_d = (uint32_t *)(base + o.jump);
         ih.adv_d = (uint32_t *)(base + o.adv); ih.cand32_d = (uint32_t *)(base + o.cand32);
         ih.nn16_d = (uint16_t *)(base + o.nn16); ih.nnls_d = (int *)(base + o.nnls);
+        ih.nnr16_d = (uint16_t *)(base + o.nnr16); ih.perm_d = (uint16_t *)(base + o.perm);
+        ih.rank_d = (uint16_t *)(base + o.rank); ih.demr_d = (int *)(base + o.demr);
+        ih.order_d = o.order ? (uint16_t *)(base + o.order) : nullptr;
+        ih.cdist_d = o.cdist ? (float *)(base + o.cdist) : nullptr;
         ih.nnr_d = (float2 *)(base + o.nnr);
         ih.seeds_d = (int *)(base + o.seeds); ih.sol_d = (int *)(base + o.sol);
         ih.lens_d = (float *)(base + o_lens_all) + slot_base_h_[b]; ih.elites_d = (int *)(base + o.elites);
@@ -705,7 +717,8 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         pa.n = n; pa.ld = ih.ld; pa.depth = ih.depth; pa.K = ih.K; pa.Kp = ih.Kp; pa.nn_ls = ih.nn_ls;
         pa.dist_type = ih.dist_type; pa.device_prep = ih.device_prep ? 1 : 0; pa.n_ants = ih.A;
         pa.x = ih.xy_d; pa.y = ih.xy_d ? ih.xy_d + ih.n4 : nullptr; pa.dist = ih.dist_d; pa.demand = ih.dem_d;
-        pa.nn16 = ih.nn16_d; pa.cand32 = ih.cand32_d; pa.nnls = ih.nnls_d; pa.nnr = ih.nnr_d; pa.seeds = ih.seeds_d;
+        pa.nn16 = ih.nn16_d; pa.cand32 = ih.cand32_d; pa.nnr16 = ih.nnr16_d; pa.perm = ih.perm_d;
+        pa.rank = ih.rank_d; pa.demr = ih.demr_d; pa.cdist = ih.cdist_d; pa.nnls = ih.nnls_d; pa.nnr = ih.nnr_d; pa.seeds = ih.seeds_d;
         if (ih.device_prep) {
             n_prep = std::max(n_prep, n);
         } else {
@@ -726,16 +739,10 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
             up(ih.adv_d, adv.data(), adv.size() * 4);
         }
         if (ih.K > 0 && !ih.device_prep) {
-            std::vector<uint16_t> nn16((size_t)n * ih.Kp, 0);
-            std::vector<uint32_t> cand32((size_t)n * ih.Kp, 0); // padding entries: node 0 (always visited)
+            std::vector<uint16_t> nn16((size_t)n * ih.Kp, 0); // padding entries: node 0 (always visited)
             for (int i = 0; i < n; i++)
-                for (int j = 0; j < ih.K; j++) {
-                    const int c = ih.nn[(size_t)i * ih.depth + j];
-                    nn16[(size_t)i * ih.Kp + j] = (uint16_t)c;
-                    cand32[(size_t)i * ih.Kp + j] = (uint32_t)c | ((uint32_t)(ih.demand[c] & 0xFFFF) << 16);
-                }
+                for (int j = 0; j < ih.K; j++) nn16[(size_t)i * ih.Kp + j] = (uint16_t)ih.nn[(size_t)i * ih.depth + j];
             up(ih.nn16_d, nn16.data(), nn16.size() * 2);
-            up(ih.cand32_d, cand32.data(), cand32.size() * 4);
         }
         if (!ih.device_prep) {
             std::vector<int> nnls((size_t)n * std::max(1, ih.nn_ls), 0);
@@ -750,7 +757,8 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         c.n = n; c.ld = ih.ld; c.n_ants = ih.A; c.T = ih.T; c.nloc = ih.nloc; c.log2_nloc = ih.lg; c.kmax = ih.kmax;
         c.capacity = ih.capacity; c.max_dist = ih.max_dist; c.serv_time = ih.serv_time;
         c.total = ih.total_d; c.dist = ih.dist_d; c.demand = ih.dem_d; c.tiekey = ih.key_d; c.jump = ih.jump_d;
-        c.adv = ih.adv_d; c.nn16 = ih.nn16_d; c.cand32 = ih.cand32_d; c.chc = ih.chc_d; c.K = ih.K; c.Kp = ih.Kp;
+        c.adv = ih.adv_d; c.demr = ih.demr_d; c.perm = ih.perm_d; c.order = ih.order_d; c.nn16 = ih.nnr16_d; c.cdist = ih.cdist_d;
+        c.cand32 = ih.cand32_d; c.chc = ih.chc_d; c.K = ih.K; c.Kp = ih.Kp;
         c.smat = ih.smat ? 1 : 0; c.packed = ih.packed ? 1 : 0; c.gtab = ih.gtab ? 1 : 0;
         c.nn_list = ih.nnls_d; c.nnr = ih.nnr_d; c.nn_ls = ih.nn_ls; c.pass_limit = p.ls_pass_limit; c.ant_base = ant_base[b];
         c.ls_best = p.ls_best;
@@ -782,7 +790,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         u.n = n; u.ld = ih.ld; u.ras_ranks = ih.R; u.evap = 1.0f - p.rho; u.alpha = p.alpha; u.beta = p.beta;
         u.alpha_int = ai; u.beta_int = bi; u.rho = p.rho; u.tau = ih.tau_d; u.total = ih.total_d; u.heur = ih.heur_d;
         u.dist = ih.dist_d; u.succ = ih.succ_d; u.depmask = ih.dep_d; u.d_tau = ih.dtau_d; u.bsf_len = ih.lens_d + ih.A;
-        u.chc = ih.K > 0 ? ih.chc_d : nullptr; u.nn16 = ih.nn16_d; u.K = ih.K; u.Kp = ih.Kp;
+        u.chc = ih.K > 0 ? ih.chc_d : nullptr; u.nn16 = ih.nn16_d; u.rank = ih.rank_d; u.order = ih.order_d; u.K = ih.K; u.Kp = ih.Kp;
     }
     up(cargs_d_, cargs_h_.data(), sizeof(ConstructArgs) * count);
     up(largs_d_, largs.data(), sizeof(LocalSearchArgs) * count);
@@ -818,14 +826,15 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
 
 int Colony::run_rows(int mode, float trail)
 {
-    CK(launch_rows(uargs_d_, row_base_d_, inst.size() > 1 ? row_inst_d_ : nullptr, total_rows, mode, trail, sm_count,
-                   st));
+    CK(launch_rows(uargs_d_, row_base_d_, inst.size() > 1 ? row_inst_d_ : nullptr, total_rows,
+                   p.mode == ACO_MODE_THROUGHPUT ? (int)inst.size() : 0, mode, trail, sm_count, st));
     return ACO_OK;
 }
 
 int Colony::run_rows_one(int b, int mode)
 {
-    CK(launch_rows(uargs_d_ + b, zero_base_d_, nullptr, inst[b].n, mode, 0.f, sm_count, st));
+    CK(launch_rows(uargs_d_ + b, zero_base_d_, nullptr, inst[b].n, p.mode == ACO_MODE_THROUGHPUT ? 1 : 0, mode, 0.f,
+                   sm_count, st));
     return ACO_OK;
 }
 

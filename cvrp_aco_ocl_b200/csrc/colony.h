@@ -52,7 +52,9 @@ struct InstHost {
     int *dem_d = nullptr, *nnls_d = nullptr, *seeds_d = nullptr, *sol_d = nullptr, *elites_d = nullptr;
     int *succ_d = nullptr, *nbsf_d = nullptr, *iter_d = nullptr;
     uint32_t *key_d = nullptr, *jump_d = nullptr, *adv_d = nullptr, *cand32_d = nullptr, *dep_d = nullptr;
-    uint16_t *nn16_d = nullptr;
+    uint16_t *nn16_d = nullptr, *nnr16_d = nullptr, *perm_d = nullptr, *rank_d = nullptr, *order_d = nullptr;
+    int *demr_d = nullptr;
+    float *cdist_d = nullptr; // null: no route length limit
     float2 *nnr_d = nullptr;
     float *xy_d = nullptr; // device preprocessing: coordinates (x, then y at n4)
     float *lens_d = nullptr, *dtau_d = nullptr;

@@ -25,6 +25,8 @@
 
 namespace aco {
 
+constexpr int kOrderNodes = 1024; // largest instance whose depot row is kept sorted
+
 struct ConstructArgs {
     int n, ld, n_ants, T, nloc, log2_nloc, kmax;
     int capacity;
@@ -35,9 +37,16 @@ struct ConstructArgs {
     const uint32_t *tiekey;// n (padded): ((0xFFFF - prio) << 16) | node
     const uint32_t *jump;  // kmax (padded): 16807^(k+1) mod m
     const uint32_t *adv;   // nloc: 16807^(draws of lane l per step) mod m
-    const uint16_t *nn16;  // n x Kp candidate lists (throughput), uint16 node ids
-    const uint32_t *cand32;// n x Kp candidate lists, packed node | demand << 16
+    // throughput construct: nodes by their rank in (demand, node) order, the depot
+    // rank 0; rows and entries of the candidate tables are ranks
+    const int *demr;       // n (padded): demand of rank r (INT_MIN for the depot)
+    const uint16_t *perm;  // n (padded): node of rank r
+    const uint16_t *nn16;  // n x Kp candidate lists, ranks
+    const uint32_t *cand32;// n x Kp candidate lists, packed rank | demand << 16
     const float *chc;      // n x Kp: 1 / total_info of the candidates (+inf for weight 0)
+    const float *cdist;    // n x Kp: their distances (finite max_dist only)
+    const uint16_t *order; // n (padded): ranks of the customers by total_info from the depot, largest
+                           // first, equal ones by node, or null (never above kOrderNodes nodes)
     int K, Kp;             // candidate-list length and padded row length (multiple of 8)
     int smat;              // throughput construct: stage the whole total_info matrix
     int packed;            // throughput construct: use cand32 (else nn16 + demand lookups)
@@ -114,7 +123,9 @@ struct UpdateArgs {
     const float *d_tau;
     const float *bsf_len;    // lens[A] (trail_0 = 1/(rho * bsf))
     float *chc;              // n x Kp reciprocal candidate weights, or null (no candidate table)
-    const uint16_t *nn16;    // n x Kp
+    const uint16_t *nn16;    // n x Kp candidate lists (node ids)
+    const uint16_t *rank;    // n: the candidate table's row of a node (ConstructArgs)
+    uint16_t *order;         // n: written with the candidate table (ConstructArgs), or null
     int K, Kp;
 };
 
@@ -183,7 +194,7 @@ cudaError_t launch_stats(const StatsArgs *d_args, int n_inst, int do_elites, siz
 // one warp per row over all instances; d_row_base[b] = first global row of instance b,
 // d_row_inst[g] = the instance of global row g (null: one instance).
 cudaError_t launch_rows(const UpdateArgs *d_args, const int *d_row_base, const int *d_row_inst, int total_rows,
-                        int mode, float trail, int sm_count, cudaStream_t st);
+                        int sorted, int mode, float trail, int sm_count, cudaStream_t st);
 // lens[A] = +inf, num_bsf = 0, iteration = 0 of every instance (init_aco).
 cudaError_t launch_reset_slots(const StatsArgs *d_args, int count, cudaStream_t st);
 cudaError_t launch_t0(unsigned long long *t0, cudaStream_t st);
@@ -238,16 +249,21 @@ struct PrepArgs {
     const float *x, *y;
     float *dist;
     const int *demand;
-    uint16_t *nn16;   // n x Kp: first K of the list, padded with node 0
-    uint32_t *cand32; // n x Kp: the same with the demand in the high half
+    uint16_t *nn16;   // n x Kp: first K of the list, padded with node 0 (from the host without device_prep)
+    // the construct's tables by demand rank (ConstructArgs), made here for every instance
+    int *demr;
+    uint16_t *perm, *rank, *nnr16;
+    uint32_t *cand32;
+    float *cdist; // null: no route length limit
     int *nnls;        // n x nn_ls: the 2-opt list
     float2 *nnr;      // n: the 2-opt list's last distance (LocalSearchArgs)
     int *seeds;       // n_ants x nloc
 };
 // Every instance of a batch in one launch per step (global row g: row g -
 // row_base[b] of instance b = row_inst[g]; global ant g: ant g - ant_base[b] of
-// b = ant_inst[g]): distances, then the lists (the reference's quicksort per
-// row) with the candidate and 2-opt tables, then the lane seeds (rnd_seed + b).
+// b = ant_inst[g]): distances and demand ranks, then the lists (the reference's
+// quicksort per row) with the candidate and 2-opt tables, then the lane seeds
+// (rnd_seed + b).
 cudaError_t launch_prep_batch(const PrepArgs *d_args, const int *d_row_base, const int *d_row_inst, int total_rows,
                               int n_max, const int *d_ant_base, const int *d_ant_inst, int total_ants, int nloc,
                               int seed_time, int rnd_seed, int *status, int sm_count, cudaStream_t st);

@@ -357,6 +357,7 @@ __device__ __forceinline__ void row_pass(const UpdateArgs &a, int i, int mode, f
     const int n = a.n, q4 = (n + 3) >> 2;
     // the row's candidate ids, fetched with the row's first loads (ROW_GATHER reads them after the row)
     const int cid = a.chc && lane < a.K ? (int)__ldg(a.nn16 + (size_t)i * a.Kp + lane) : 0;
+    const size_t crow = a.chc ? (size_t)__ldg(a.rank + i) * a.Kp : 0; // its row of the candidate table
     const size_t off = (size_t)i * a.ld;
     const float4 *heur4 = reinterpret_cast<const float4 *>(a.heur + off);
     float4 *tau4 = reinterpret_cast<float4 *>(a.tau + off);
@@ -417,29 +418,123 @@ __device__ __forceinline__ void row_pass(const UpdateArgs &a, int i, int mode, f
             else update_row_stream<1, false>(a, i, lane, q4, tau4, heur4, tot4, s_col, s_amt);
         }
     }
-    if (a.chc) { // compact candidate table: chc[i][j] = 1 / total[i][nn[i][j]] (the race's reciprocal weight)
+    if (a.chc) { // compact candidate table: row rank(i) holds 1 / total[i][nn[i][j]] (the race's reciprocal weight)
         // the row was written by this warp; __syncwarp orders those stores before
         // the re-reads below, which read L2, where the lines were just written
         __syncwarp();
-        if (lane < a.K) a.chc[(size_t)i * a.Kp + lane] = __fdiv_rn(1.0f, __ldcg(a.total + off + cid));
+        if (lane < a.K) a.chc[crow + lane] = __fdiv_rn(1.0f, __ldcg(a.total + off + cid));
     }
+}
+
+// Ascending bitonic sort of P <= kOrderNodes keys (a power of two, at least 32) in
+// shared memory: strides below 32 by shuffles in registers, the others through
+// shared memory.
+__device__ __forceinline__ void sort_keys(unsigned long long *key, int P)
+{
+    for (int size = 2; size <= P; size = size < 32 ? 64 : size * 2) {
+        for (int stride = size >> 1; stride >= 32; stride >>= 1) {
+            for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
+                const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+                const unsigned long long x = key[i], y = key[j];
+                if ((x > y) == ((i & size) == 0)) {
+                    key[i] = y;
+                    key[j] = x;
+                }
+            }
+            __syncthreads();
+        }
+        for (int i = threadIdx.x; i < P; i += blockDim.x) { // whole warps: P is a multiple of 32
+            unsigned long long x = key[i];
+            // the first round does every size up to 32
+            for (int sz = size < 32 ? 2 : size; sz <= (size < 32 ? 32 : size); sz *= 2)
+                for (int stride = sz > 32 ? 16 : sz >> 1; stride > 0; stride >>= 1) {
+                    const unsigned long long y = __shfl_xor_sync(FULL, x, stride);
+                    const bool low = (i & stride) == 0, up = (i & sz) == 0;
+                    x = (low == up) == (x < y) ? x : y;
+                }
+            key[i] = x;
+        }
+        __syncthreads();
+    }
+}
+
+// The depot's row of an instance whose candidate table is kept sorted too: the
+// CTA makes the row, its candidate reciprocals, and sorts its customers by
+// total_info (the key is the complement of the value's bits over node and rank).  The
+// construct's steps that find no listed candidate at the depot (6% of them on the
+// batch) then take the first unvisited customer of this order instead of scanning
+// the row.
+__device__ __noinline__ void depot_order(const UpdateArgs &a, int mode, float trail, float *s_amt,
+                                         unsigned long long *s_key)
+{
+    const int n = a.n;
+    int P = 32;
+    while (P < n - 1) P *= 2;
+    const float tr = mode == ROW_INIT_BSF ? __fdiv_rn(1.0f, __fmul_rn(a.rho, *a.bsf_len)) : trail;
+    const int cid = (int)threadIdx.x < a.K ? __ldg(a.nn16 + threadIdx.x) : 0; // the depot's candidates
+    if (mode == ROW_UPDATE) { // the elites' amounts, read once
+        if ((int)threadIdx.x < a.ras_ranks) s_amt[threadIdx.x] = __ldg(a.d_tau + threadIdx.x);
+        __syncthreads();
+    }
+    for (int c = threadIdx.x; c < n; c += blockDim.x) { // a column each, the row passes' operations
+        const uint32_t rank = __ldg(a.rank + c);
+        float tot;
+        if (mode == ROW_GATHER) {
+            tot = a.total[c];
+        } else {
+            const float h = a.heur[c];
+            float t;
+            if (mode == ROW_UPDATE) {
+                t = __fmul_rn(a.evap, a.tau[c]);
+                const uint32_t m = __ldg(a.depmask + c);
+                for (int r = 0; r < a.ras_ranks; r++)
+                    if ((m >> r) & 1u) t = __fadd_rn(t, s_amt[r]);
+            } else {
+                t = mode == ROW_TOTAL ? a.tau[c] : tr;
+            }
+            tot = __fmul_rn(pow_rule(t, a.alpha, a.alpha_int), h);
+            if (mode != ROW_TOTAL) a.tau[c] = t;
+            a.total[c] = tot;
+        }
+        if (c > 0) s_key[c - 1] = ((unsigned long long)~__float_as_uint(tot) << 32) | ((uint32_t)c << 16) | rank;
+    }
+    for (int k = n - 1 + threadIdx.x; k < P; k += blockDim.x) s_key[k] = ~0ull;
+    __syncthreads();
+    if ((int)threadIdx.x < a.K) // the depot is rank 0: the table's first row
+        a.chc[threadIdx.x] = __fdiv_rn(1.0f, __uint_as_float(~(uint32_t)(s_key[cid - 1] >> 32)));
+    __syncthreads();
+    sort_keys(s_key, P);
+    for (int k = threadIdx.x; k < n - 1; k += blockDim.x) a.order[k] = (uint16_t)s_key[k];
 }
 
 // Global row g (over the instances' rows in order) belongs to instance
 // row_inst[g] (null: a single instance); row_base[b] is instance b's first.
+// The first `sorted` CTAs take the instances' depot rows where these are kept
+// sorted (depot_order); the others the rest.
 template <int MODE>
 __global__ void __launch_bounds__(kRowWarps * 32, 4) rows_kernel(const UpdateArgs *args, const int *row_base,
-                                                                 const int *row_inst, int total_rows, float trail)
+                                                                 const int *row_inst, int total_rows, int sorted,
+                                                                 float trail)
 {
     constexpr int mode = MODE;
+    constexpr bool kTable = MODE != ROW_HEUR && MODE != ROW_PRIOR; // the candidate table is made
     __shared__ int s_col[kRowWarps][32];
     __shared__ float s_amt[kRowWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
+    if (kTable) {
+        __shared__ unsigned long long s_key[kOrderNodes];
+        if ((int)blockIdx.x < sorted) {
+            if (args[blockIdx.x].order) depot_order(args[blockIdx.x], mode, trail, s_amt[0], s_key);
+            return;
+        }
+    }
+    const int gw = ((blockIdx.x - (kTable ? sorted : 0)) * blockDim.x + threadIdx.x) >> 5;
+    const int nw = ((gridDim.x - (kTable ? sorted : 0)) * blockDim.x) >> 5;
     for (int g = gw; g < total_rows; g += nw) {
         const int b = row_inst ? __ldg(row_inst + g) : 0;
-        row_pass(args[b], g - __ldg(row_base + b), mode, trail, lane, s_col[warp], s_amt[warp]);
+        const int i = g - __ldg(row_base + b);
+        if (kTable && i == 0 && sorted > 0 && args[b].order) continue;
+        row_pass(args[b], i, mode, trail, lane, s_col[warp], s_amt[warp]);
     }
 }
 
@@ -479,31 +574,21 @@ cudaError_t launch_stats(const StatsArgs *d_args, int n_inst, int do_elites, siz
 }
 
 cudaError_t launch_rows(const UpdateArgs *d_args, const int *d_row_base, const int *d_row_inst, int total_rows,
-                        int mode, float trail, int sm_count, cudaStream_t st)
+                        int sorted, int mode, float trail, int sm_count, cudaStream_t st)
 {
     int blocks = (total_rows + kRowWarps - 1) / kRowWarps; // one warp per row
     const int cap = sm_count * 4;      // grid-stride beyond 4 CTAs (32 warps) per SM
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    switch (mode) {
-    case ROW_HEUR: rows_kernel<ROW_HEUR><<<blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, trail); break;
-    case ROW_INIT_TRAIL:
-        rows_kernel<ROW_INIT_TRAIL><<<blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, trail);
-        break;
-    case ROW_INIT_BSF:
-        rows_kernel<ROW_INIT_BSF><<<blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, trail);
-        break;
-    case ROW_UPDATE:
-        rows_kernel<ROW_UPDATE><<<blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, trail);
-        break;
-    case ROW_PRIOR:
-        rows_kernel<ROW_PRIOR><<<blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, trail);
-        break;
-    case ROW_TOTAL:
-        rows_kernel<ROW_TOTAL><<<blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, trail);
-        break;
-    default: rows_kernel<ROW_GATHER><<<blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, trail); break;
-    }
+    if (mode == ROW_HEUR || mode == ROW_PRIOR) sorted = 0;
+    auto kern = mode == ROW_HEUR         ? rows_kernel<ROW_HEUR>
+                : mode == ROW_INIT_TRAIL ? rows_kernel<ROW_INIT_TRAIL>
+                : mode == ROW_INIT_BSF   ? rows_kernel<ROW_INIT_BSF>
+                : mode == ROW_UPDATE     ? rows_kernel<ROW_UPDATE>
+                : mode == ROW_PRIOR      ? rows_kernel<ROW_PRIOR>
+                : mode == ROW_TOTAL      ? rows_kernel<ROW_TOTAL>
+                                         : rows_kernel<ROW_GATHER>;
+    kern<<<sorted + blocks, kRowWarps * 32, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows, sorted, trail);
     return cudaGetLastError();
 }
 

@@ -162,7 +162,9 @@ __global__ void nn_kernel(int n, const float *dist, int ld, int depth, int rows_
 }
 
 
-// Distances of every instance's rows, a warp per row (same bits as dist_kernel).
+// Distances of every instance's rows, a warp per row (same bits as dist_kernel),
+// and the node's rank by (demand, node) for the construct's tables: the number
+// of customers before it, the depot first.
 __global__ void dist_rows_kernel(const PrepArgs *pa, const int *row_base, const int *row_inst, int total_rows)
 {
     const int lane = threadIdx.x & 31;
@@ -170,17 +172,32 @@ __global__ void dist_rows_kernel(const PrepArgs *pa, const int *row_base, const 
     for (int g = w0; g < total_rows; g += nw) {
         const int b = row_inst[g];
         const PrepArgs &a = pa[b];
-        if (!a.device_prep) continue;
         const int i = g - row_base[b];
+        if (a.K > 0) {
+            const int d = a.demand[i];
+            int before = 0;
+            if (i != 0)
+                for (int j = 1 + lane; j < a.n; j += 32) {
+                    const int e = a.demand[j];
+                    before += e < d || (e == d && j < i);
+                }
+            const int r = i != 0 ? 1 + (int)__reduce_add_sync(0xffffffffu, (unsigned)before) : 0;
+            if (lane == 0) {
+                a.rank[i] = (uint16_t)r;
+                a.perm[r] = (uint16_t)i;
+                a.demr[r] = i != 0 ? d : (int)0x80000000;
+            }
+        }
+        if (!a.device_prep) continue;
         float *row = a.dist + (size_t)i * a.ld;
         for (int j = lane; j < a.n; j += 32) row[j] = dist_of(a.x, a.y, a.dist_type, i, j);
     }
 }
 
 // Lists and tables of every instance's rows: a warp per row stages it and picks
-// its list (row_list, as nn_kernel), and the lanes write the candidate tables
-// (first K, padded with node 0 to Kp; demand in the high half of cand32) and
-// the 2-opt list (first nn_ls) straight from the list.
+// its list (row_list, as nn_kernel), and the lanes write the candidate list
+// (first K, padded with node 0 to Kp) and the 2-opt list (first nn_ls) straight
+// from the list; then, with host-made lists too, the construct's tables by rank.
 __global__ void lists_rows_kernel(const PrepArgs *pa, const int *row_base, const int *row_inst, int total_rows,
                                   int rows_per_cta, int n_max, int *status)
 {
@@ -191,33 +208,41 @@ __global__ void lists_rows_kernel(const PrepArgs *pa, const int *row_base, const
     for (int g = blockIdx.x * rows_per_cta + w; g < total_rows; g += gridDim.x * rows_per_cta) {
         const int b = row_inst[g];
         const PrepArgs &a = pa[b];
-        if (!a.device_prep || a.depth <= 0) continue;
         const int n = a.n, i = g - row_base[b];
-        for (int k = lane; k < n; k += 32) {
-            v[k] = a.dist[(size_t)i * a.ld + k];
-            idx[k] = k;
+        const size_t crow = (size_t)i * a.Kp;
+        if (a.device_prep && a.depth > 0) {
+            for (int k = lane; k < n; k += 32) {
+                v[k] = a.dist[(size_t)i * a.ld + k];
+                idx[k] = k;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                v[i] = __int_as_float(0x7f800000); // the node itself and the depot never make the list
+                v[0] = __int_as_float(0x7f800000);
+            }
+            __syncwarp();
+            row_list(v, idx, n, a.depth, lane, status);
+            if (a.K > 0)
+                for (int j = lane; j < a.Kp; j += 32) a.nn16[crow + j] = (uint16_t)(j < a.K ? idx[j] : 0);
+            for (int j = lane; j < a.nn_ls; j += 32) a.nnls[(size_t)i * a.nn_ls + j] = idx[j];
+            if (a.nn_ls > 0) { // the list's last distance, and whether unlisted nodes are as far
+                const float *row = a.dist + (size_t)i * a.ld;
+                const float last = row[idx[a.nn_ls - 1]];
+                int more = 0; // nodes at that distance, less the listed ones
+                for (int k = lane; k < n; k += 32) more += k != 0 && k != i && row[k] == last;
+                for (int j = lane; j < a.nn_ls; j += 32) more -= row[idx[j]] == last;
+                more = __reduce_add_sync(0xffffffffu, more);
+                if (lane == 0) a.nnr[i] = make_float2(last, more != 0 ? 1.f : 0.f);
+            }
         }
-        __syncwarp();
-        if (lane == 0) {
-            v[i] = __int_as_float(0x7f800000); // the node itself and the depot never make the list
-            v[0] = __int_as_float(0x7f800000);
-        }
-        __syncwarp();
-        row_list(v, idx, n, a.depth, lane, status);
-        for (int j = lane; j < a.Kp; j += 32) {
-            const int c = j < a.K ? idx[j] : 0;
-            a.nn16[(size_t)i * a.Kp + j] = (uint16_t)c;
-            a.cand32[(size_t)i * a.Kp + j] = (uint32_t)c | ((uint32_t)(a.demand[c] & 0xFFFF) << 16);
-        }
-        for (int j = lane; j < a.nn_ls; j += 32) a.nnls[(size_t)i * a.nn_ls + j] = idx[j];
-        if (a.nn_ls > 0) { // the list's last distance, and whether unlisted nodes are as far
-            const float *row = a.dist + (size_t)i * a.ld;
-            const float last = row[idx[a.nn_ls - 1]];
-            int more = 0; // nodes at that distance, less the listed ones
-            for (int k = lane; k < n; k += 32) more += k != 0 && k != i && row[k] == last;
-            for (int j = lane; j < a.nn_ls; j += 32) more -= row[idx[j]] == last;
-            more = __reduce_add_sync(0xffffffffu, more);
-            if (lane == 0) a.nnr[i] = make_float2(last, more != 0 ? 1.f : 0.f);
+        if (a.K > 0) {
+            const size_t rrow = (size_t)a.rank[i] * a.Kp;
+            for (int j = lane; j < a.Kp; j += 32) { // a lane reads back the entries it wrote
+                const int c = a.nn16[crow + j], r = a.rank[c];
+                a.nnr16[rrow + j] = (uint16_t)r;
+                a.cand32[rrow + j] = (uint32_t)r | ((uint32_t)(a.demand[c] & 0xFFFF) << 16);
+                if (a.cdist) a.cdist[rrow + j] = a.dist[(size_t)i * a.ld + c];
+            }
         }
         __syncwarp(); // the row's buffers are reused by the warp's next row
     }
