@@ -51,6 +51,8 @@ size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Uploads collected into one host blob; flush() copies it to a temporary
 // device buffer in one transfer and scatters the pieces with one kernel.
+constexpr size_t kScatterPiece = 16 * 1024; // a CTA's share of a large upload
+
 struct Staging {
     std::vector<unsigned char> blob;
     std::vector<ScatterPiece> pieces;
@@ -60,8 +62,9 @@ struct Staging {
         const size_t off = (blob.size() + 15) & ~(size_t)15;
         blob.resize(off + bytes);
         std::memcpy(blob.data() + off, src, bytes);
-        pieces.push_back(ScatterPiece{(unsigned long long)(uintptr_t)dst, (unsigned long long)off,
-                                      (unsigned long long)bytes});
+        for (size_t at = 0; at < bytes; at += kScatterPiece)
+            pieces.push_back(ScatterPiece{(unsigned long long)(uintptr_t)dst + at, (unsigned long long)(off + at),
+                                          (unsigned long long)std::min(kScatterPiece, bytes - at)});
     }
     cudaError_t flush(cudaMemPool_t pool, int sm_count, cudaStream_t st)
     {
@@ -75,7 +78,7 @@ struct Staging {
         e = cudaMemcpyAsync(d, blob.data(), blob.size(), cudaMemcpyHostToDevice, st); // pageable: staged on return
         if (e == cudaSuccess)
             e = launch_scatter(reinterpret_cast<const ScatterPiece *>(static_cast<unsigned char *>(d) + poff),
-                               (int)pieces.size(), static_cast<const unsigned char *>(d), poff, sm_count, st);
+                               (int)pieces.size(), static_cast<const unsigned char *>(d), sm_count, st);
         const cudaError_t f = cudaFreeAsync(d, st);
         blob.clear();
         pieces.clear();

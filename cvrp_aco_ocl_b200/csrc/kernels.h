@@ -149,8 +149,8 @@ enum RowMode {
 struct ScatterPiece {
     unsigned long long dst, src_off, bytes;
 };
-cudaError_t launch_scatter(const ScatterPiece *d_pieces, int count, const unsigned char *d_blob,
-                           unsigned long long total_bytes, int sm_count, cudaStream_t st);
+cudaError_t launch_scatter(const ScatterPiece *d_pieces, int count, const unsigned char *d_blob, int sm_count,
+                           cudaStream_t st);
 
 cudaError_t launch_construct_parity(const ConstructArgs &a, int warps_per_ant, int ants_per_block, bool stage_total,
                                     cudaStream_t st);

@@ -10,8 +10,8 @@
 // differ between math libraries; it stays on the host.
 //
 // Lists: one warp per row stages it; when the list's nodes and the next one have
-// distinct distances the warp extracts them by repeated warp minima, otherwise
-// its first lane runs the reference's quicksort (middle pivot swapped to the
+// distinct distances the warp collects and sorts them (row_list), otherwise
+// it runs the reference's quicksort (middle pivot swapped to the
 // left end, Lomuto partition with strict <, both halves recursed) on its row in
 // shared memory.  Only positions below the list depth
 // are needed, so ranges starting at or beyond it are skipped; the ranges are
@@ -93,48 +93,139 @@ __device__ void sort_row(float *v, int *idx, int n, int depth, int *status)
     }
 }
 
+// The same sort of a whole row by the warp.  While the range [0, r] is long and the
+// part right of the pivot starts at or beyond `depth`, only the left part is ever
+// looked at again, and the partition leaves it in a simple order: the smaller
+// elements in their order, the last of them first, the pivot at the end.  The warp
+// makes that by compaction; lane 0 sorts what is left as written.
+__device__ void sort_row_warp(float *v, int *idx, int n, int depth, int lane, int *status)
+{
+    const unsigned FULLM = 0xffffffffu;
+    auto swap = [&](int a, int b) {
+        if (lane == 0) {
+            const float tv = v[a]; v[a] = v[b]; v[b] = tv;
+            const int ti = idx[a]; idx[a] = idx[b]; idx[b] = ti;
+        }
+        __syncwarp();
+    };
+    int r = n - 1;
+    while (r >= 64) {
+        swap(0, r / 2);
+        const float pv = v[0];
+        int last = 0;
+        for (int k = 1 + lane; k <= r; k += 32) last += v[k] < pv;
+        last = (int)__reduce_add_sync(FULLM, (unsigned)last);
+        if (last + 1 < depth) { // the right part is needed too
+            swap(0, r / 2);
+            break;
+        }
+        int cnt = 0;
+        for (int k0 = 1; k0 <= r; k0 += 32) {
+            const int k = k0 + lane;
+            const float x = k <= r ? v[k] : 0.f;
+            const int ix = k <= r ? idx[k] : 0;
+            const bool small = k <= r && x < pv;
+            const unsigned m = __ballot_sync(FULLM, small);
+            if (small) { // at or before its own place: nothing unread is overwritten
+                const int to = 1 + cnt + __popc(m & ((1u << lane) - 1u));
+                v[to] = x;
+                idx[to] = ix;
+            }
+            cnt += __popc(m);
+            __syncwarp();
+        }
+        swap(0, last);
+        r = last;
+    }
+    if (lane == 0) sort_row(v, idx, r + 1, depth, status);
+    __syncwarp();
+}
+
+constexpr int kPick = 64;      // candidates the list's extraction sorts
+constexpr int kListWarps = 8;  // warps (rows) of a CTA of the list kernels
+
 // The first `depth` entries of a staged row's list, warp-wide.  When the
 // depth + 1 smallest values are all distinct, every correct sort puts the same
-// nodes in the first depth positions, so the warp extracts them in depth + 1
-// rounds of a 64-bit warp minimum over (value bits, index) -- for values from
-// +0 to +inf the bits order as the floats.  Otherwise (a tie decides which node
-// comes first, as with integer coordinates, or a row holds a negative value,
-// -0 or NaN) lane 0 runs the reference's quicksort,
-// whose partition order settles ties exactly as the host's.  On return idx[0,
-// depth) holds the list.
-__device__ void row_list(float *v, int *idx, int n, int depth, int lane, int *status)
+// nodes in the first depth positions, so the warp bisects for a value that at
+// least depth + 1 and at most kPick of the row are no larger than, collects those
+// and sorts them by (value bits, index) -- for values from +0 to +inf the bits
+// order as the floats.  Otherwise (a tie decides which node comes first, as with
+// integer coordinates, or a row holds a negative value, -0 or NaN) the reference's
+// quicksort runs (sort_row_warp), whose partition order settles ties exactly as
+// the host's.  On return idx[0, depth) holds the list.  buf: kPick keys of the warp.
+// 25.8 k rows of 101-701 nodes, depth 25: 453 -> 148 us against extracting
+// the minima one by one (a pass over the row for each) and one lane sorting ties.
+__device__ void row_list(float *v, int *idx, unsigned long long *buf, int n, int depth, int lane, int *status)
 {
     const unsigned FULLM = 0xffffffffu;
     if (depth < 32) {
-        unsigned long long prev = 0ull, mine = ~0ull;
-        bool first = true, odd = false; // odd: a negative value, -0 or NaN (their bits do not order as the floats)
-        for (int r = 0; r <= depth; r++) {
-            unsigned long long best = ~0ull;
-            for (int i = lane; i < n; i += 32) {
-                const uint32_t b = __float_as_uint(v[i]);
-                if (first) odd = odd || b > 0x7f800000u;
-                const unsigned long long k = ((unsigned long long)b << 32) | (unsigned)i;
-                if ((first || k > prev) && k < best) best = k;
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const unsigned long long w = __shfl_xor_sync(FULLM, best, o);
-                best = w < best ? w : best;
-            }
-            if (lane == r) mine = best;
-            prev = best;
-            first = false;
+        const uint32_t *bits = reinterpret_cast<const uint32_t *>(v);
+        uint32_t lo = 0x7f800000u, hi = 0u; // smallest, largest finite value
+        bool odd = false;                   // a negative value, -0 or NaN
+        for (int i = lane; i < n; i += 32) {
+            const uint32_t b = bits[i];
+            odd = odd || b > 0x7f800000u;
+            lo = min(lo, b);
+            hi = b < 0x7f800000u ? max(hi, b) : hi;
         }
-        // lanes 0..depth hold the depth + 1 smallest in order: a tie among them ends the fast path
-        const unsigned nxt = __shfl_down_sync(FULLM, (unsigned)(mine >> 32), 1);
-        const bool tie = lane < depth && (unsigned)(mine >> 32) == nxt;
-        if (!__any_sync(FULLM, tie || odd)) {
-            if (lane < depth) idx[lane] = (int)(mine & 0xffffffffu);
+        lo = __reduce_min_sync(FULLM, lo);
+        hi = __reduce_max_sync(FULLM, hi);
+        bool sorted = !__any_sync(FULLM, odd);
+        uint32_t t = 0x7f800000u; // every value is a candidate of a short row
+        if (sorted && n > kPick) {
+            sorted = false;
+            uint32_t below = lo; // the bisection's lower end: too few values up to below - 1
+            for (int it = 0; it < 32 && below <= hi; it++) {
+                t = below + ((hi - below) >> 1);
+                int c = 0;
+                for (int i = lane; i < n; i += 32) c += bits[i] <= t;
+                c = (int)__reduce_add_sync(FULLM, (unsigned)c);
+                if (c > depth && c <= kPick) {
+                    sorted = true;
+                    break;
+                }
+                if (c <= depth) below = t + 1u;
+                else if (t == 0u) break;
+                else hi = t - 1u;
+            }
+        }
+        if (sorted) {
+            int cnt = 0;
+            for (int i0 = 0; i0 < n; i0 += 32) {
+                const int i = i0 + lane;
+                const bool in = i < n && bits[i] <= t;
+                const unsigned m = __ballot_sync(FULLM, in);
+                if (in) buf[cnt + __popc(m & ((1u << lane) - 1u))] = ((unsigned long long)bits[i] << 32) | (unsigned)i;
+                cnt += __popc(m);
+            }
             __syncwarp();
-            return;
+            unsigned long long x = lane < cnt ? buf[lane] : ~0ull, y = lane + 32 < cnt ? buf[lane + 32] : ~0ull;
+            // bitonic sort of 64: positions lane and lane + 32
+            for (int size = 2; size <= 64; size *= 2) {
+                if (size == 64) { // positions lane and lane + 32
+                    const unsigned long long l = x < y ? x : y;
+                    y = x < y ? y : x;
+                    x = l;
+                }
+                for (int stride = size > 32 ? 16 : size >> 1; stride > 0; stride >>= 1) {
+                    const unsigned long long ox = __shfl_xor_sync(FULLM, x, stride), oy = __shfl_xor_sync(FULLM, y, stride);
+                    const bool low = (lane & stride) == 0;
+                    const bool upx = size >= 64 || (lane & size) == 0, upy = size >= 64 || ((lane + 32) & size) == 0;
+                    x = (low == upx) == (x < ox) ? x : ox;
+                    y = (low == upy) == (y < oy) ? y : oy;
+                }
+            }
+            // lanes 0..depth hold the depth + 1 smallest in order: a tie among them ends the fast path
+            const unsigned nxt = __shfl_down_sync(FULLM, (unsigned)(x >> 32), 1);
+            const bool tie = lane < depth && (unsigned)(x >> 32) == nxt;
+            if (!__any_sync(FULLM, tie)) {
+                if (lane < depth) idx[lane] = (int)(x & 0xffffffffu);
+                __syncwarp();
+                return;
+            }
         }
     }
-    if (lane == 0) sort_row(v, idx, n, depth, status);
-    __syncwarp();
+    sort_row_warp(v, idx, n, depth, lane, status);
 }
 
 // One warp per row: the lanes stage the row and pick its list (row_list), the
@@ -142,6 +233,7 @@ __device__ void row_list(float *v, int *idx, int n, int depth, int lane, int *st
 __global__ void nn_kernel(int n, const float *dist, int ld, int depth, int rows_per_cta, int *nn, int *status)
 {
     extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ unsigned long long buf[kListWarps][kPick];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * rows_per_cta + w;
     if (w >= rows_per_cta || row >= n) return;
@@ -157,7 +249,7 @@ __global__ void nn_kernel(int n, const float *dist, int ld, int depth, int rows_
         v[0] = __int_as_float(0x7f800000);
     }
     __syncwarp();
-    row_list(v, idx, n, depth, lane, status);
+    row_list(v, idx, buf[w], n, depth, lane, status);
     for (int i = lane; i < depth; i += 32) nn[(size_t)row * depth + i] = idx[i];
 }
 
@@ -202,6 +294,7 @@ __global__ void lists_rows_kernel(const PrepArgs *pa, const int *row_base, const
                                   int rows_per_cta, int n_max, int *status)
 {
     extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ unsigned long long buf[kListWarps][kPick];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float *v = reinterpret_cast<float *>(sm) + (size_t)w * 2 * n_max;
     int *idx = reinterpret_cast<int *>(v + n_max);
@@ -221,7 +314,7 @@ __global__ void lists_rows_kernel(const PrepArgs *pa, const int *row_base, const
                 v[0] = __int_as_float(0x7f800000);
             }
             __syncwarp();
-            row_list(v, idx, n, a.depth, lane, status);
+            row_list(v, idx, buf[w], n, a.depth, lane, status);
             if (a.K > 0)
                 for (int j = lane; j < a.Kp; j += 32) a.nn16[crow + j] = (uint16_t)(j < a.K ? idx[j] : 0);
             for (int j = lane; j < a.nn_ls; j += 32) a.nnls[(size_t)i * a.nn_ls + j] = idx[j];
@@ -272,7 +365,7 @@ cudaError_t launch_nn(int n, const float *dist, int ld, int depth, int *nn, int 
 {
     int rows = (int)nn_rows_per_cta(n);
     if (rows < 1) return cudaErrorInvalidValue;
-    if (rows > 8) rows = 8; // warps (rows) per CTA
+    if (rows > kListWarps) rows = kListWarps;
     const size_t smem = (size_t)rows * 8 * n;
     cudaError_t e = cudaFuncSetAttribute(nn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -314,37 +407,32 @@ __global__ void seeds_kernel(const PrepArgs *pa, const int *ant_base, const int 
 }
 
 // Scatter of staged uploads: piece k copies bytes [src_off, src_off + bytes)
-// of the blob to dst.  The whole grid works on one piece after another, so a
-// large piece (the seeds) spreads over every CTA.
+// of the blob to dst, a CTA a piece (the host cuts large ones, kScatterPiece).  With
+// the whole grid on one piece after another, 194 pieces took 105 us; now 6.
 __global__ void scatter_kernel(const ScatterPiece *pieces, int count, const unsigned char *blob)
 {
-    const unsigned long long t0 = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-    for (int k = 0; k < count; k++) {
+    for (int k = blockIdx.x; k < count; k += gridDim.x) {
         const ScatterPiece pc = pieces[k];
         unsigned char *dst = reinterpret_cast<unsigned char *>(pc.dst);
         const unsigned char *src = blob + pc.src_off;
-        const unsigned long long b = pc.bytes;
+        const unsigned b = (unsigned)pc.bytes, t0 = threadIdx.x, stride = blockDim.x;
         if (((pc.dst | pc.src_off | b) & 15ull) == 0) {
-            for (unsigned long long i = t0; i < b / 16; i += stride)
+            for (unsigned i = t0; i < b / 16; i += stride)
                 reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
         } else if (((pc.dst | pc.src_off | b) & 3ull) == 0) {
-            for (unsigned long long i = t0; i < b / 4; i += stride)
+            for (unsigned i = t0; i < b / 4; i += stride)
                 reinterpret_cast<uint32_t *>(dst)[i] = reinterpret_cast<const uint32_t *>(src)[i];
         } else {
-            for (unsigned long long i = t0; i < b; i += stride) dst[i] = src[i];
+            for (unsigned i = t0; i < b; i += stride) dst[i] = src[i];
         }
     }
 }
 
-cudaError_t launch_scatter(const ScatterPiece *d_pieces, int count, const unsigned char *d_blob,
-                           unsigned long long total_bytes, int sm_count, cudaStream_t st)
+cudaError_t launch_scatter(const ScatterPiece *d_pieces, int count, const unsigned char *d_blob, int sm_count,
+                           cudaStream_t st)
 {
     if (count <= 0) return cudaSuccess;
-    unsigned long long blocks = (total_bytes / 16 + 255) / 256;
-    if (blocks > (unsigned long long)sm_count * 4) blocks = (unsigned long long)sm_count * 4;
-    if (blocks < 1) blocks = 1;
-    scatter_kernel<<<(unsigned)blocks, 256, 0, st>>>(d_pieces, count, d_blob);
+    scatter_kernel<<<std::min(count, sm_count * 8), 256, 0, st>>>(d_pieces, count, d_blob);
     return cudaGetLastError();
 }
 
@@ -357,7 +445,7 @@ cudaError_t launch_prep_batch(const PrepArgs *d_args, const int *d_row_base, con
         dist_rows_kernel<<<std::max(blocks, 1), 256, 0, st>>>(d_args, d_row_base, d_row_inst, total_rows);
         int rows = (int)nn_rows_per_cta(n_max);
         if (rows < 1) return cudaErrorInvalidValue;
-        if (rows > 8) rows = 8;
+        if (rows > kListWarps) rows = kListWarps;
         const size_t smem = (size_t)rows * 8 * n_max;
         cudaError_t e = cudaFuncSetAttribute(lists_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
