@@ -407,7 +407,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
     {
         int n_max = 0;
         bool sym = true;
-        long long cap = 0;
+        long long cap = 0, routes = 0; // capacity of the list; the most routes an ant needs
         for (const InstHost &ih : inst) {
             n_max = std::max(n_max, ih.n);
             // routes per tour: at least total demand / capacity; twice that plus a margin,
@@ -416,12 +416,15 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
             for (int i = 1; i < ih.n; i++) dem += ih.demand[i];
             const long long per = ih.capacity > 0 ? 2 * ((dem + ih.capacity - 1) / ih.capacity) + 16 : ih.n - 1;
             cap += (long long)ih.A * std::min<long long>(ih.n - 1, per);
+            if (ih.capacity > 0) routes = std::max(routes, dem / ih.capacity);
             sym = sym && ih.sym; // coordinate formulas are symmetric; a given matrix was checked
         }
-        // measured: with few ants per SM the per-ant kernel is as fast (the slowest
-        // route sets the time either way) and the list costs the construct a pass
-        use_routes_ = p.mode == ACO_MODE_THROUGHPUT && (p.ls_flag & 1) && sym && n_max <= 4096 &&
-                      cap < (1ll << 30) && (p.route_ls > 0 || (p.route_ls == 0 && total_ants > 4 * sm_count));
+        // With few ants per SM the per-ant kernel is as fast (the slowest route sets the
+        // time either way) and the list costs the construct a pass: 201 nodes 592 ants 41 us
+        // for 47, 501 nodes 590 ants 84 for 89.  From about 60 routes an ant its warps
+        // queue: 1001 nodes 300 / 590 ants 103 / 147 us, with the list 88 / 138.
+        use_routes_ = p.mode == ACO_MODE_THROUGHPUT && (p.ls_flag & 1) && sym && n_max <= 4096 && cap < (1ll << 30) &&
+                      (p.route_ls > 0 || (p.route_ls == 0 && (total_ants > 4 * sm_count || routes >= 60)));
         route_cap_ = use_routes_ ? (int)cap : 0;
     }
     const size_t o_rdesc = take((size_t)route_cap_ * sizeof(int2)), o_rctr = take(16);
@@ -530,12 +533,19 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         if (cp_apc * cp_wpa > 16) return ACO_ERR_INVALID; // 512 threads per CTA at most
         cp_stage = construct_parity_smem(ih.n, ih.nloc, ih.kmax, wpa, cp_apc, true, fin_any) <= kSmemBudget;
     } else {
-        // ants per work item: enough CTAs to cover the SMs for one instance,
-        // larger items for big batches (the staging is shared by the item's ants)
-        // (one warp per ant, at most 16 warps: the kernel's launch bound is 512 threads)
-        if (p.ants_per_block > 0) cn_apc = std::min(16, p.ants_per_block);
-        else if (count == 1) cn_apc = std::max(1, std::min(8, (inst[0].A + sm_count - 1) / sm_count));
-        else cn_apc = std::max(1, std::min(16, total_ants / (sm_count * 2)));
+        // Ants per work item (one warp per ant, at most 16 warps: the kernel's launch bound
+        // is 512 threads).  An item takes about the time of one ant, so fewer, larger items
+        // finish sooner while every SM has one; items of 8 leave room for a second CTA
+        // on the SM and even out the sizes until there are more than 16 ants an SM.
+        // Construct of one iteration, us: 8 instances x 64 ants at 1 / 4 / 8 ants an item
+        // 294 / 159 / 177; 12 x 128 at 5 / 8 / 16: 364 / 290 / 440; 30 x 64 at 6 / 8 / 16:
+        // 396 / 300 / 451; 64 x 64 at 13 / 16: 322 / 293; 100 x 32 at 10 / 16: 232 / 163.
+        if (p.ants_per_block > 0) {
+            cn_apc = std::min(16, p.ants_per_block);
+        } else {
+            const int per_sm = (total_ants + sm_count - 1) / sm_count;
+            cn_apc = per_sm <= 8 ? per_sm : per_sm <= 16 ? 8 : 16;
+        }
         // helper draw warps while the construct is latency bound (few ants per SM)
         cn_draw = p.draw_warps > 0 || (p.draw_warps == 0 && p.construct_ctas != 2 && total_ants <= 4 * sm_count);
         if (cn_draw) cn_apc = std::min(cn_apc, 8);
@@ -603,6 +613,21 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
             }
         }
         cn_draw = cn_draw && cn_lsw == 0 && cn_apc <= 8; // as the last plan sized the shared memory
+        if (cn_draw && p.draw_warps == 0) {
+            // helper warps whose ring costs a candidate table its place in shared memory are
+            // not worth it (1001 nodes, 450 ants: 367 us, without them 309)
+            auto unstaged = [&]() {
+                int k = 0;
+                for (const InstHost &ih : inst) k += ih.gtab ? 1 : 0;
+                return k;
+            };
+            const int with = unstaged();
+            cn_draw = false;
+            if (with == 0 || !plan(cn_apc, 0, kSmemBudget) || unstaged() >= with) {
+                cn_draw = true;
+                plan(cn_apc, 0, kSmemBudget);
+            }
+        }
     }
     {
         // 2-opt CTA shape: ants per CTA x warps.  Cost model: waves of CTAs over
