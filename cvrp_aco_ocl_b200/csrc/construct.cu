@@ -594,12 +594,10 @@ __device__ void fused_ls_warp(const ConstructArgs &a, unsigned char *smem, const
         } else {
             // as the 2-opt kernels (local_search.cu)
             const int v = lane < R ? (int)tb[rb + lane] : 0;
-            const uint32_t nm = route_tile<8>(lane, R, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, tile);
-            int tq = lane < R ? lane : 0;
-            float dq = lane < R ? tile[lane * kRL + (lane + 1 < R ? lane + 1 : 0)] : 0.f; // dist_tour_wrk
-            const int st = a.ls_best ? two_opt_route_best(lane, R, tile, tpos, tq, dq, a.pass_limit)
-                                     : two_opt_route_regs<false>(lane, R, r == 0, tile, nm, v, a.nn_list, a.nn_ls, tq,
-                                                                 dq, a.pass_limit);
+            int tq;
+            float dq; // dist_tour_wrk
+            const int st = two_opt_route<8>(lane, R, r == 0, a.ls_best, false, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls,
+                                            tile, tpos, tq, dq, a.pass_limit);
             if (st != ACO_OK) status = st;
             const int node = __shfl_sync(kFullMask, v, tq);
             if (lane < R) {

@@ -449,14 +449,10 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
         } else if (small) {
             // lane q holds route node q
             const int v = lane < R ? (int)tour[rb + lane] : 0;
-            const uint32_t nm = route_tile<kLsRows>(lane, R, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, tile);
-            int tq = lane < R ? lane : 0;
-            // edge lengths: position q -> q+1, the last one back to the next depot (node 0 = local 0)
-            float dq = lane < R ? tile[lane * kRL + (lane + 1 < R ? lane + 1 : 0)] : 0.f;
-            st = a.best  ? two_opt_route_best(lane, R, tile, tpos, tq, dq, a.pass_limit)
-                 : a.sym ? two_opt_route_regs<true>(lane, R, r == 0, tile, nm, v, a.nn_list, a.nn_ls, tq, dq, a.pass_limit)
-                         : two_opt_route_regs<false>(lane, R, r == 0, tile, nm, v, a.nn_list, a.nn_ls, tq, dq,
-                                                     a.pass_limit);
+            int tq;
+            float dq;
+            st = two_opt_route<kLsRows>(lane, R, r == 0, a.best, a.sym, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, tile,
+                                        tpos, tq, dq, a.pass_limit);
             const int node = __shfl_sync(FULL, v, tq);
             if (lane < R) {
                 tour[rb + lane] = (uint16_t)node;
@@ -782,13 +778,10 @@ __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs
             __syncwarp();
         } else {
         const int v = lane < R ? gt[rb + lane] : 0;
-        const uint32_t nm = route_tile<kRouteRows>(lane, R, v, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, tile);
-        // edge lengths: position q -> q+1, the last one back to the next depot (node 0 = local 0)
-        int tq = lane < R ? lane : 0;
-        float dq = lane < R ? tile[lane * kRL + (lane + 1 < R ? lane + 1 : 0)] : 0.f;
-        const int st = a.best ? two_opt_route_best(lane, R, tile, tpos, tq, dq, a.pass_limit)
-                              : two_opt_route_regs<true>(lane, R, rb == 0, tile, nm, v, a.nn_list, a.nn_ls, tq, dq,
-                                                         a.pass_limit);
+        int tq;
+        float dq;
+        const int st = two_opt_route<kRouteRows>(lane, R, rb == 0, a.best, true, v, a.dist, a.ld, a.nnr, a.nn_list,
+                                                 a.nn_ls, tile, tpos, tq, dq, a.pass_limit);
         if (st != ACO_OK && lane == 0) set_status(a.status, st);
         const int node = __shfl_sync(FULL, v, tq);
         if (lane < R) __stcs(gt + rb + lane, node); // evict first: not read again before the statistics

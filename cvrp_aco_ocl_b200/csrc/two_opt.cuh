@@ -21,8 +21,10 @@
 //
 // Warp instructions: about 45 an examination and 45 a move (90 and 75 with the
 // lists filtered into shared memory and the partner's words fetched by shuffle),
-// 10 a row to build the tile (60 with the list filtering).  512 instances, 2.9 M
-// routes of 14 nodes: 9.81 -> 6.58 ms; 201 ants with full lists: 74 -> 28 us.
+// 10 a row to build the tile (60 with the list filtering); routes of at most 16
+// nodes take two examinations and two rows at a time.  The issue slots bound it.
+// 512 instances, 2.9 M routes of 14 nodes: 9.81 ms with the lists in shared memory,
+// 6.58 by position, 5.89 with the pairs; 201 ants with full lists: 74 -> 27 us.
 #pragma once
 
 #include <cstdint>
@@ -39,29 +41,34 @@ constexpr unsigned kFullMask = 0xffffffffu;
 // The distance tile of a route and, as the return value of lane k, the mask of
 // the route's customers on the neighbour list of route node k (its own bit and
 // the depot's are never set).  Lane q < R holds route node q's global id (v); a
-// round of ROWS rows has its loads in flight together.
-template <int ROWS>
+// round's loads are in flight together.  PAIR (R <= 16, lanes 16-31 repeat lanes
+// 0-15): each half of the warp takes a row, the tile's rows are 16 entries.
+template <int ROWS, bool PAIR>
 __device__ __forceinline__ uint32_t route_tile(int lane, int R, int v, const float *dist, int ld, const float2 *nnr,
                                                const int *nn, int nn_ls, float *tile)
 {
+    constexpr int W = PAIR ? 16 : kRL, PER = PAIR ? 2 : 1; // row length, rows a load takes
+    const int l = PAIR ? lane & 15 : lane, h = PAIR ? lane >> 4 : 0;
     const uint32_t cust = (R >= 32 ? kFullMask : (1u << R) - 1u) & ~1u;
     float2 last = make_float2(-__int_as_float(0x7f800000), 0.f); // the list's last distance; 1: others share it
     if (lane < R && nn_ls > 0) last = __ldg(nnr + v);
     uint32_t nm = 0u;
-    for (int k0 = 0; k0 < R; k0 += ROWS) {
+    for (int k0 = 0; k0 < R; k0 += PER * ROWS) {
         float d[ROWS];
 #pragma unroll
         for (int u = 0; u < ROWS; u++) {
-            const int node1 = __shfl_sync(kFullMask, v, (k0 + u) & 31);
-            d[u] = (k0 + u < R && lane < R) ? __ldg(dist + (size_t)node1 * ld + v) : 0.f;
+            const int k = k0 + PER * u + h;
+            const int node1 = __shfl_sync(kFullMask, v, k & (W - 1));
+            d[u] = (k < R && l < R) ? __ldg(dist + (size_t)node1 * ld + v) : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < ROWS; u++) {
-            const int k1 = k0 + u;
+            const int k1 = k0 + PER * u;
             if (k1 >= R) break; // warp-uniform
-            tile[k1 * kRL + lane] = d[u];
-            const uint32_t m = __ballot_sync(kFullMask, d[u] <= __shfl_sync(kFullMask, last.x, k1));
-            if (lane == k1) nm = m & cust & ~(1u << k1);
+            tile[k1 * W + lane] = d[u];
+            const uint32_t m =
+                __ballot_sync(kFullMask, d[u] <= __shfl_sync(kFullMask, last.x, (k1 + h) & (W - 1)));
+            if (l / PER == k1 / PER) nm = (PAIR && (l & 1) ? m >> 16 : m) & cust & ~(1u << l);
         }
     }
     // lists that end inside a group of equal distances: look those route nodes up
@@ -69,12 +76,11 @@ __device__ __forceinline__ uint32_t route_tile(int lane, int R, int v, const flo
         const int k1 = __ffs(amb) - 1;
         const float thr = __shfl_sync(kFullMask, last.x, k1);
         const int *list = nn + (size_t)__shfl_sync(kFullMask, v, k1) * nn_ls;
-        for (uint32_t at = __ballot_sync(kFullMask, tile[k1 * kRL + lane] == thr) & cust & ~(1u << k1); at;
-             at &= at - 1u) {
+        for (uint32_t at = __ballot_sync(kFullMask, tile[k1 * W + l] == thr) & cust & ~(1u << k1); at; at &= at - 1u) {
             const int b = __ffs(at) - 1, node = __shfl_sync(kFullMask, v, b);
             bool hit = false;
-            for (int h = lane; h < nn_ls; h += 32) hit = hit || __ldg(list + h) == node;
-            if (!__any_sync(kFullMask, hit) && lane == k1) nm &= ~(1u << b);
+            for (int h1 = lane; h1 < nn_ls; h1 += 32) hit = hit || __ldg(list + h1) == node;
+            if (!__any_sync(kFullMask, hit) && l == k1) nm &= ~(1u << b);
         }
     }
     __syncwarp();
@@ -103,16 +109,23 @@ __device__ __noinline__ int first_listed(uint32_t mv, int lane, float d12, int g
 // node p and edge length, on return the improved route's; nm: lane k's mask
 // (route_tile); v: lane k's global node.  SYM: the distances are symmetric, so
 // an edge's length is its dist_tour_wrk entry (otherwise the tile's).
+// PAIR (R <= 16, lanes 16-31 hold copies of lanes 0-15): lanes 16-31 examine the
+// position after the one that lanes 0-15 examine.  An examination that finds no
+// move changes nothing but its own don't-look bit, so the second one stands when
+// the first finds none, and is dropped otherwise.
 // ---------------------------------------------------------------------------
-template <bool SYM>
+template <bool SYM, bool PAIR>
 __device__ int two_opt_route_regs(int lane, int R, bool first_route, const float *tile, uint32_t nm, int v,
                                   const int *nn, int nn_ls, int &tq, float &dq, int pass_limit)
 {
+    constexpr int W = PAIR ? 16 : kRL;
+    constexpr uint32_t ROW = PAIR ? 0xffffu : kFullMask; // a half's lanes in a ballot
+    const int l = PAIR ? lane & 15 : lane;
     // `open`: bit p set while the don't-look bit of position p's node is clear; a
     // move carries it along with the positions it reverses
     uint32_t open = (R >= 32 ? kFullMask : (1u << R) - 1u) & ~(first_route ? 0u : 1u);
     if (!open) return ACO_OK;
-    const int pn = lane + 1 < R ? lane + 1 : 0, pp = lane > 0 ? lane - 1 : R - 1; // next and previous position
+    const int pn = l + 1 < R ? l + 1 : 0, pp = l > 0 ? l - 1 : R - 1; // next and previous position
     int ts, tp;   // the local nodes there
     float dqp;    // dist_tour_wrk of the previous position
     uint32_t word; // tq | ts << 8 | tp << 16
@@ -127,12 +140,15 @@ __device__ int two_opt_route_regs(int lane, int R, bool first_route, const float
     bool imp = false;
     int q1 = __ffs(open) - 1;
     for (;;) {
-        const uint32_t w1 = __shfl_sync(kFullMask, word, q1), m1 = __shfl_sync(kFullMask, nm, q1);
+        uint32_t next = open & (0xfffffffeu << q1); // open positions left in this pass
+        const int q2 = PAIR && next ? __ffs(next) - 1 : q1;
+        const int q = PAIR && lane >= 16 ? q2 : q1;
+        const uint32_t w1 = __shfl_sync(kFullMask, word, q), m1 = __shfl_sync(kFullMask, nm, q);
         const int k1 = w1 & 0xff, ks1 = (w1 >> 8) & 0xff, kp1 = w1 >> 16;
-        const float d12 = tile[k1 * kRL + tq], xs = tile[ks1 * kRL + ts], xp = tile[kp1 * kRL + tp];
+        const float d12 = tile[k1 * W + tq], xs = tile[ks1 * W + ts], xp = tile[kp1 * W + tp];
         // radii: the examined node's two tour edges
-        const float rs = SYM ? __shfl_sync(kFullMask, dq, q1) : tile[k1 * kRL + ks1];
-        const float rp = SYM ? __shfl_sync(kFullMask, dqp, q1) : tile[kp1 * kRL + k1];
+        const float rs = SYM ? __shfl_sync(kFullMask, dq, q) : tile[k1 * W + ks1];
+        const float rp = SYM ? __shfl_sync(kFullMask, dqp, q) : tile[kp1 * W + k1];
         const bool act = (m1 >> tq) & 1u;
         // successor and predecessor searches (kernel.cl:180-198, 202-230); -r + d is -(r - d)
         const float us = __fsub_rn(rs, d12), up = __fsub_rn(rp, d12);
@@ -140,34 +156,40 @@ __device__ int two_opt_route_regs(int lane, int R, bool first_route, const float
         const uint32_t smove = __ballot_sync(kFullMask, act & (us > kEps) & (gs < -kEps));
         const uint32_t pmove =
             __ballot_sync(kFullMask, act & (up > kEps) & (tp != k1) & (tq != kp1) & (gp < -kEps));
-        const uint32_t later = 0xfffffffeu << q1; // positions after q1
-        uint32_t next;
         if ((smove | pmove) == 0u) {
-            open &= ~(1u << q1); // kernel.cl:232
-            next = open & later;
+            open &= ~((1u << q1) | (1u << q2)); // kernel.cl:232
+            if (PAIR) next &= next - 1u;        // q2 is done as well
         } else { // the predecessor's result counts only when the successor search finds no move
             imp = true;
-            const uint32_t mv = smove ? smove : pmove;
+            int at = 0; // the first lane of the examination that moves
+            if (PAIR && ((smove | pmove) & ROW) == 0u) {
+                at = 16;
+                open &= ~(1u << q1);
+                q1 = q2;
+            }
+            const uint32_t sm = (smove >> at) & ROW;
+            const uint32_t mv = sm ? sm : (pmove >> at) & ROW;
             int f = __ffs(mv) - 1;
             if (mv & (mv - 1u))
-                f = first_listed(mv, lane, d12, __shfl_sync(kFullMask, v, tq),
-                                 nn + (size_t)__shfl_sync(kFullMask, v, k1) * nn_ls, nn_ls);
+                f = first_listed(mv << at, lane, d12, __shfl_sync(kFullMask, v, tq),
+                                 nn + (size_t)__shfl_sync(kFullMask, v, __shfl_sync(kFullMask, k1, at)) * nn_ls,
+                                 nn_ls) & (W - 1);
             // exchange (kernel.cl:235-270): the edges leaving positions i < j make way for
             // (i, j) and (i + 1, j + 1); positions i + 1 .. j are reversed
-            const int pa = smove ? q1 : (q1 > 0 ? q1 - 1 : R - 1), pb = smove ? f : f - 1;
+            const int pa = sm ? q1 : (q1 > 0 ? q1 - 1 : R - 1), pb = sm ? f : f - 1;
             const int i = min(pa, pb), j = max(pa, pb), jn = j + 1 < R ? j + 1 : 0;
             const uint32_t wi = __shfl_sync(kFullMask, word, i), wj = __shfl_sync(kFullMask, word, j);
-            const float d13 = tile[(wi & 0xff) * kRL + (wj & 0xff)];
-            const float d24 = tile[((wi >> 8) & 0xff) * kRL + ((wj >> 8) & 0xff)];
-            const bool in = lane > i && lane <= j;
-            const int src = in ? i + 1 + j - lane : lane;
+            const float d13 = tile[(wi & 0xff) * W + (wj & 0xff)];
+            const float d24 = tile[((wi >> 8) & 0xff) * W + ((wj >> 8) & 0xff)];
+            const bool in = l > i && l <= j;
+            const int src = in ? i + 1 + j - l : l;
             tq = __shfl_sync(kFullMask, tq, src);
             nm = __shfl_sync(kFullMask, nm, src);
-            const float dr = __shfl_sync(kFullMask, dq, in && lane < j ? i + j - lane : lane);
-            dq = lane == j ? d24 : lane == i ? d13 : dr;
-            open = __ballot_sync(kFullMask, (open >> src) & 1u) | (1u << i) | (2u << i) | (1u << j) | (1u << jn);
+            const float dr = __shfl_sync(kFullMask, dq, in && l < j ? i + j - l : l);
+            dq = l == j ? d24 : l == i ? d13 : dr;
+            open = (__ballot_sync(kFullMask, (open >> src) & 1u) & ROW) | (1u << i) | (2u << i) | (1u << j) | (1u << jn);
             neighbours();
-            next = open & later;
+            next = open & (0xfffffffeu << q1);
         }
         if (next == 0u) { // end of the pass
             if (!imp || open == 0u) break;
@@ -233,6 +255,31 @@ __device__ int two_opt_route_best(int lane, int R, const float *tile, uint8_t *t
         if (lane >= a && lane <= jj) tq = tsrc;
     }
     return ACO_OK;
+}
+
+// A route of at most 32 nodes: lane q < R brings route node q's global id (v) and
+// takes back the local node at position q and the edge length there.
+template <int ROWS>
+__device__ __forceinline__ int two_opt_route(int lane, int R, bool first_route, bool best, bool sym, int v,
+                                             const float *dist, int ld, const float2 *nnr, const int *nn, int nn_ls,
+                                             float *tile, uint8_t *tpos, int &tq, float &dq, int pass_limit)
+{
+    const int l = R <= 16 && !best ? lane & 15 : lane;
+    tq = l < R ? l : 0;
+    // edge lengths: position q -> q+1, the last one back to the next depot (node 0 = local 0)
+    const int to = l + 1 < R ? l + 1 : 0;
+    if (R <= 16 && !best) {
+        v = __shfl_sync(kFullMask, v, l);
+        const uint32_t nm = route_tile<ROWS, true>(lane, R, v, dist, ld, nnr, nn, nn_ls, tile);
+        dq = l < R ? tile[l * 16 + to] : 0.f;
+        return sym ? two_opt_route_regs<true, true>(lane, R, first_route, tile, nm, v, nn, nn_ls, tq, dq, pass_limit)
+                   : two_opt_route_regs<false, true>(lane, R, first_route, tile, nm, v, nn, nn_ls, tq, dq, pass_limit);
+    }
+    const uint32_t nm = route_tile<ROWS, false>(lane, R, v, dist, ld, nnr, nn, nn_ls, tile);
+    dq = l < R ? tile[l * kRL + to] : 0.f;
+    if (best) return two_opt_route_best(lane, R, tile, tpos, tq, dq, pass_limit);
+    return sym ? two_opt_route_regs<true, false>(lane, R, first_route, tile, nm, v, nn, nn_ls, tq, dq, pass_limit)
+               : two_opt_route_regs<false, false>(lane, R, first_route, tile, nm, v, nn, nn_ls, tq, dq, pass_limit);
 }
 
 } // namespace
