@@ -427,7 +427,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
                       (p.route_ls > 0 || (p.route_ls == 0 && (total_ants > 4 * sm_count || routes >= 60)));
         route_cap_ = use_routes_ ? (int)cap : 0;
     }
-    const size_t o_rdesc = take((size_t)route_cap_ * sizeof(int2)), o_rctr = take(16);
+    const size_t o_rdesc = take((size_t)route_cap_ * sizeof(int2)), o_rctr = take(32);
     const size_t o_lslist = take((size_t)total_ants * 4), o_lsctr = take(16); // flagged ants for the per-ant 2-opt
     const size_t o_rrem = take((size_t)total_ants * 4);
 
@@ -798,6 +798,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         c.ls_list = ls_list_d_;
         c.ls_list_ctr = ls_list_ctr_d_;
         c.route_cap = route_cap_;
+        c.route_short = ih.finite || p.ls_best ? kRegRoute : 0;
         c.seeds = ih.seeds_d; c.solutions = ih.sol_d; c.lens = ih.lens_d; c.status = status_d;
         c.wait_limit = wait_d;
         LocalSearchArgs &l = largs[b];
@@ -1076,7 +1077,7 @@ int Colony::construct(bool in_iteration)
     // the route list is rewound by the 2-opt kernel that consumes it; a second
     // construct without one in between starts it afresh
     if (use_routes_ && lsw == 0 && routes_pending_) {
-        CK(cudaMemsetAsync(route_ctr_d_, 0, 16, st));
+        CK(cudaMemsetAsync(route_ctr_d_, 0, 32, st));
         CK(cudaMemsetAsync(ls_list_ctr_d_, 0, 16, st));
     }
     routes_pending_ = use_routes_ && lsw == 0;

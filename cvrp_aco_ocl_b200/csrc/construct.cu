@@ -643,47 +643,66 @@ __device__ __forceinline__ void draw_warp(uint32_t xs, float *ring, const int *f
 // The route list entries of one finished ant (warp-wide): route r is the
 // positions [depot r, depot r+1) of its tour, listed as {ant, first position |
 // nodes << 16} for the route-level 2-opt, which improves routes of at most
-// kListedRoute nodes (its local node ids are bytes).  An ant with a longer
-// route, or whose routes do not fit the list, lists none and is flagged
-// (ls_needed 2) for the per-ant kernel, which improves all of its routes.
+// kListedRoute nodes (its local node ids are bytes): short routes from the front
+// of the list, the others from its back.  Both ends are reserved by one atomic, so
+// the ants that fit are those before the first that does not, which notes the
+// counts it found.  An ant with a longer route, or whose routes do not fit the
+// list, lists none and is flagged (ls_needed 2) for the per-ant kernel, which
+// improves all of its routes.
 constexpr int kListedRoute = 255;
 
 __device__ __forceinline__ void emit_routes(const ConstructArgs &a, const uint16_t *tbuf, int size, int g, int lane)
 {
-    const unsigned FULL = 0xffffffffu;
-    int nr = 0, prev = 0;
+    const unsigned FULL = 0xffffffffu, lt = (1u << lane) - 1u;
+    // the routes that end (at a depot) among the 32 positions from `base`: their mask,
+    // and on a lane that ends one its nodes and, in prev, its first position
+    int carry = 0;
+    auto ends = [&](int base, int &prev, int &R) {
+        const int p = base + lane;
+        const unsigned m = __ballot_sync(FULL, p >= 1 && p < size && tbuf[p < size ? p : 0] == 0);
+        prev = m & lt ? base + 31 - __clz(m & lt) : carry;
+        R = (m >> lane) & 1u ? p - prev : 0;
+        if (m) carry = base + 31 - __clz(m);
+        return m;
+    };
+    int nr = 0, nl = 0, prev, R;
     bool toolong = false;
     for (int base = 0; base < size; base += 32) { // count
-        const int p = base + lane;
-        unsigned m = __ballot_sync(FULL, p >= 1 && p < size && tbuf[p < size ? p : 0] == 0);
-        while (m) {
-            const int q = base + __ffs(m) - 1;
-            m &= m - 1;
-            nr++;
-            toolong = toolong || q - prev > kListedRoute;
-            prev = q;
+        nr += __popc(ends(base, prev, R));
+        nl += __popc(__ballot_sync(FULL, R > a.route_short));
+        toolong = toolong || R > kListedRoute;
+    }
+    unsigned s0 = 0, l0 = 0;
+    bool fits = !__any_sync(FULL, toolong);
+    if (fits) {
+        if (lane == 0) {
+            unsigned long long *ctr = reinterpret_cast<unsigned long long *>(a.route_ctr);
+            unsigned long long old = *const_cast<volatile unsigned long long *>(ctr);
+            if ((old >> 32) + (old & 0xffffffffu) <= (unsigned)a.route_cap)
+                old = atomicAdd(ctr, (unsigned)(nr - nl) | (unsigned long long)nl << 32);
+            s0 = (unsigned)old;
+            l0 = (unsigned)(old >> 32);
+        }
+        s0 = __shfl_sync(FULL, s0, 0);
+        l0 = __shfl_sync(FULL, l0, 0);
+        const bool full = s0 + l0 > (unsigned)a.route_cap;
+        fits = !full && s0 + l0 + nr <= (unsigned)a.route_cap;
+        if (!full && !fits && lane == 0) { // the first ant that does not fit
+            a.route_ctr[2] = (int)s0;
+            a.route_ctr[3] = (int)l0;
         }
     }
-    int rbase = 0;
-    if (lane == 0 && !toolong) rbase = atomicAdd(a.route_ctr, nr);
-    rbase = __shfl_sync(FULL, rbase, 0);
-    const bool fits = !toolong && rbase + nr <= a.route_cap;
     if (fits) { // write
-        int k = 0;
-        prev = 0;
+        int at_s = (int)s0, at_l = a.route_cap - 1 - (int)l0;
+        carry = 0;
         for (int base = 0; base < size; base += 32) {
-            const int p = base + lane;
-            unsigned m = __ballot_sync(FULL, p >= 1 && p < size && tbuf[p < size ? p : 0] == 0);
-            while (m) {
-                const int q = base + __ffs(m) - 1;
-                m &= m - 1;
-                if (lane == (k & 31)) a.route_desc[rbase + k] = make_int2(g, prev | ((q - prev) << 16));
-                k++;
-                prev = q;
-            }
+            const unsigned m = ends(base, prev, R), ml = __ballot_sync(FULL, R > a.route_short), ms = m & ~ml;
+            if (R > 0)
+                a.route_desc[(ml >> lane) & 1u ? at_l - __popc(ml & lt) : at_s + __popc(ms & lt)] =
+                    make_int2(g, prev | (R << 16));
+            at_s += __popc(ms);
+            at_l -= __popc(ml);
         }
-    } else if (!toolong) { // entries of this reservation below the capacity are read: mark them empty
-        for (int k = lane; k < nr && rbase + k < a.route_cap; k += 32) a.route_desc[rbase + k] = make_int2(-1, 0);
     }
     if (lane == 0) {
         a.route_rem[g] = fits ? nr : 0;

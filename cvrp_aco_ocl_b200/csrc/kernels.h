@@ -27,6 +27,8 @@ namespace aco {
 
 constexpr int kOrderNodes = 1024; // largest instance whose depot row is kept sorted
 
+constexpr int kRegRoute = 32; // largest route (nodes, depot included) of the 2-opt's register path
+
 struct ConstructArgs {
     int n, ld, n_ants, T, nloc, log2_nloc, kmax;
     int capacity;
@@ -60,14 +62,19 @@ struct ConstructArgs {
     int sym;               // symmetric distances (swap stage)
     uint8_t *ls_needed;    // total ants of the colony
     // route list for the route-level 2-opt (null: not used): every route of at
-    // most 255 nodes as {global ant, first position | nodes << 16}; route_ctr[0]
-    // counts the entries (capacity route_cap), route_rem[g] the entries of ant g.
+    // most 255 nodes as {global ant, first position | nodes << 16}, those of at
+    // most route_short nodes from the front, the others (list-scanning or two
+    // positions a lane: an order of magnitude slower each, taken first) from the
+    // back.  route_ctr (8 ints): entries reserved at the front and at the back
+    // (together more than route_cap: the list was full), the two counts at which
+    // it filled up, then the 2-opt kernel's claims from the back and the front and
+    // its CTAs that are done.  route_rem[g]: the entries of ant g.
     // ls_needed[g]: 2 = none of its routes listed (a longer route, or the list
     // was full) -- the per-ant kernel does those; 1 (fused construct only) = the
     // ant's routes of more than 32 nodes are left to the per-ant kernel.
     int2 *route_desc;
     int *route_ctr, *route_rem;
-    int route_cap;
+    int route_cap, route_short;
     // the ants whose ls_needed is set, listed for the per-ant 2-opt kernel
     // (route-list mode): ls_list_ctr[0] entries, capacity = the colony's ants
     int *ls_list, *ls_list_ctr;

@@ -19,9 +19,10 @@
 // them from a shared counter, longest first; route_opt_kernel: a persistent
 // grid over the construct's list of every ant's routes (see below).  A route of
 // at most 32 nodes (depot included) runs entirely in one warp's registers
-// (two_opt.cuh); longer ones, and all routes of an instance whose distances are
-// not all finite, take the list-scanning paths over shared-memory arrays and the
-// L2-resident distance matrix.
+// (two_opt.cuh), one of at most 64 in registers but for its distances; longer
+// ones, and all routes of an instance whose distances are not all finite, take
+// the list-scanning paths over shared-memory arrays and the L2-resident
+// distance matrix.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -459,6 +460,9 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
                 dt[rb + lane] = dq;
             }
             __syncwarp();
+        } else if (R > kRL && R <= kRW && !a.generic) {
+            st = two_opt_route_wide(lane, R, r == 0, a.sym, tour + rb, dt + rb, a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls,
+                                    a.pass_limit);
         } else {
             for (int p = rb + lane; p <= re; p += 32) dt[p] = __ldg(a.dist + (size_t)tour[p] * a.ld + tour[p + 1]);
             __syncwarp();
@@ -523,10 +527,12 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
 // most 255 nodes) is one entry of the list the construct kernel wrote, and the
 // warps of a persistent grid take entries from a counter, so the routes of
 // one ant spread over all SMs instead of queueing in one CTA.  A route needs
-// no state of its ant beyond its own nodes.  Routes of at most 32 nodes run in
+// no state of its ant beyond its own nodes.  Routes of at most 64 nodes run in
 // registers (two_opt.cuh), longer ones through two_opt_route_local, whose
 // membership test is a per-warp node -> local index map in shared memory, set for
-// the route and cleared after it.  The warp that improves an ant's last listed route sums the ant's
+// the route and cleared after it.  Routes of more than 32 nodes are taken first,
+// in a loop of their own (in one loop with the others their registers cost the
+// batch 2-8%).  The warp that improves an ant's last listed route sums the ant's
 // tour length (kernel.cl:534-538) from the distances of its final tour edges,
 // which equal the 2-opt's edge lengths for a symmetric matrix (the only case
 // this kernel is used for); ants flagged for the per-ant kernel get their
@@ -534,7 +540,8 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
 // ---------------------------------------------------------------------------
 constexpr int kRouteRows = 8; // tile rows loaded per round
 
-// Routes of 33..255 nodes in the route-level kernel: kernel.cl:126-277 with
+// Routes of 65..255 nodes (and those of instances with distances that are not
+// finite) in the route-level kernel: kernel.cl:126-277 with
 // the route's state in the warp's shared memory (the area of the register
 // path's distance tile) and local node ids: nodes[k] is the global node of
 // local id k (0: the depot), tk[p] the local id at route position p, pk[k] the
@@ -731,6 +738,84 @@ __host__ __device__ inline size_t route_warp_bytes(int n_max)
     return kRL * kRL * 4 + kRL + al16((size_t)n_max);
 }
 
+// A listed route that the register path does not take: of more than 32 nodes, or
+// of an instance with distances that are not finite.
+__device__ __forceinline__ void long_route(const LocalSearchArgs &a, int *gt, int rb, int R, unsigned char *wbase,
+                                           uint8_t *loc, int lane)
+{
+    int st;
+    if (R > kRL && R <= kRW && !a.generic) {
+        uint16_t *nodes = reinterpret_cast<uint16_t *>(wbase);
+        for (int k = lane; k < R; k += 32) nodes[k] = (uint16_t)gt[rb + k];
+        __syncwarp();
+        st = two_opt_route_wide(lane, R, rb == 0, true, nodes, reinterpret_cast<float *>(wbase + 2 * kRW),
+                                a.dist, a.ld, a.nnr, a.nn_list, a.nn_ls, a.pass_limit);
+        for (int k = lane; k < R; k += 32) __stcs(gt + rb + k, (int)nodes[k]);
+        __syncwarp();
+    } else { // the list-scanning path
+        uint16_t *nodes = reinterpret_cast<uint16_t *>(wbase);
+        uint8_t *tk = wbase + 512, *pk = tk + 256, *dlb = pk + 256;
+        float *dq = reinterpret_cast<float *>(wbase + 1280);
+        for (int k = lane; k < R; k += 32) {
+            const int node = gt[rb + k];
+            nodes[k] = (uint16_t)node;
+            tk[k] = (uint8_t)k;
+            pk[k] = (uint8_t)k;
+            dlb[k] = (uint8_t)(k == 0 && rb != 0 ? 1 : 0); // the depot's bit: clear entering route 0 only
+            if (k >= 1) loc[node] = (uint8_t)k;
+        }
+        __syncwarp();
+        for (int k = lane; k < R; k += 32) dq[k] = __ldg(a.dist + (size_t)nodes[k] * a.ld + nodes[k + 1 < R ? k + 1 : 0]);
+        __syncwarp();
+        st = two_opt_route_local(lane, R, a.dist, a.ld, a.nn_list, a.nn_ls, loc, nodes, tk, pk, dlb, dq,
+                                 a.pass_limit);
+        for (int k = lane; k < R; k += 32) __stcs(gt + rb + k, (int)nodes[tk[k]]);
+        for (int k = 1 + lane; k < R; k += 32) loc[nodes[k]] = 0;
+        __syncwarp();
+    }
+    if (st != ACO_OK && lane == 0) set_status(a.status, st);
+}
+
+// One route of ant g is final; after its last one its tour length is summed.
+__device__ __forceinline__ void route_done(const LocalSearchArgs &a, int g, int ant, int *rem, const uint8_t *flagged,
+                                           int lane)
+{
+    __threadfence();
+    int last = 0;
+    if (lane == 0) last = atomicSub(rem + g, 1) == 1;
+    last = __shfl_sync(FULL, last, 0);
+    if (!last || flagged[g]) return;
+    __threadfence();
+    const int *gt = a.solutions + (size_t)ant * a.T;
+    const int size = __ldcg(gt + a.T - 1);
+    float len = 0.f;
+    // four chunks of 32 edges: their tour and distance loads in flight before the sums
+    for (int base = 0; base < size - 1; base += 128) {
+        int u[4], w[4];
+        float e[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int p = base + 32 * c + lane;
+            u[c] = p < size - 1 ? __ldcg(gt + p) : 0;
+            w[c] = p < size - 1 ? __ldcg(gt + p + 1) : 0;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) e[c] = __ldg(a.dist + (size_t)u[c] * a.ld + w[c]);
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int m = size - 1 - (base + 32 * c);
+#pragma unroll
+            for (int k = 0; k < 32; k++) {
+                const float x = __shfl_sync(FULL, e[c], k);
+                if (k < m) len = __fadd_rn(len, x);
+            }
+        }
+    }
+    if (lane == 0) a.lens[ant] = len;
+}
+
+// ctr: as ConstructArgs.route_ctr.  The warps first take the long routes, each of
+// which is as slow as a few dozen short ones, then the short ones.
 __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs *args, const int *ant_inst,
                                                            const int *ant_base, const int2 *desc, int *ctr, int cap,
                                                            int *rem, const uint8_t *flagged, int n_max)
@@ -740,43 +825,31 @@ __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs
     unsigned char *wbase = smem + (size_t)warp * route_warp_bytes(n_max);
     float *tile = reinterpret_cast<float *>(wbase);
     uint8_t *tpos = wbase + kRL * kRL * 4;
-    uint8_t *loc = tpos + kRL; // node -> local index (0: not in the route; longer routes only)
-    for (int i = lane; i < n_max; i += 32) loc[i] = 0;
-    __syncwarp();
-    const int total = min(ctr[0], cap);
-    for (;;) {
+    const bool full = (unsigned)ctr[0] + (unsigned)ctr[1] > (unsigned)cap;
+    const int n_short = full ? ctr[2] : ctr[0], n_long = full ? ctr[3] : ctr[1];
+    auto claim = [&](int *at) {
         int idx = 0;
-        if (lane == 0) idx = atomicAdd(&ctr[1], 1);
-        idx = __shfl_sync(FULL, idx, 0);
-        if (idx >= total) break;
+        if (lane == 0) idx = atomicAdd(at, 1);
+        return __shfl_sync(FULL, idx, 0);
+    };
+    if (n_long > 0) {
+        uint8_t *loc = tpos + kRL; // node -> local index (0: not in the route)
+        for (int i = lane; i < n_max; i += 32) loc[i] = 0;
+        __syncwarp();
+        for (int idx; (idx = claim(ctr + 4)) < n_long;) {
+            const int2 d = desc[cap - 1 - idx];
+            const int b = __ldg(ant_inst + d.x), ant = d.x - __ldg(ant_base + b);
+            const LocalSearchArgs &a = args[b];
+            long_route(a, a.solutions + (size_t)ant * a.T, d.y & 0xFFFF, d.y >> 16, wbase, loc, lane);
+            route_done(a, d.x, ant, rem, flagged, lane);
+        }
+    }
+    for (int idx; (idx = claim(ctr + 5)) < n_short;) {
         const int2 d = desc[idx];
-        if (d.x < 0) continue; // an empty entry
         const int g = d.x, rb = d.y & 0xFFFF, R = d.y >> 16;
         const int b = __ldg(ant_inst + g), ant = g - __ldg(ant_base + b);
         const LocalSearchArgs a = args[b];
         int *gt = a.solutions + (size_t)ant * a.T;
-        if (R > kRL || (a.generic && !a.best)) { // the route-local generic path in the warp's tile area
-            uint16_t *nodes = reinterpret_cast<uint16_t *>(wbase);
-            uint8_t *tk = wbase + 512, *pk = tk + 256, *dlb = pk + 256;
-            float *dq = reinterpret_cast<float *>(wbase + 1280);
-            for (int k = lane; k < R; k += 32) {
-                const int node = gt[rb + k];
-                nodes[k] = (uint16_t)node;
-                tk[k] = (uint8_t)k;
-                pk[k] = (uint8_t)k;
-                dlb[k] = (uint8_t)(k == 0 && rb != 0 ? 1 : 0); // the depot's bit: clear entering route 0 only
-                if (k >= 1) loc[node] = (uint8_t)k;
-            }
-            __syncwarp();
-            for (int k = lane; k < R; k += 32) dq[k] = __ldg(a.dist + (size_t)nodes[k] * a.ld + nodes[k + 1 < R ? k + 1 : 0]);
-            __syncwarp();
-            const int st = two_opt_route_local(lane, R, a.dist, a.ld, a.nn_list, a.nn_ls, loc, nodes, tk, pk, dlb, dq,
-                                               a.pass_limit);
-            if (st != ACO_OK && lane == 0) set_status(a.status, st);
-            for (int k = lane; k < R; k += 32) __stcs(gt + rb + k, (int)nodes[tk[k]]);
-            for (int k = 1 + lane; k < R; k += 32) loc[nodes[k]] = 0;
-            __syncwarp();
-        } else {
         const int v = lane < R ? gt[rb + lane] : 0;
         int tq;
         float dq;
@@ -786,49 +859,14 @@ __global__ void __launch_bounds__(512, 2) route_opt_kernel(const LocalSearchArgs
         const int node = __shfl_sync(FULL, v, tq);
         if (lane < R) __stcs(gt + rb + lane, node); // evict first: not read again before the statistics
         __syncwarp();
-        }
-        __threadfence();
-        int last = 0;
-        if (lane == 0) last = atomicSub(rem + g, 1) == 1;
-        last = __shfl_sync(FULL, last, 0);
-        if (last && !flagged[g]) { // every route of the ant is final: its length
-            __threadfence();
-            const int size = __ldcg(gt + a.T - 1);
-            float len = 0.f;
-            // four chunks of 32 edges: their tour and distance loads in flight before the sums
-            for (int base = 0; base < size - 1; base += 128) {
-                int u[4], w[4];
-                float e[4];
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int p = base + 32 * c + lane;
-                    u[c] = p < size - 1 ? __ldcg(gt + p) : 0;
-                    w[c] = p < size - 1 ? __ldcg(gt + p + 1) : 0;
-                }
-#pragma unroll
-                for (int c = 0; c < 4; c++) e[c] = __ldg(a.dist + (size_t)u[c] * a.ld + w[c]);
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int m = size - 1 - (base + 32 * c);
-#pragma unroll
-                    for (int k = 0; k < 32; k++) {
-                        const float x = __shfl_sync(FULL, e[c], k);
-                        if (k < m) len = __fadd_rn(len, x);
-                    }
-                }
-            }
-            if (lane == 0) a.lens[ant] = len;
-        }
+        route_done(a, g, ant, rem, flagged, lane);
     }
     // the last CTA to finish rewinds the list for the next iteration
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(&ctr[2], 1) == (int)gridDim.x - 1) {
-            ctr[0] = 0;
-            ctr[1] = 0;
-            ctr[2] = 0;
-        }
+        if (atomicAdd(&ctr[6], 1) == (int)gridDim.x - 1)
+            for (int i = 0; i < 8; i++) ctr[i] = 0;
     }
 }
 

@@ -24,7 +24,7 @@
 // 10 a row to build the tile (60 with the list filtering); routes of at most 16
 // nodes take two examinations and two rows at a time.  The issue slots bound it.
 // 512 instances, 2.9 M routes of 14 nodes: 9.81 ms with the lists in shared memory,
-// 6.58 by position, 5.89 with the pairs; 201 ants with full lists: 74 -> 27 us.
+// 6.58 by position, 5.78 with the pairs; 201 ants with full lists: 74 -> 27 us.
 #pragma once
 
 #include <cstdint>
@@ -34,7 +34,7 @@
 namespace aco {
 namespace {
 
-constexpr int kRL = 32; // largest route (nodes, depot included) of the register path
+constexpr int kRL = kRegRoute; // largest route (nodes, depot included) of the register path
 
 constexpr unsigned kFullMask = 0xffffffffu;
 
@@ -89,7 +89,7 @@ __device__ __forceinline__ uint32_t route_tile(int lane, int R, int v, const flo
 
 // The lane of `mv` (improving partners) the scan reaches first: the smallest
 // distance, equal ones in list order.  gnode: the lane's global node.
-__device__ __noinline__ int first_listed(uint32_t mv, int lane, float d12, int gnode, const int *list, int nn_ls)
+__device__ __forceinline__ int first_listed(uint32_t mv, int lane, float d12, int gnode, const int *list, int nn_ls)
 {
     const uint32_t b = __float_as_uint(__fadd_rn(d12, 0.f)); // -0 as +0
     const uint32_t ord = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
@@ -255,6 +255,209 @@ __device__ int two_opt_route_best(int lane, int R, const float *tile, uint8_t *t
         if (lane >= a && lane <= jj) tq = tsrc;
     }
     return ACO_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Routes of 33 to 64 nodes: as two_opt_route_regs with two positions a lane
+// (p and p + 32).  Their tile would not fit the warp's share of shared memory,
+// so the three distances of a partner come from the matrix, loaded together: one
+// trip to the cache an examination, where the list-scanning path waits for its
+// list entry, its distance and its neighbour's distance in turn.  1001 nodes, 256
+// ants, 2% of the routes of 33-48 nodes: 2-opt 160 -> 113 us with these taken first.
+// nodes: the route's nodes in sequence, on return the improved ones; dist_tour:
+// on return its edge lengths.
+// ---------------------------------------------------------------------------
+constexpr int kRW = 64; // largest route of this path
+
+__device__ __forceinline__ int two_opt_route_wide(int lane, int R, bool first_route, bool sym, uint16_t *nodes,
+                                               float *dist_tour, const float *dist, int ld, const float2 *nnr,
+                                               const int *nn, int nn_ls, int pass_limit)
+{
+    auto D = [&](int a, int b) { return __ldg(dist + (size_t)a * ld + b); };
+    // position q of an array held two a lane: q per lane, and q the same in all lanes
+    auto any = [&](auto x0, auto x1, int q) {
+        const auto y0 = __shfl_sync(kFullMask, x0, q & 31), y1 = __shfl_sync(kFullMask, x1, q & 31);
+        return q & 32 ? y1 : y0;
+    };
+    auto one = [&](auto x0, auto x1, int q) { return __shfl_sync(kFullMask, q & 32 ? x1 : x0, q & 31); };
+
+    int id[2], g[2], gs[2], gp[2], pn[2], pp[2]; // local id (entry position), node, its neighbours; their positions
+    float dq[2], dqp[2];
+    uint32_t lo[2] = {0u, 0u}, hi[2] = {0u, 0u}; // the route's customers on the node's list, by local id
+    float2 last[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int p = lane + 32 * u;
+        id[u] = p < R ? p : 0;
+        g[u] = p < R ? (int)nodes[p] : 0;
+        pn[u] = p + 1 < R ? p + 1 : 0;
+        pp[u] = p == 0 ? R - 1 : p - 1;
+        last[u] = make_float2(-__int_as_float(0x7f800000), 0.f);
+        if (p < R && nn_ls > 0) last[u] = __ldg(nnr + g[u]);
+    }
+    const bool has1 = lane + 32 < R; // position lane < R always
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+        for (int k0 = 32 * u; k0 < min(R, 32 * u + 32); k0 += 4) {
+            float d0[4], d1[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const int node1 = __shfl_sync(kFullMask, g[u], (k0 + c) & 31);
+                d0[c] = k0 + c < R ? D(node1, g[0]) : 0.f;
+                d1[c] = k0 + c < R && has1 ? D(node1, g[1]) : 0.f;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float thr = __shfl_sync(kFullMask, last[u].x, (k0 + c) & 31);
+                const uint32_t b0 = __ballot_sync(kFullMask, d0[c] <= thr);
+                const uint32_t b1 = __ballot_sync(kFullMask, has1 && d1[c] <= thr);
+                if (lane == ((k0 + c) & 31)) {
+                    lo[u] = b0 & ~1u & ~(u == 0 ? 1u << lane : 0u);
+                    hi[u] = b1 & ~(u == 1 ? 1u << lane : 0u);
+                }
+            }
+        }
+    // lists that end inside a group of equal distances (see route_tile)
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+        for (uint32_t amb = __ballot_sync(kFullMask, lane + 32 * u < R && last[u].y != 0.f); amb; amb &= amb - 1u) {
+            const int k1 = __ffs(amb) - 1, node1 = __shfl_sync(kFullMask, g[u], k1);
+            const float thr = __shfl_sync(kFullMask, last[u].x, k1);
+            const int *list = nn + (size_t)node1 * nn_ls;
+#pragma unroll
+            for (int w = 0; w < 2; w++) {
+                const bool in = w == 0 ? lane > 0 : has1;
+                for (uint32_t at = __ballot_sync(kFullMask, in && D(node1, g[w]) == thr) & ~(u == w ? 1u << k1 : 0u); at;
+                     at &= at - 1u) {
+                    const int b = __ffs(at) - 1, node = __shfl_sync(kFullMask, g[w], b);
+                    bool hit = false;
+                    for (int h = lane; h < nn_ls; h += 32) hit = hit || __ldg(list + h) == node;
+                    if (!__any_sync(kFullMask, hit) && lane == k1) (w == 0 ? lo[u] : hi[u]) &= ~(1u << b);
+                }
+            }
+        }
+    auto neighbours = [&]() {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            gs[u] = any(g[0], g[1], pn[u]);
+            gp[u] = any(g[0], g[1], pp[u]);
+            dqp[u] = any(dq[0], dq[1], pp[u]);
+        }
+    };
+    dq[0] = dq[1] = 0.f;
+    neighbours();
+    dq[0] = D(g[0], gs[0]);
+    dq[1] = has1 ? D(g[1], gs[1]) : 0.f;
+    neighbours();
+
+    unsigned long long open = (R >= 64 ? ~0ull : (1ull << R) - 1ull) & ~(first_route ? 0ull : 1ull);
+    int passes = 1, q1 = __ffsll((long long)open) - 1, status = ACO_OK;
+    bool imp = false;
+    for (;;) {
+        const int g1 = one(g[0], g[1], q1), gs1 = one(gs[0], gs[1], q1), gp1 = one(gp[0], gp[1], q1);
+        const uint32_t mlo = one(lo[0], lo[1], q1), mhi = one(hi[0], hi[1], q1);
+        const float rs = sym ? one(dq[0], dq[1], q1) : D(g1, gs1), rp = sym ? one(dqp[0], dqp[1], q1) : D(gp1, g1);
+        float d12[2], xs[2], xp[2];
+        bool act[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            act[u] = ((id[u] & 32 ? mhi : mlo) >> (id[u] & 31)) & 1u;
+            d12[u] = act[u] ? D(g1, g[u]) : 0.f;
+            xs[u] = act[u] ? D(gs1, gs[u]) : 0.f;
+            xp[u] = act[u] ? D(gp1, gp[u]) : 0.f;
+        }
+        uint32_t sm[2], pm[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const float us = __fsub_rn(rs, d12[u]), up = __fsub_rn(rp, d12[u]);
+            const float gsu = __fsub_rn(__fsub_rn(xs[u], us), dq[u]), gpu = __fsub_rn(__fsub_rn(xp[u], up), dqp[u]);
+            sm[u] = __ballot_sync(kFullMask, act[u] & (us > kEps) & (gsu < -kEps));
+            pm[u] = __ballot_sync(kFullMask, act[u] & (up > kEps) & (gp[u] != g1) & (g[u] != gp1) & (gpu < -kEps));
+        }
+        if ((sm[0] | sm[1] | pm[0] | pm[1]) == 0u) {
+            open &= ~(1ull << q1);
+        } else {
+            imp = true;
+            const bool succ = (sm[0] | sm[1]) != 0u;
+            const uint32_t m0 = succ ? sm[0] : pm[0], m1 = succ ? sm[1] : pm[1];
+            int f = m0 ? __ffs(m0) - 1 : __ffs(m1) + 31;
+            if (__popc(m0) + __popc(m1) > 1) { // the nearest, equal ones in list order
+                uint32_t ord[2];
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const uint32_t b = __float_as_uint(__fadd_rn(d12[u], 0.f)); // -0 as +0
+                    ord[u] = ((u == 0 ? m0 : m1) >> lane) & 1u ? ((b & 0x80000000u) ? ~b : (b | 0x80000000u)) : 0xffffffffu;
+                }
+                const uint32_t near = __reduce_min_sync(kFullMask, min(ord[0], ord[1]));
+                const uint32_t t0 = __ballot_sync(kFullMask, ((m0 >> lane) & 1u) && ord[0] == near);
+                const uint32_t t1 = __ballot_sync(kFullMask, ((m1 >> lane) & 1u) && ord[1] == near);
+                f = t0 ? __ffs(t0) - 1 : __ffs(t1) + 31;
+                if (__popc(t0) + __popc(t1) > 1) {
+                    const int *list = nn + (size_t)g1 * nn_ls;
+                    for (int h = 0; h < nn_ls; h++) {
+                        const int node = __ldg(list + h);
+                        const uint32_t e0 = __ballot_sync(kFullMask, ((t0 >> lane) & 1u) && g[0] == node);
+                        const uint32_t e1 = __ballot_sync(kFullMask, ((t1 >> lane) & 1u) && g[1] == node);
+                        if (e0 | e1) {
+                            f = e0 ? __ffs(e0) - 1 : __ffs(e1) + 31;
+                            break;
+                        }
+                    }
+                }
+            }
+            const int pa = succ ? q1 : (q1 > 0 ? q1 - 1 : R - 1), pb = succ ? f : f - 1;
+            const int i = min(pa, pb), j = max(pa, pb), jn = j + 1 < R ? j + 1 : 0;
+            const float d13 = D(one(g[0], g[1], i), one(g[0], g[1], j));
+            const float d24 = D(one(gs[0], gs[1], i), one(gs[0], gs[1], j));
+            int nid[2], ng[2];
+            uint32_t nlo[2], nhi[2], nop[2];
+            float nd[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int p = lane + 32 * u;
+                const bool in = p > i && p <= j;
+                const int src = in ? i + 1 + j - p : p, dsrc = in && p < j ? i + j - p : p;
+                nid[u] = any(id[0], id[1], src);
+                ng[u] = any(g[0], g[1], src);
+                nlo[u] = any(lo[0], lo[1], src);
+                nhi[u] = any(hi[0], hi[1], src);
+                nd[u] = any(dq[0], dq[1], dsrc);
+                nd[u] = p == j ? d24 : p == i ? d13 : nd[u];
+                nop[u] = __ballot_sync(kFullMask, (open >> src) & 1ull);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                id[u] = nid[u];
+                g[u] = ng[u];
+                lo[u] = nlo[u];
+                hi[u] = nhi[u];
+                dq[u] = nd[u];
+            }
+            open = nop[0] | (unsigned long long)nop[1] << 32 | 1ull << i | 2ull << i | 1ull << j | 1ull << jn;
+            neighbours();
+        }
+        unsigned long long next = open & (~1ull << q1); // open positions left in this pass
+        if (next == 0ull) {
+            if (!imp) break;
+            if (pass_limit > 0 && passes >= pass_limit) {
+                status = ACO_ERR_LS_LIMIT;
+                break;
+            }
+            passes++;
+            imp = false;
+            if (open == 0ull) break;
+            next = open;
+        }
+        q1 = __ffsll((long long)next) - 1;
+    }
+    nodes[lane] = (uint16_t)g[0];
+    dist_tour[lane] = dq[0];
+    if (has1) {
+        nodes[lane + 32] = (uint16_t)g[1];
+        dist_tour[lane + 32] = dq[1];
+    }
+    __syncwarp();
+    return status;
 }
 
 // A route of at most 32 nodes: lane q < R brings route node q's global id (v) and
