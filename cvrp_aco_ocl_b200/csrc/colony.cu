@@ -420,9 +420,9 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
             sym = sym && ih.sym; // coordinate formulas are symmetric; a given matrix was checked
         }
         // With few ants per SM the per-ant kernel is as fast (the slowest route sets the
-        // time either way) and the list costs the construct a pass: 201 nodes 592 ants 41 us
-        // for 47, 501 nodes 590 ants 84 for 89.  From about 60 routes an ant its warps
-        // queue: 1001 nodes 300 / 590 ants 103 / 147 us, with the list 88 / 138.
+        // time either way) and the list costs the construct a pass: 201 nodes 592 ants 37 us
+        // for 43, 501 nodes 590 ants 77 for 83.  From about 60 routes an ant its warps
+        // queue: 1001 nodes 300 / 590 ants 96 / 135 us, with the list 83 / 128.
         use_routes_ = p.mode == ACO_MODE_THROUGHPUT && (p.ls_flag & 1) && sym && n_max <= 4096 && cap < (1ll << 30) &&
                       (p.route_ls > 0 || (p.route_ls == 0 && (total_ants > 4 * sm_count || routes >= 60)));
         route_cap_ = use_routes_ ? (int)cap : 0;

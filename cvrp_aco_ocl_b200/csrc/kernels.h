@@ -199,7 +199,8 @@ cudaError_t launch_stats(const StatsArgs *d_args, int n_inst, int do_elites, siz
                          const StatsArgs *one = nullptr);
 // Row passes (heuristic matrix, pheromone init, fused update, candidate gather):
 // one warp per row over all instances; d_row_base[b] = first global row of instance b,
-// d_row_inst[g] = the instance of global row g (null: one instance).
+// d_row_inst[g] = the instance of global row g (null: one instance).  sorted: the
+// instances whose depot row is put in order as well (throughput mode), 0 for none.
 cudaError_t launch_rows(const UpdateArgs *d_args, const int *d_row_base, const int *d_row_inst, int total_rows,
                         int sorted, int mode, float trail, int sm_count, cudaStream_t st);
 // lens[A] = +inf, num_bsf = 0, iteration = 0 of every instance (init_aco).

@@ -102,11 +102,12 @@ typedef struct aco_params {
     int ls_ants;          /* 0 = autotuned; else ants per 2-opt CTA (1..8), whose routes its warps share */
     int draw_warps;       /* throughput construct: 1 = a helper warp per ant makes the ant's draws ahead of it
                              (at most 8 ants per CTA), -1 = the ant's warp draws, 0 = automatic (helper warps
-                             while there are at most 4 ants per SM); same results either way */
+                             while there are at most 4 ants per SM, unless their buffers cost a candidate table
+                             its place in shared memory); same results either way */
     int route_ls;         /* throughput mode with 2-opt, symmetric distances: 1 = the construct lists every route
                              (of at most 255 nodes) and one persistent kernel improves them all, spread over the SMs;
-                             -1 = one CTA per group of ants; 0 = automatic (the list above 4 ants per SM); same
-                             results either way */
+                             -1 = one CTA per group of ants; 0 = automatic (the list above 4 ants per SM or
+                             from about 60 routes an ant); same results either way */
     int wait_limit;       /* polls of an mbarrier before a device wait gives up with ACO_ERR_TIMEOUT (0 = the
                              default, 2^24 polls, about a second); no reference counterpart (kernel.cl has no
                              bounded waits) */
