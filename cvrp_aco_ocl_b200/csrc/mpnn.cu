@@ -19,20 +19,28 @@
 // another: no operand is staged twice.  The accumulator goes through a shared
 // FP32 tile (row stride 68) that takes the place of the operand tiles once the
 // product is done, which keeps a CTA at 44 KB and three CTAs on an SM.
-// Forward tiles hold whole nodes, so the per-node sums need no atomics.
-// Backward sums into dP are 16-byte vector reductions; weight gradients
-// accumulate in tensor memory over the tiles of a persistent CTA, bias
-// gradients in registers, and are added to the gradient buffer once per CTA.
-// Layer 0 makes its edge embedding from the edge feature on the fly (it is
-// never stored), and the backward of that layer sums the embedding's gradient
-// from its tiles.  The backward keeps the sign of q as one nibble a lane (16
-// bytes a row) in place of q itself.
+// Edge tiles hold whole nodes, so the per-node sums need no atomics: a node's dB
+// is the sum of its k rows in edge order.  Sums over a node's in-edges (dV, dC)
+// are 16-byte vector reductions; weight gradients accumulate in tensor memory
+// over the tiles of a persistent CTA, bias gradients row by row in registers,
+// and are added to the gradient buffer once per CTA.  Layer 0 makes its edge
+// embedding from the edge feature on the fly (it is never stored).  The backward
+// keeps the sign of q as one nibble a lane (16 bytes a row) in place of q itself.
 //
-// Measured on 32 graphs (9.2 k nodes, 185 k edges, k = 20), launch times under
-// ncu, before (one thread a row, an atomic a channel) and now, us: edge forward
-// 162 -> 55, head 1362 -> 36, edge backward 970 -> 97 (last layer 51), node
-// backward 82 -> 18, node GEMM 30 -> 7, embedding backward 419 -> none of its
-// own; the whole step 5.50 -> 0.545 ms.
+// Order of the sums.  The biases and embeddings enter the network in FP32, and a
+// last-bit change of one moves the BF16 operands of the next step by whole BF16
+// units.  Their gradients are therefore summed in orders that do not depend on
+// timing, but for what has no order of its own: dV and dC, and the last sum of
+// a bias over the CTAs.
+//
+// Measured on 32 graphs (9.2 k nodes, 185 k edges, k = 20), us, with one thread a
+// row and an atomic a channel, and now: edge forward 162 -> 51, head 1362 -> 35,
+// edge backward 970 -> 113 (last layer 66), node backward 82 -> 17, node GEMM
+// 30 -> 6, embedding backward 419 -> 25; the whole step 5.50 -> 0.62 ms.  The sums in
+// order cost 76 us of it: 128-row tiles across nodes take five rounds of the 296
+// CTAs where whole nodes take six, and the embedding's strands are a pass of
+// their own.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -85,12 +93,13 @@ __host__ __device__ inline ParamOffsets param_offsets(int L)
 
 // ---- workspace layout ------------------------------------------------------
 struct Workspace {
-    int *status;
+    int *status; // [0] the call's status, [4] embed_bwd_kernel's counter
     float *loss;
     float *h, *e, *P, *u; // saved activations (e: layers 1..L, e0 is made from the edge feature)
     uint8_t *qm;          // sign of q: bit i of byte 16 r + l is q > 0 at row r, channel 4 l + i
     float *s;             // edge logits
     float *dh, *de, *dP;  // backward
+    float *emb;           // embed_bwd_kernel's partial sums
     size_t bytes;
 };
 
@@ -111,7 +120,7 @@ Workspace carve(void *base, int N, int k, int L)
     const size_t o_P = take(sizeof(float) * L * N * 4 * H), o_q = take(L * E * (H / 4));
     const size_t o_u = take(sizeof(float) * L * N * H), o_s = take(sizeof(float) * E);
     const size_t o_dh = take(sizeof(float) * N * H), o_de = take(sizeof(float) * E * H);
-    const size_t o_dP = take(sizeof(float) * N * 4 * H);
+    const size_t o_dP = take(sizeof(float) * N * 4 * H), o_emb = take(sizeof(float) * 16 * (FN + 3) * H);
     w.bytes = off;
     if (base) {
         char *b = static_cast<char *>(base);
@@ -126,6 +135,7 @@ Workspace carve(void *base, int N, int k, int L)
         w.dh = (float *)(b + o_dh);
         w.de = (float *)(b + o_de);
         w.dP = (float *)(b + o_dP);
+        w.emb = (float *)(b + o_emb);
     }
     return w;
 }
@@ -138,12 +148,35 @@ __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 
+// The components of v whose bit of m is set.
+__device__ __forceinline__ float4 masked4(float4 v, unsigned m)
+{
+    return make_float4(m & 1u ? v.x : 0.f, m & 2u ? v.y : 0.f, m & 4u ? v.z : 0.f, m & 8u ? v.w : 0.f);
+}
+
 __device__ __forceinline__ void acc4(float4 &a, float4 b)
 {
     a.x += b.x;
     a.y += b.y;
     a.z += b.z;
     a.w += b.w;
+}
+
+// Asynchronous copies into shared memory, in groups of a thread's own.
+template <int BYTES>
+__device__ __forceinline__ void async_copy(void *dst, const void *src)
+{
+    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+// All but the thread's last N groups are there.
+template <int N>
+__device__ __forceinline__ void async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // 16-byte vector reduction into global memory.
@@ -266,21 +299,6 @@ __device__ __forceinline__ void acc_to_tile(uint32_t base, int col0, float *ms)
     float *row = ms + (size_t)(lane0 + (threadIdx.x & 31)) * MS + c0;
 #pragma unroll
     for (int i = 0; i < 32; i += 4) st4(row + i, make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
-}
-
-// Per-thread sums of channels 4 hl .. + 3 added up over the CTA's half-warps and
-// into dst[0..63].  buf: 16 x 64 floats.
-__device__ __forceinline__ void add_channel_sums(float4 v, float *buf, float *dst)
-{
-    const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
-    __syncthreads();
-    st4(buf + hw * H + 4 * hl, v);
-    __syncthreads();
-    if (threadIdx.x < H) {
-        float s = 0.f;
-        for (int i = 0; i < TPB / 16; i++) s += buf[i * H + threadIdx.x];
-        atomicAdd(dst + threadIdx.x, s);
-    }
 }
 
 // Rows [0, 64) of the FP32 tile added into a 64 x 64 gradient.
@@ -611,18 +629,16 @@ __global__ void __launch_bounds__(TPB, 3) head_kernel(size_t E, const float *prm
 }
 
 // ---- backward ------------------------------------------------------------------
-// Edge layer backward on tiles of 128 edges.  dh = dL/dh', de = dL/de'
-// (overwritten by dL/de); dP receives du (owned), dV, dB and dC (vector
-// reductions into a zeroed buffer; a half-warp sums the rows of one node
-// before it adds them to dB).  LAST: the last layer, where dh = 0 and so du and
-// dV are zero.  EMBED: layer 0, whose e_in is made from the edge feature and
-// whose dL/de goes straight into the embedding's gradient (gwe, gbe).
+// Edge layer backward on tiles of npt = 128/k nodes.  dh = dL/dh', de = dL/de'
+// (overwritten by dL/de); dP receives du and dB (owned) and dV and dC (vector
+// reductions into a zeroed buffer).  LAST: the last layer, where dh = 0 and so
+// du and dV are zero.  EMBED: layer 0, whose e_in is made from the edge feature.
 template <bool LAST, bool EMBED>
-__global__ void __launch_bounds__(TPB, 2) edge_bwd_kernel(size_t E, int N, int k, const float *A_w, const float *P,
+__global__ void __launch_bounds__(TPB, 2) edge_bwd_kernel(int N, int k, const float *A_w, const float *P,
                                                           const float *u, const uint8_t *qm, const float *e_in,
                                                           const float *w_e, const float *b_e, const float *e_out,
                                                           const int *nbr, const float *dh, float *de, float *dP,
-                                                          float *gA, float *ga, float *gwe, float *gbe, int *status)
+                                                          float *gA, float *ga, int *status)
 {
     extern __shared__ uint8_t sm_raw[];
     __shared__ uint64_t bar;
@@ -635,42 +651,41 @@ __global__ void __launch_bounds__(TPB, 2) edge_bwd_kernel(size_t E, int N, int k
     uint32_t phase = 0;
     stage_tile(Ws, A_w, H, H, H); // A[o][i]
     const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15, c = 4 * hl;
-    float4 we = zero4(), be = zero4(), sum_a = zero4(), sum_we = zero4(), sum_be = zero4();
+    constexpr int kNodeThreads = TPB - H; // the last H threads sum the columns, the others the nodes
+    float4 we = zero4(), be = zero4();
     if (EMBED) {
         we = ldg4(w_e + c);
         be = ldg4(b_e + c);
     }
     const float kf = (float)k;
+    float sum_a = 0.f;
     bool wg_started = false;
-    const size_t tiles = (E + RT - 1) / RT;
-    for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const size_t e0 = t * RT;
-        const int rows = (int)min((size_t)RT, E - e0);
-        int src = (int)((e0 + hw * RPH) / (size_t)k), rem = (int)((e0 + hw * RPH) - (size_t)src * k);
-        float4 dt[RPH], node = zero4();
-        float ef[RPH];
+    const int npt = RT / k, tiles = (N + npt - 1) / npt, q0 = hw * RPH / k, rem0 = hw * RPH - q0 * k;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int n0 = t * npt, nodes = min(npt, N - n0), rows = nodes * k;
+        const size_t e0 = (size_t)n0 * k;
+        int src = n0 + q0, rem = rem0;
+        float4 dt[RPH];
+        int jn[RPH];
+        uint32_t mask = 0u; // the rows' signs of q, a nibble each
 #pragma unroll
         for (int s = 0; s < RPH; s++) {
             const int r = hw * RPH + s;
             float4 dq = zero4(), ei4 = zero4();
             dt[s] = zero4();
-            ef[s] = 0.f;
             if (r < rows) {
                 const size_t ei = e0 + r;
                 int j = __ldg(nbr + ei);
-                if (EMBED) {
-                    ef[s] = __ldg(e_in + ei);
-                    ei4 = embed4(ef[s], we, be);
-                } else {
-                    ei4 = ldg4(e_in + ei * H + c);
-                }
+                if (EMBED) ei4 = embed4(__ldg(e_in + ei), we, be);
+                else ei4 = ldg4(e_in + ei * H + c);
                 const unsigned m = qm[ei * 16 + hl];
+                mask |= m << (4 * s);
                 float4 d = ld4(de + ei * H + c);
                 if ((unsigned)j >= (unsigned)N) {
                     if (hl == 0) set_status(status, ACO_ERR_INVALID);
                     j = 0;
                 }
-                float *dPj = dP + (size_t)j * 4 * H + c;
+                jn[s] = j;
                 if (!LAST) {
                     const float4 eo = ldg4(e_out + ei * H + c), vj = ldg4(P + (size_t)j * 4 * H + H + c);
                     const float4 uu = ldg4(u + (size_t)src * H + c), hh = ldg4(dh + (size_t)src * H + c);
@@ -679,28 +694,22 @@ __global__ void __launch_bounds__(TPB, 2) edge_bwd_kernel(size_t E, int N, int k
                     if (rem == 0) st4(dP + (size_t)src * 4 * H + c, du);
                     const float4 du_e = make_float4(du.x / kf, du.y / kf, du.z / kf, du.w / kf);
                     const float g0 = sigmoidf_(eo.x), g1 = sigmoidf_(eo.y), g2 = sigmoidf_(eo.z), g3 = sigmoidf_(eo.w);
-                    red4(dPj + H, make_float4(du_e.x * g0, du_e.y * g1, du_e.z * g2, du_e.w * g3));
+                    red4(dP + (size_t)j * 4 * H + H + c, make_float4(du_e.x * g0, du_e.y * g1, du_e.z * g2, du_e.w * g3));
                     d.x += du_e.x * vj.x * g0 * (1.f - g0);
                     d.y += du_e.y * vj.y * g1 * (1.f - g1);
                     d.z += du_e.z * vj.z * g2 * (1.f - g2);
                     d.w += du_e.w * vj.w * g3 * (1.f - g3);
                 }
                 dt[s] = d; // the residual part; the product is added below
-                dq = make_float4(m & 1u ? d.x : 0.f, m & 2u ? d.y : 0.f, m & 4u ? d.z : 0.f, m & 8u ? d.w : 0.f);
-                red4(dPj + 3 * H, dq);
-                acc4(node, dq);
-                acc4(sum_a, dq);
-                if (rem == k - 1 || s == RPH - 1 || r == rows - 1) { // this node's rows here are done
-                    red4(dP + (size_t)src * 4 * H + 2 * H + c, node);
-                    node = zero4();
-                }
-                if (++rem == k) {
-                    rem = 0;
-                    src++;
-                }
+                dq = masked4(d, m);
+                if (!LAST) red4(dP + (size_t)j * 4 * H + 3 * H + c, dq);
             }
             put4(DQs, r, hl, dq);
             put4(Es, r, hl, ei4);
+            if (++rem == k) {
+                rem = 0;
+                src++;
+            }
         }
         operands_ready();
         gemm_rows_cols(tm, DQs, Ws, true, H);           // dq A
@@ -713,15 +722,29 @@ __global__ void __launch_bounds__(TPB, 2) edge_bwd_kernel(size_t E, int N, int k
         for (int s = 0; s < RPH; s++) {
             const int r = hw * RPH + s;
             if (r < rows) {
-                float4 d = ld4(ms + (size_t)r * MS + c);
-                d = make_float4(dt[s].x + d.x, dt[s].y + d.y, dt[s].z + d.z, dt[s].w + d.w);
-                if (EMBED) {
-                    acc4(sum_be, d);
-                    acc4(sum_we, make_float4(d.x * ef[s], d.y * ef[s], d.z * ef[s], d.w * ef[s]));
-                } else {
-                    st4(de + (e0 + r) * H + c, d);
-                }
+                float *mr = ms + (size_t)r * MS + c;
+                const float4 d = ld4(mr);
+                st4(de + (e0 + r) * H + c,
+                    make_float4(dt[s].x + d.x, dt[s].y + d.y, dt[s].z + d.z, dt[s].w + d.w));
+                const float4 dq = masked4(dt[s], mask >> (4 * s));
+                if (LAST) red4(dP + (size_t)jn[s] * 4 * H + 3 * H + c, dq); // out of the way of the rows' reads
+                st4(mr, dq); // replaces the product
             }
+        }
+        __syncthreads();
+        if (threadIdx.x < kNodeThreads) {
+            for (int idx = threadIdx.x; idx < nodes * H; idx += kNodeThreads) {
+                const int qn = idx / H, cc = idx - qn * H;
+                float acc = 0.f;
+                for (int j = 0; j < k; j++) acc += ms[(size_t)(qn * k + j) * MS + cc];
+                dP[(size_t)(n0 + qn) * 4 * H + 2 * H + cc] = acc;
+            }
+        } else {
+            const float *col = ms + (threadIdx.x - kNodeThreads);
+            float acc = 0.f;
+#pragma unroll 8
+            for (int r = 0; r < rows; r++) acc += col[(size_t)r * MS];
+            sum_a += acc;
         }
         umma::fence_before();
         __syncthreads();
@@ -733,35 +756,44 @@ __global__ void __launch_bounds__(TPB, 2) edge_bwd_kernel(size_t E, int N, int k
         __syncthreads();
         add_tile_rows(ms, gA);
     }
-    add_channel_sums(sum_a, ms, ga);
-    if (EMBED) {
-        add_channel_sums(sum_we, ms, gwe);
-        add_channel_sums(sum_be, ms, gbe);
-    }
+    if (threadIdx.x >= kNodeThreads) atomicAdd(ga + (threadIdx.x - kNodeThreads), sum_a);
     tmem_teardown(tm, 128);
 }
 
-// dh += dP W (K = 256), dW += dP^T h (two halves of 128 outputs), db += sum dP,
-// on tiles of 64 nodes (twice the CTAs of 128: 9.2 k nodes give 144).  The
+// dh += dP W (K = 256), dW += dP^T h (two halves of 128 outputs) on tiles of 64
+// nodes (twice the CTAs of 128: 9.2 k nodes give 144), db += sum dP.  The
 // accumulator of dP W has 128 rows; its upper 64 come from whatever follows
 // the operand's 64 rows in shared memory and are not read.  LAST: dh = 0 on
-// entry.  EMBED: layer 0, whose dL/dh goes into the node embedding's gradient.
+// entry.  db: the first bias_groups CTAs sum an output a thread over every
+// bias_groups-th 128 nodes in order, beside the others (two CTAs fit an SM).
 struct NodeBwdSmem {
     static constexpr int NT = 64;
     static constexpr size_t A = 0, W = A + 4 * NT * H * 2, HT = W + 4 * H * H * 2, M = HT + NT * H * 2,
                             END = M + (size_t)RT * MS * 4, BYTES = END + 1024;
 };
 
-template <bool LAST, bool EMBED>
-__global__ void __launch_bounds__(TPB) node_bwd_kernel(int N, const float *W, const float *h_in, const float *dP,
-                                                       float *dh, const float *nf, float *gW, float *gb, float *gwn,
-                                                       float *gbn, int *status)
+template <bool LAST>
+__global__ void __launch_bounds__(TPB, 2) node_bwd_kernel(int N, const float *W, const float *h_in, const float *dP,
+                                                       float *dh, float *gW, float *gb, int bias_groups, int *status)
 {
     extern __shared__ uint8_t sm_raw[];
     __shared__ uint64_t bar;
     __shared__ uint32_t slot;
     constexpr int NT = NodeBwdSmem::NT, RH = NT / (TPB / 16);
     constexpr uint32_t kAtom = NT * H * 2; // bytes of 64 channels of the dP tile
+    if ((int)blockIdx.x < bias_groups) {
+        float sum = 0.f;
+        for (int i0 = (int)blockIdx.x * RT; i0 < N; i0 += bias_groups * RT) {
+            const float *col = dP + (size_t)i0 * 4 * H + threadIdx.x;
+            const int rows = min(RT, N - i0);
+            float acc = 0.f;
+#pragma unroll 64
+            for (int i = 0; i < rows; i++) acc += __ldg(col + (size_t)i * 4 * H);
+            sum += acc;
+        }
+        atomicAdd(gb + threadIdx.x, sum);
+        return;
+    }
     uint8_t *sm = tiles_base(sm_raw);
     uint8_t *As = sm + NodeBwdSmem::A, *Ws = sm + NodeBwdSmem::W, *Hs = sm + NodeBwdSmem::HT;
     float *ms = reinterpret_cast<float *>(sm + NodeBwdSmem::M);
@@ -771,19 +803,14 @@ __global__ void __launch_bounds__(TPB) node_bwd_kernel(int N, const float *W, co
     stage_tile(Ws, W, H, 4 * H, 4 * H); // W[o][c], 256 rows
     const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15, c = 4 * hl;
     const int sec = (threadIdx.x >> 4) & 3, rq = threadIdx.x >> 6; // staging: section and row group of the thread
-    float4 sum_b = zero4();
-    float4 sum_n[FN + 1];
-#pragma unroll
-    for (int f = 0; f <= FN; f++) sum_n[f] = zero4();
     bool wg_started = false;
     const int tiles = (N + NT - 1) / NT;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    for (int t = (int)blockIdx.x - bias_groups; t < tiles; t += (int)gridDim.x - bias_groups) {
         const int r0 = t * NT, valid = min(NT, N - r0);
 #pragma unroll 8
         for (int r = rq; r < NT; r += 4) {
             const float4 v = r < valid ? ldg4(dP + (size_t)(r0 + r) * 4 * H + sec * H + c) : zero4();
             put4(As + sec * kAtom, r, hl, v);
-            acc4(sum_b, v);
         }
         stage_tile(Hs, h_in + (size_t)r0 * H, H, NT, valid);
         operands_ready();
@@ -809,17 +836,7 @@ __global__ void __launch_bounds__(TPB) node_bwd_kernel(int N, const float *W, co
                     const float4 o = ld4(row);
                     d = make_float4(o.x + d.x, o.y + d.y, o.z + d.z, o.w + d.w);
                 }
-                if (EMBED) {
-                    const float *f5 = nf + (size_t)(r0 + r) * FN;
-#pragma unroll
-                    for (int f = 0; f < FN; f++) {
-                        const float x = __ldg(f5 + f);
-                        acc4(sum_n[f], make_float4(d.x * x, d.y * x, d.z * x, d.w * x));
-                    }
-                    acc4(sum_n[FN], d);
-                } else {
-                    st4(row, d);
-                }
+                st4(row, d);
             }
         }
         umma::fence_before();
@@ -835,29 +852,120 @@ __global__ void __launch_bounds__(TPB) node_bwd_kernel(int N, const float *W, co
             __syncthreads();
         }
     }
-    // db: the four row groups of a section add up
-    st4(ms + (size_t)rq * 4 * H + sec * H + c, sum_b);
-    __syncthreads();
-    {
-        const int oo = threadIdx.x;
-        atomicAdd(&gb[oo], ((ms[oo] + ms[4 * H + oo]) + ms[8 * H + oo]) + ms[12 * H + oo]);
-    }
-    if (EMBED) {
-        __syncthreads();
+    tmem_teardown(tm, 256);
+}
+
+// Gradients of the input embeddings (K = 5 and 1).  Strand t of 256 sums the nodes
+// and the edges t, t + 256, ... in order; each 32 strands then add up in a
+// butterfly (lanes 16 apart, 8, 4, 2, 1), and the eight results in turn.  A CTA
+// takes all channels of two strands 16 apart, a cluster the even or the odd
+// lanes of a butterfly, and the last CTA to finish adds the 16 clusters' sums
+// (half, a counter in done).  The edge rows come through a ring of asynchronous
+// copies made by half of the CTA's warps, 32 KB of them in flight a CTA: the 16 k
+// chains of sums are too few to hide the reads by themselves.
+constexpr int kStrands = 256, kEmbedSums = (FN + 3) * H, kEmbedCtas = kStrands / 2;
+
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(4 * H)
+    embed_bwd_kernel(int N, int E, const float *nf, const float *ef, const float *dh, const float *de, float *half,
+                     int *done, float *gwn, float *gbn, float *gwe, float *gbe)
+{
+    static_assert(FN + 3 == 8, "a CTA of the cluster adds one of the sums");
+    constexpr int R = 16, D = 5; // rows of a strand a stage, stages of the ring
+    __shared__ __align__(16) float rows[D][2][R][H];
+    __shared__ float feat[D][2][R], part[2][FN + 3][H], pair[FN + 3][H];
+    __shared__ int last;
+    const auto cluster = cooperative_groups::this_cluster();
+    const int c = threadIdx.x % H, s = (threadIdx.x / H) & 1, r = (int)cluster.block_rank(), q = (int)(blockIdx.x >> 3);
+    const int t0 = 32 * (q >> 1) + 2 * r + (q & 1), t = t0 + 16 * s; // its first strand, the thread's
+    auto strand = [](int n, int t) { return n > t ? (n - t + kStrands - 1) / kStrands : 0; };
+    const int n_nodes = strand(N, t), n_edges = strand(E, t), stages = (strand(E, t0) + R - 1) / R;
+    // threads from 2 H on: 16 bytes of row p (and p + 8 of the stage, in both strands)
+    const bool copies = threadIdx.x >= 2 * H;
+    const int p = (threadIdx.x >> 4) & 7, c4 = 4 * (threadIdx.x & 15);
+    auto fetch = [&](int i) { // stage i, if there is one, into its place of the ring
 #pragma unroll
-        for (int f = 0; f <= FN; f++) {
-            // W_n is 64 x FN: channel sums of feature f go FN floats apart
-            __syncthreads();
-            st4(ms + hw * H + c, sum_n[f]);
-            __syncthreads();
-            if (threadIdx.x < H) {
-                float s = 0.f;
-                for (int i = 0; i < TPB / 16; i++) s += ms[i * H + threadIdx.x];
-                atomicAdd(f < FN ? gwn + threadIdx.x * FN + f : gbn + threadIdx.x, s);
-            }
+        for (int j = 0; j < 4; j++) {
+            const int k = p + 8 * (j & 1), ss = j >> 1;
+            const size_t e = ((size_t)i * R + k) * kStrands + t0 + 16 * ss;
+            if (e >= (size_t)E) continue;
+            async_copy<16>(&rows[i % D][ss][k][c4], de + e * H + c4);
+            if (c4 == 0) async_copy<4>(&feat[i % D][ss][k], ef + e);
+        }
+        async_commit();
+    };
+    if (copies)
+        for (int i = 0; i < D - 1; i++) fetch(i);
+    float acc[FN + 3];
+#pragma unroll
+    for (int f = 0; f < FN + 3; f++) acc[f] = 0.f;
+    constexpr int UN = 12; // nodes in flight
+    for (int i0 = 0; i0 < n_nodes && !copies; i0 += UN) {
+        const size_t at = (size_t)i0 * kStrands + t;
+        const float *pd = dh + at * H + c, *pf = nf + at * FN;
+        float d[UN], x[UN][FN];
+#pragma unroll
+        for (int i = 0; i < UN; i++) {
+            const bool in = i0 + i < n_nodes;
+            d[i] = in ? __ldg(pd + i * kStrands * H) : 0.f;
+#pragma unroll
+            for (int f = 0; f < FN; f++) x[i][f] = in ? __ldg(pf + i * kStrands * FN + f) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < UN; i++) {
+            if (i0 + i >= n_nodes) break;
+#pragma unroll
+            for (int f = 0; f < FN; f++) acc[f] += d[i] * x[i][f];
+            acc[FN] += d[i];
         }
     }
-    tmem_teardown(tm, 256);
+    for (int i = 0; i < stages; i++) {
+        if (copies) async_wait<D - 2>();
+        __syncthreads(); // stage i is there, and the place of stage i - 1 is free
+        if (copies) {
+            fetch(i + D - 1);
+            continue;
+        }
+        float d[R], x[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            d[k] = rows[i % D][s][k][c];
+            x[k] = feat[i % D][s][k];
+        }
+#pragma unroll
+        for (int k = 0; k < R; k++)
+            if (i * R + k < n_edges) {
+                acc[FN + 1] += d[k] * x[k];
+                acc[FN + 2] += d[k];
+            }
+    }
+    if (!copies)
+#pragma unroll
+        for (int f = 0; f < FN + 3; f++) part[s][f][c] = acc[f];
+    __syncthreads();
+    for (int i = threadIdx.x; i < kEmbedSums; i += 4 * H) pair[0][i] = part[0][0][i] + part[1][0][i];
+    cluster.sync();
+    if (threadIdx.x < H) { // sum r of the cluster's 16 strands
+        float v[8];
+        for (int i = 0; i < 8; i++) v[i] = *cluster.map_shared_rank(&pair[r][c], i);
+        __stcg(half + (size_t)q * kEmbedSums + r * H + c,
+               ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7])));
+        __threadfence();
+    }
+    cluster.sync(); // the pairs have been read, the sums written
+    if (threadIdx.x == 0) last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < kEmbedSums; i += 4 * H) {
+        const int f = i / H, ch = i % H;
+        float v = 0.f;
+        for (int w = 0; w < 8; w++)
+            v += __ldcg(half + (size_t)(2 * w) * kEmbedSums + i) + __ldcg(half + (size_t)(2 * w + 1) * kEmbedSums + i);
+        if (f < FN) gwn[ch * FN + f] = v;
+        else if (f == FN) gbn[ch] = v;
+        else if (f == FN + 1) gwe[ch] = v;
+        else gbe[ch] = v;
+    }
 }
 
 __global__ void adam_kernel(int n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2,
@@ -949,22 +1057,23 @@ cudaError_t launch_head(size_t E, const float *prm, const ParamOffsets &o, const
 }
 
 template <bool LAST, bool EMBED>
-cudaError_t launch_layer_bwd(int N, int k, const float *prm, const ParamOffsets &o, int l, const float *nf,
-                             const float *ef, const int *nbr, const Workspace &w, float *grad, cudaStream_t st)
+cudaError_t launch_layer_bwd(int N, int k, const float *prm, const ParamOffsets &o, int l, const float *ef,
+                             const int *nbr, const Workspace &w, float *grad, cudaStream_t st)
 {
     const size_t E = (size_t)N * k;
     cudaError_t e = cudaMemsetAsync(w.dP, 0, sizeof(float) * N * 4 * H, st);
     if (e == cudaSuccess) e = set_smem(edge_bwd_kernel<LAST, EMBED>, TileSmem::BYTES);
-    if (e == cudaSuccess) e = set_smem(node_bwd_kernel<LAST, EMBED>, NodeBwdSmem::BYTES);
+    if (e == cudaSuccess) e = set_smem(node_bwd_kernel<LAST>, NodeBwdSmem::BYTES);
     if (e != cudaSuccess) return e;
-    edge_bwd_kernel<LAST, EMBED><<<grid_of((E + RT - 1) / RT, 2), TPB, TileSmem::BYTES, st>>>(
-        E, N, k, prm + o.A[l], w.P + (size_t)l * N * 4 * H, w.u + (size_t)l * N * H, w.qm + (size_t)l * E * 16,
+    const int npt = RT / k;
+    edge_bwd_kernel<LAST, EMBED><<<grid_of((N + npt - 1) / npt, 2), TPB, TileSmem::BYTES, st>>>(
+        N, k, prm + o.A[l], w.P + (size_t)l * N * 4 * H, w.u + (size_t)l * N * H, w.qm + (size_t)l * E * 16,
         EMBED ? ef : w.e + (size_t)(l - 1) * E * H, prm + o.W_e, prm + o.b_e, w.e + (size_t)l * E * H, nbr, w.dh, w.de,
-        w.dP, grad + o.A[l], grad + o.a[l], grad + o.W_e, grad + o.b_e, w.status);
-    constexpr int NT = NodeBwdSmem::NT;
-    node_bwd_kernel<LAST, EMBED><<<grid_of((N + NT - 1) / NT, 1), TPB, NodeBwdSmem::BYTES, st>>>(
-        N, prm + o.W[l], w.h + (size_t)l * N * H, w.dP, w.dh, nf, grad + o.W[l], grad + o.b[l], grad + o.W_n,
-        grad + o.b_n, w.status);
+        w.dP, grad + o.A[l], grad + o.a[l], w.status);
+    const unsigned bias_groups = grid_of((N + RT - 1) / RT, 2);
+    node_bwd_kernel<LAST><<<bias_groups + grid_of((N + NodeBwdSmem::NT - 1) / NodeBwdSmem::NT, 1), TPB,
+                            NodeBwdSmem::BYTES, st>>>(N, prm + o.W[l], w.h + (size_t)l * N * H, w.dP, w.dh,
+                                                      grad + o.W[l], grad + o.b[l], (int)bias_groups, w.status);
     return cudaGetLastError();
 }
 
@@ -1031,12 +1140,14 @@ int aco_mpnn_grad(int n_nodes, int k, int layers, const float *params, const flo
     for (int l = L - 1; l >= 0; l--) {
         const bool last = l == L - 1, embed = l == 0;
         const cudaError_t e =
-            last ? (embed ? launch_layer_bwd<true, true>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st)
-                          : launch_layer_bwd<true, false>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st))
-                 : (embed ? launch_layer_bwd<false, true>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st)
-                          : launch_layer_bwd<false, false>(N, k, params, o, l, node_feat, edge_feat, nbr, w, grad, st));
+            last ? (embed ? launch_layer_bwd<true, true>(N, k, params, o, l, edge_feat, nbr, w, grad, st)
+                          : launch_layer_bwd<true, false>(N, k, params, o, l, edge_feat, nbr, w, grad, st))
+                 : (embed ? launch_layer_bwd<false, true>(N, k, params, o, l, edge_feat, nbr, w, grad, st)
+                          : launch_layer_bwd<false, false>(N, k, params, o, l, edge_feat, nbr, w, grad, st));
         if (e != cudaSuccess) return ACO_ERR_CUDA;
     }
+    embed_bwd_kernel<<<kEmbedCtas, 4 * H, 0, st>>>(
+        N, (int)E, node_feat, edge_feat, w.dh, w.de, w.emb, w.status + 4, grad + o.W_n, grad + o.b_n, grad + o.W_e, grad + o.b_e);
     return cudaGetLastError() == cudaSuccess ? ACO_OK : ACO_ERR_CUDA;
 }
 
