@@ -531,6 +531,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         const int per_block = std::max(ih.n <= 128 ? 4 : 1, std::min(8, per_sm));
         cp_apc = p.ants_per_block > 0 ? p.ants_per_block : std::max(1, std::min(per_block, 16 / wpa));
         if (cp_apc * cp_wpa > 16) return ACO_ERR_INVALID; // 512 threads per CTA at most
+        if (ih.n > kParityNodes * 32 * cp_wpa) return ACO_ERR_INVALID; // whoever chose the shape
         cp_stage = construct_parity_smem(ih.n, ih.nloc, ih.kmax, wpa, cp_apc, true, fin_any) <= kSmemBudget;
     } else {
         // Ants per work item (one warp per ant, at most 16 warps: the kernel's launch bound

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(512) construct_parity_kernel(ConstructArgs a)
     int *seeds = a.seeds + (size_t)ant * nloc;
     for (int l = t; l < nlanes; l += TPA) st[l] = pm_norm(seeds[l]);
 
-    const int J = (n + TPA - 1) / TPA; // nodes per thread (<= 32: visited bits fit one register)
+    const int J = (n + TPA - 1) / TPA; // nodes per thread (<= kParityNodes: visited bits fit one register)
     uint32_t vis = (t == 0) ? 1u : 0u; // node 0 (the depot) starts visited (kernel.cl:431)
     int cur = 0, step = 0, vcnt = 1, load = 0, err = 0;
     float rdist = 0.f, tdist = 0.f, pend = 0.f;

@@ -27,6 +27,8 @@ namespace aco {
 
 constexpr int kOrderNodes = 1024; // largest instance whose depot row is kept sorted
 
+constexpr int kParityNodes = 32; // nodes of a parity construct thread: their visited bits are one word
+
 constexpr int kRegRoute = 32; // largest route (nodes, depot included) of the 2-opt's register path
 
 struct ConstructArgs {

@@ -915,7 +915,7 @@ int autotune(const InstanceSpec *specs, int count, const aco_params &p0, int ite
     } else {
         for (int wpa : {1, 2, 4, 8})
             for (int apc : {1, 2, 4, 8})
-                if (wpa * apc <= 16 && 32 * wpa <= p0.nloc) cands.push_back({apc, wpa, 0, 0});
+                if (wpa * apc <= 16 && 32 * wpa <= p0.nloc && specs[0].n <= kParityNodes * 32 * wpa) cands.push_back({apc, wpa, 0, 0});
     }
     for (const auto &cd : cands) {
         aco_params q = p0;

@@ -87,7 +87,10 @@ typedef struct aco_params {
     int device;           /* CUDA device ordinal (default 0) */
     int use_graph;        /* 1 = replay one CUDA graph per iteration (default 1) */
     int ants_per_block;   /* 0 = autotuned; else ants per CTA of the construct kernel */
-    int warps_per_ant;    /* 0 = autotuned; else warps per ant of the parity construct kernel (1,2,4,8) */
+    int warps_per_ant;    /* 0 = autotuned; else warps per ant of the parity construct kernel (1,2,4,8; at most
+                             nloc / 32).  A warp takes at most 1024 nodes and a CTA 16 warps: a shape that does
+                             not hold the instance, an ants_per_block that leaves too few warps, and parity
+                             instances of more than 8192 nodes are ACO_ERR_INVALID */
     int ls_warps;         /* 0 = autotuned; else warps per 2-opt CTA (1..32, one route per warp at a time) */
     int stage_matrix;     /* throughput construct: 0 = stage the whole total_info matrix in shared memory when
                              it fits (used by the no-candidate fallback); -1 = never, rows are read through L2 */
