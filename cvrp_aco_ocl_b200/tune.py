@@ -28,6 +28,7 @@ from ._lib import AcoInstance, AcoParams, check, lib
 
 SHAPE_FIELDS = ("ants_per_block", "warps_per_ant", "ls_warps", "stage_matrix", "ls_ants", "draw_warps", "route_ls",
                 "construct_ctas")
+PARITY_NODES_PER_WARP = 1024  # 32 a thread (include/cvrp_aco.h, warps_per_ant)
 
 
 @dataclasses.dataclass
@@ -70,17 +71,22 @@ class TuneTable:
         return cls([TuneEntry(**e) for e in d["entries"]], d.get("device", ""))
 
     def add(self, e: TuneEntry) -> None:
+        """Add an entry in place of those of its mode, kind and ant count whose
+        node ranges it overlaps (another ladder of sizes splits them elsewhere)."""
         self.entries = [x for x in self.entries
-                        if not (x.mode == e.mode and x.n_lo == e.n_lo and x.n_hi == e.n_hi and x.ants == e.ants)]
+                        if not (x.mode == e.mode and bool(x.batch) == bool(e.batch) and x.ants == e.ants
+                                and x.n_lo <= e.n_hi and e.n_lo <= x.n_hi)]
         self.entries.append(e)
         self.entries.sort(key=lambda x: (x.mode, x.n_lo, x.ants))
 
     def lookup(self, n: int, mode: int, ants: int, batch: bool = False) -> Optional[TuneEntry]:
         """The entry of this mode and kind (batch or single instance) whose node
         range holds n, with the nearest ant count (ratio distance); None when no
-        range holds n."""
+        range holds n.  A parity entry whose warps cannot hold n nodes (1024 a
+        warp) was measured on smaller instances and does not count."""
         hits = [e for e in self.entries
-                if e.mode == mode and bool(e.batch) == batch and e.n_lo <= n <= e.n_hi]
+                if e.mode == mode and bool(e.batch) == batch and e.n_lo <= n <= e.n_hi
+                and not (mode == _lib.MODE_PARITY and 0 < e.warps_per_ant * PARITY_NODES_PER_WARP < n)]
         if not hits:
             return None
         return min(hits, key=lambda e: abs((e.ants / max(ants, 1)) - 1.0))
@@ -187,10 +193,7 @@ def build_batch_entry(seed: int, count: int, n_min: int, n_max: int, ants: int, 
     e = TuneEntry(_lib.MODE_THROUGHPUT, n_min + 1, n_max + 1, ants, out.ants_per_block, out.warps_per_ant,
                   out.ls_warps, out.stage_matrix, ms, nn_ants, out.ls_ants, out.draw_warps, out.route_ls, batch=1,
                   construct_ctas=out.construct_ctas)
-    table.entries = [x for x in table.entries if not (x.batch and x.n_lo == e.n_lo and x.n_hi == e.n_hi
-                                                      and x.ants == e.ants)]
-    table.entries.append(e)
-    table.entries.sort(key=lambda x: (x.mode, x.batch, x.n_lo, x.ants))
+    table.add(e)
     if log:
         log(f"batch of {count} [{e.n_lo},{e.n_hi}] ants={ants}: apc={e.ants_per_block} stage={e.stage_matrix} "
             f"draw={e.draw_warps} route_ls={e.route_ls} ctas={e.construct_ctas} {ms:.3f} ms/iter ({time.perf_counter() - t0:.1f} s)")
