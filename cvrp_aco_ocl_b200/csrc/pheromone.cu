@@ -500,8 +500,11 @@ __device__ __noinline__ void depot_order(const UpdateArgs &a, int mode, float tr
     }
     for (int k = n - 1 + threadIdx.x; k < P; k += blockDim.x) s_key[k] = ~0ull;
     __syncthreads();
-    if ((int)threadIdx.x < a.K) // the depot is rank 0: the table's first row
-        a.chc[threadIdx.x] = __fdiv_rn(1.0f, __uint_as_float(~(uint32_t)(s_key[cid - 1] >> 32)));
+    // the depot is rank 0: the table's first row.  It lists itself, with weight 0, where fewer
+    // than K customers are at a finite distance
+    if ((int)threadIdx.x < a.K)
+        a.chc[threadIdx.x] = cid > 0 ? __fdiv_rn(1.0f, __uint_as_float(~(uint32_t)(s_key[cid - 1] >> 32)))
+                                     : __int_as_float(0x7f800000);
     __syncthreads();
     sort_keys(s_key, P);
     for (int k = threadIdx.x; k < n - 1; k += blockDim.x) a.order[k] = (uint16_t)s_key[k];
