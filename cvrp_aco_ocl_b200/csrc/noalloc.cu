@@ -103,7 +103,9 @@ __global__ void __launch_bounds__(kThreads) noalloc_update_kernel(int n, int ld,
     if (A <= kLens) { // one warp runs the rounds, without block barriers
         if (warp == 0) {
             for (int r = 1; r < R; r++) {
-                uint32_t lo = 0xffffffffu, at = 0xffffffffu;
+                // a lane without ants has no index; one whose lengths all have the largest bits
+                // (a buffer cleared to 0xff) has its first
+                uint32_t lo = 0xffffffffu, at = lane < A ? (uint32_t)lane : 0xffffffffu;
                 for (int k = lane; k < A; k += 32) {
                     const uint32_t b = __float_as_uint(s_len[k]);
                     at = b < lo ? (uint32_t)k : at;
