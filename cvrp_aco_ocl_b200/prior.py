@@ -126,6 +126,8 @@ class GraphBatch:
         n = x.shape[0]
         if n - 2 < k:
             raise ValueError(f"graph degree {k} needs at least {k + 2} nodes, the instance has {n}")
+        if problem.distance is not None and np.shape(problem.distance) != (n, n):
+            raise ValueError(f"distances of shape {np.shape(problem.distance)}, the instance has {n} nodes")
         nf, s = _node_features(problem, x, y)
         dev = torch.device("cuda", device)
         with torch.cuda.device(dev):
