@@ -565,15 +565,16 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
                 for (int i = 0; i < ih.n; i++)
                     if (ih.demand[i] < 0 || ih.demand[i] > 0xFFFF) packable = false;
                 ih.smat = !wide && p.stage_matrix >= 0 && ih.n <= 1024 && packable &&
-                          construct_nn_smem(ih.n, ih.K, ih.Kp, apc, true, true, false, lsw, draw) <= budget;
+                          construct_nn_smem(ih.n, ih.K, ih.Kp, apc, true, true, false, false, lsw, draw) <= budget;
                 ih.packed =
-                    packable && construct_nn_smem(ih.n, ih.K, ih.Kp, apc, ih.smat, true, false, lsw, draw) <= budget;
+                    packable && construct_nn_smem(ih.n, ih.K, ih.Kp, apc, ih.smat, true, false, false, lsw, draw) <= budget;
                 ih.gtab = false;
-                size_t need = construct_nn_smem(ih.n, ih.K, ih.Kp, apc, ih.smat, ih.packed, false, lsw, draw);
+                size_t need = construct_nn_smem(ih.n, ih.K, ih.Kp, apc, ih.smat, ih.packed, false, false, lsw, draw);
                 if (need > budget || (wide && ih.n > 1024)) {
                     ih.gtab = true; // the candidate table stays in global memory (read through L2)
                     ih.packed = packable;
-                    need = construct_nn_smem(ih.n, ih.K, ih.Kp, apc, false, ih.packed, true, lsw, draw);
+                    need = construct_nn_smem(ih.n, ih.K, ih.Kp, apc, false, ih.packed, true, cn_gperm && ih.n > 1024,
+                                             lsw, draw);
                 }
                 if (need > budget) return false;
                 mx = std::max(mx, need);
@@ -608,10 +609,16 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
                 } else if (cn_wide) { // not even one ant fits half an SM: one CTA per SM
                     cn_wide = false;
                     cn_apc = apc0;
+                } else if (!cn_gperm) {
+                    // the largest instances leave the rank -> node table in L2: with it in shared
+                    // memory one ant's CTA ends at 16352 nodes, without it at 19072.  (Everywhere
+                    // above 1024 nodes that costs 2-8% of the construct.)
+                    cn_gperm = true;
                 } else {
-                    return ACO_ERR_INVALID; // candidate table of this size cannot be staged
+                    return ACO_ERR_INVALID; // the tables of one ant cannot be staged
                 }
             }
+            if (cn_gperm) cn_draw = false; // a hint (same results): there is no such kernel with helper warps
         }
         cn_draw = cn_draw && cn_lsw == 0 && cn_apc <= 8; // as the last plan sized the shared memory
         if (cn_draw && p.draw_warps == 0) {
@@ -1085,7 +1092,7 @@ int Colony::construct(bool in_iteration)
     // inside an iteration the 2-opt follows and, with the route list, writes every tour length
     const bool lens_later = in_iteration && routes_pending_ && (p.ls_flag & 1);
     CK(launch_construct_nn(cargs_d_, items_d_, n_items, queue_d_, cn_apc, cn_smem, sm_count, fin_any, st, lsw,
-                           cn_draw, lens_later, cn_wide && lsw == 0));
+                           cn_draw, lens_later, cn_wide && lsw == 0, cn_gperm));
     return ACO_OK;
 }
 

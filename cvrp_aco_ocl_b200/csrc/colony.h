@@ -120,6 +120,7 @@ public:
     bool cp_stage = false;
     int cn_apc = 1, cn_lsw = 0; // throughput construct: ants per CTA, fused 2-opt warps (0 = separate kernel)
     bool cn_draw = false;       // throughput construct: helper warps make the race draws
+    bool cn_gperm = false;      // throughput construct: the rank -> node table of large instances stays in L2
     bool cn_wide = false;       // throughput construct: two CTAs per SM (64 registers, half the shared memory each)
     StatsArgs stats_one_{};     // a single instance's statistics arguments, passed by value
     size_t cn_smem = 0;

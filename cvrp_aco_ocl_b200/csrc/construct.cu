@@ -503,10 +503,11 @@ __host__ __device__ inline size_t perm_bytes(int n) { return ((size_t)n * 2 + 15
 
 // gtab: the candidate table is read from global memory (L2) instead of being
 // staged (instances whose table does not fit next to the per-ant buffers).
+// gperm: the rank -> node table too (the largest instances, gtab only).
 // lsw > 0: the fused 2-opt (lsw improving warps): per ant the edge lengths, and
 // the route queue.
 __host__ __device__ inline NNLayout nn_layout(int n, int K, int Kp, int apc, bool smat, bool packed, bool gtab,
-                                              int lsw = 0, bool draw = false)
+                                              bool gperm, int lsw = 0, bool draw = false)
 {
     const size_t n4 = (size_t)((n + 3) & ~3);
     const size_t words = (size_t)((n + 31) / 32);
@@ -514,7 +515,7 @@ __host__ __device__ inline NNLayout nn_layout(int n, int K, int Kp, int apc, boo
     size_t o = 0;
     L.bar = o; o = al128(o + 16);
     L.dem = o; o = al128(o + n4 * 4);
-    L.perm = o; o = al128(o + perm_bytes(n));
+    L.perm = o; if (!gperm) o = al128(o + perm_bytes(n));
     L.order = o; if (n <= kOrderNodes) o = al128(o + perm_bytes(n));
     L.d0 = o; o = al128(o + n4 * 4);
     L.cand = o; if (!gtab) o = al128(o + (size_t)n * Kp * (packed ? 4 : 2));
@@ -834,16 +835,17 @@ __device__ __noinline__ int fallback_pick(const float *row, const uint16_t *s_pe
 
 // lens_later: the route-level 2-opt follows and writes every listed ant's
 // length, so the construct leaves it out (error paths still write +inf).
-template <bool FIN, bool SMAT, bool PACKED, bool REGVIS, bool GTAB = false, bool LSF = false, bool DRAW = false>
+template <bool FIN, bool SMAT, bool PACKED, bool REGVIS, bool GTAB = false, bool LSF = false, bool DRAW = false,
+          bool GPERM = false>
 __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int apc, int ant0, unsigned char *smem, uint32_t phase,
                                   int lsw = 0, bool lens_later = false)
 {
     const int n = a.n, ld = a.ld, K = a.K, Kp = a.Kp, T = a.T;
     const int n4 = (n + 3) & ~3;
-    const NNLayout L = nn_layout(n, K, Kp, apc, SMAT, PACKED, GTAB, LSF ? lsw : 0, DRAW);
+    const NNLayout L = nn_layout(n, K, Kp, apc, SMAT, PACKED, GTAB, GPERM, LSF ? lsw : 0, DRAW);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L.bar);
     int *s_dem = reinterpret_cast<int *>(smem + L.dem); // by rank
-    uint16_t *s_perm = reinterpret_cast<uint16_t *>(smem + L.perm);
+    const uint16_t *s_perm = GPERM ? a.perm : reinterpret_cast<const uint16_t *>(smem + L.perm);
     uint16_t *s_order = reinterpret_cast<uint16_t *>(smem + L.order); // customers by total_info from the depot
     const bool ordered = REGVIS && a.order != nullptr;
     float *s_d0 = reinterpret_cast<float *>(smem + L.d0);
@@ -860,11 +862,12 @@ __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int ap
 
     const uint32_t cand_bytes = (uint32_t)(n * Kp * (PACKED ? 4 : 2));
     if (threadIdx.x == 0) {
-        uint32_t bytes = (uint32_t)(n4 * 4) + (ordered ? 2u : 1u) * (uint32_t)perm_bytes(n) + (GTAB ? 0u : cand_bytes + (uint32_t)(n * Kp * 4));
+        uint32_t bytes = (uint32_t)(n4 * 4) + ((ordered ? 1u : 0u) + (GPERM ? 0u : 1u)) * (uint32_t)perm_bytes(n) +
+                         (GTAB ? 0u : cand_bytes + (uint32_t)(n * Kp * 4));
         if (SMAT) bytes += (uint32_t)(n * n4 * 4);
         mbar_arrive_expect_tx(bar, bytes);
         tma_bulk_g2s(s_dem, a.demr, n4 * 4, bar);
-        tma_bulk_g2s(s_perm, a.perm, (uint32_t)perm_bytes(n), bar);
+        if (!GPERM) tma_bulk_g2s(smem + L.perm, a.perm, (uint32_t)perm_bytes(n), bar);
         if (ordered) tma_bulk_g2s(s_order, a.order, (uint32_t)perm_bytes(n), bar);
         if (!GTAB) {
             tma_bulk_g2s(smem + L.cand, PACKED ? (const void *)a.cand32 : (const void *)a.nn16, cand_bytes, bar);
@@ -1020,10 +1023,12 @@ __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int ap
             } else {
                 const int at = s_perm[cur];
                 const float *row = SMAT ? s_mat + at * n4 : a.total + (size_t)at * ld, *drow = a.dist + (size_t)at * ld;
-                nxt = DRAW ? best_of_row<FIN, REGVIS>(row, s_perm, s_dem, s_d0, drow, vis, vism, n, words, lane,
-                                                      glast, cap - load, rdist, a.serv_time, a.max_dist)
-                           : fallback_pick<FIN, REGVIS>(row, s_perm, s_dem, s_d0, drow, vis, vism, n, words, lane,
-                                                        glast, cap - load, rdist, a.serv_time, a.max_dist);
+                // (a global s_perm in the shared call would make its reads generic for every caller)
+                nxt = DRAW || GPERM
+                          ? best_of_row<FIN, REGVIS>(row, s_perm, s_dem, s_d0, drow, vis, vism, n, words, lane, glast,
+                                                     cap - load, rdist, a.serv_time, a.max_dist)
+                          : fallback_pick<FIN, REGVIS>(row, s_perm, s_dem, s_d0, drow, vis, vism, n, words, lane, glast,
+                                                       cap - load, rdist, a.serv_time, a.max_dist);
                 if (nxt >= 0) {
                     nd = s_dem[nxt];
                     if (FIN) ed = __ldg(drow + s_perm[nxt]);
@@ -1141,8 +1146,10 @@ __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int ap
 }
 
 // The item without fused 2-opt: candidate table staged or in global memory,
-// register or shared visited set, with or without helper-warp draws.
-template <bool FIN, bool DRAW>
+// register or shared visited set, with or without helper-warp draws.  GPERM: an
+// instance above 1024 nodes whose candidate table is not staged reads the rank ->
+// node table from global memory too.
+template <bool FIN, bool DRAW, bool GPERM>
 __device__ __forceinline__ bool construct_nn_plain(const ConstructArgs &a, int apc, int ant0, unsigned char *smem,
                                                    uint32_t phase, bool ll)
 {
@@ -1150,8 +1157,9 @@ __device__ __forceinline__ bool construct_nn_plain(const ConstructArgs &a, int a
         return a.packed ? construct_nn_item<FIN, false, true, true, true, false, DRAW>(a, apc, ant0, smem, phase, 0, ll)
                         : construct_nn_item<FIN, false, false, true, true, false, DRAW>(a, apc, ant0, smem, phase, 0, ll);
     if (a.gtab)
-        return a.packed ? construct_nn_item<FIN, false, true, false, true, false, DRAW>(a, apc, ant0, smem, phase, 0, ll)
-                        : construct_nn_item<FIN, false, false, false, true, false, DRAW>(a, apc, ant0, smem, phase, 0, ll);
+        return a.packed
+                   ? construct_nn_item<FIN, false, true, false, true, false, DRAW, GPERM>(a, apc, ant0, smem, phase, 0, ll)
+                   : construct_nn_item<FIN, false, false, false, true, false, DRAW, GPERM>(a, apc, ant0, smem, phase, 0, ll);
     if (a.n <= 1024) {
         if (a.smat)
             return a.packed ? construct_nn_item<FIN, true, true, true, false, false, DRAW>(a, apc, ant0, smem, phase, 0, ll)
@@ -1181,7 +1189,7 @@ __device__ __forceinline__ bool construct_nn_wide(const ConstructArgs &a, int ap
 }
 
 // KIND: 0 = plain, 1 = helper-warp draws, 2 = fused 2-opt (lsw improving warps),
-// 3 = plain at two CTAs per SM
+// 3 = plain at two CTAs per SM, 4 = plain with GPERM
 template <bool FIN, int KIND>
 __device__ __forceinline__ void construct_nn_body(const ConstructArgs *args, const int2 *items, int n_items, int *queue,
                                                   int apc, int lsw, bool lens_later)
@@ -1215,7 +1223,7 @@ __device__ __forceinline__ void construct_nn_body(const ConstructArgs *args, con
         } else if (KIND == 3) {
             ok = construct_nn_wide<FIN>(a, apc, ant0, smem, phase, lens_later && a.route_desc != nullptr);
         } else {
-            ok = construct_nn_plain<FIN, KIND == 1>(a, apc, ant0, smem, phase, lens_later && a.route_desc != nullptr);
+            ok = construct_nn_plain<FIN, KIND == 1, KIND == 4>(a, apc, ant0, smem, phase, lens_later && a.route_desc != nullptr);
         }
         if (!ok) break; // uniform: decided by __syncthreads_or
         phase ^= 1u;
@@ -1312,21 +1320,22 @@ size_t construct_parity_smem(int n, int nloc, int kmax, int wpa, int apc, bool s
     return parity_layout(n, nloc, kmax, wpa, apc, stage_total).bytes;
 }
 
-size_t construct_nn_smem(int n, int K, int Kp, int apc, bool stage_total, bool packed, bool global_table, int ls_warps,
-                         bool draw)
+size_t construct_nn_smem(int n, int K, int Kp, int apc, bool stage_total, bool packed, bool global_table,
+                         bool global_perm, int ls_warps, bool draw)
 {
-    return nn_layout(n, K, Kp, apc, stage_total, packed, global_table, ls_warps, draw && ls_warps == 0).bytes;
+    return nn_layout(n, K, Kp, apc, stage_total, packed, global_table, global_perm, ls_warps, draw && ls_warps == 0).bytes;
 }
 
 cudaError_t launch_construct_nn(const ConstructArgs *d_args, const int2 *d_items, int n_items, int *d_queue, int apc,
                                 size_t smem, int sm_count, bool finite_maxd, cudaStream_t st, int ls_warps, bool draw,
-                                bool lens_later, bool wide)
+                                bool lens_later, bool wide, bool gperm)
 {
     if (ls_warps > 0) draw = false;
     if (ls_warps > 0 || draw) wide = false;
     auto kern = ls_warps > 0 ? (finite_maxd ? construct_nn_kernel<true, 2> : construct_nn_kernel<false, 2>)
                 : draw       ? (finite_maxd ? construct_nn_draw_kernel<true> : construct_nn_draw_kernel<false>)
                 : wide       ? (finite_maxd ? construct_nn_wide_kernel<true> : construct_nn_wide_kernel<false>)
+                : gperm      ? (finite_maxd ? construct_nn_kernel<true, 4> : construct_nn_kernel<false, 4>)
                              : (finite_maxd ? construct_nn_kernel<true, 0> : construct_nn_kernel<false, 0>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -174,10 +174,13 @@ cudaError_t launch_construct_parity(const ConstructArgs &a, int warps_per_ant, i
 // the lengths of every ant it gets from the route list; the construct leaves
 // them out for instances that have the list.
 // wide (no helper draws, no fused 2-opt): the 64-register kernel that runs two
-// CTAs per SM; `smem` must then leave room for the second CTA.
+// CTAs per SM; `smem` must then leave room for the second CTA.  gperm (none of
+// these): instances above 1024 nodes whose candidate table is not staged do not
+// stage perm either.
 cudaError_t launch_construct_nn(const ConstructArgs *d_args, const int2 *d_items, int n_items, int *d_queue,
                                 int ants_per_cta, size_t smem, int sm_count, bool finite_maxd, cudaStream_t st,
-                                int ls_warps = 0, bool draw = false, bool lens_later = false, bool wide = false);
+                                int ls_warps = 0, bool draw = false, bool lens_later = false, bool wide = false,
+                                bool gperm = false);
 // 2-opt: one CTA of `warps` warps per ant; d_ant_inst[g] = instance of global ant g,
 // d_ant_base[b] = first global ant of instance b.
 // Route-level 2-opt over the construct's route list (d_ctr: {entries, next,
@@ -216,7 +219,7 @@ size_t construct_parity_smem(int n, int nloc, int kmax, int warps_per_ant, int a
 // draw: a helper warp per ant makes the race draws ahead (ants_per_cta <= 8;
 // ignored with ls_warps > 0)
 size_t construct_nn_smem(int n, int K, int Kp, int ants_per_cta, bool stage_total, bool packed,
-                         bool global_table = false, int ls_warps = 0, bool draw = false);
+                         bool global_table, bool global_perm, int ls_warps, bool draw);
 size_t local_search_smem(int n_max, int ants_per_cta, int warps);
 // resident 2-opt CTAs per SM for this shape (0 = cannot launch)
 int local_search_occupancy(int warps, size_t smem);
