@@ -811,7 +811,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         c.wait_limit = wait_d;
         LocalSearchArgs &l = largs[b];
         l = LocalSearchArgs{};
-        l.n = n; l.ld = ih.ld; l.n_ants = ih.A; l.T = ih.T; l.nn_ls = ih.nn_ls; l.rmax = 32;
+        l.n = n; l.ld = ih.ld; l.n_ants = ih.A; l.T = ih.T; l.nn_ls = ih.nn_ls;
         l.pass_limit = p.ls_pass_limit; l.dist = ih.dist_d; l.nn_list = ih.nnls_d; l.solutions = ih.sol_d;
         l.nnr = ih.nnr_d; l.sym = ih.sym ? 1 : 0; l.generic = ih.finite ? 0 : 1;
         l.best = p.ls_best;

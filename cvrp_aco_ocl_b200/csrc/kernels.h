@@ -88,7 +88,7 @@ struct ConstructArgs {
 };
 
 struct LocalSearchArgs {
-    int n, ld, n_ants, T, nn_ls, rmax, pass_limit;
+    int n, ld, n_ants, T, nn_ls, pass_limit;
     int best;              // 1: best-improvement 2-opt for routes of at most 32 nodes (aco_params.ls_best)
     const float *dist;     // n x ld
     const int *nn_list;    // n x nn_ls

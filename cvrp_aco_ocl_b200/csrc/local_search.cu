@@ -44,7 +44,7 @@ __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~(size_t)15
 // Shared memory: one block per ant of the CTA (sized for the colony's largest
 // instance), then one block per warp.
 struct LsAnt {
-    size_t tour, pos, li, rid, dlb, rstart, dt, bytes;
+    size_t tour, pos, rid, dlb, rstart, dt, bytes;
 };
 
 __host__ __device__ inline LsAnt ls_ant_layout(int n)
@@ -54,7 +54,6 @@ __host__ __device__ inline LsAnt ls_ant_layout(int n)
     size_t o = 0;
     L.tour = o; o = al16(o + (size_t)T * 2);
     L.pos = o; o = al16(o + (size_t)n * 2);
-    L.li = o; o = al16(o + (size_t)n);
     L.rid = o; o = al16(o + (size_t)n * 2);
     L.dlb = o; o = al16(o + (size_t)n);
     L.rstart = o; o = al16(o + (size_t)(n + 1) * 2);
@@ -357,9 +356,7 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
             uint16_t *pos = reinterpret_cast<uint16_t *>(ant_ptr(j, AL.pos));
             uint16_t *rstart = reinterpret_cast<uint16_t *>(ant_ptr(j, AL.rstart));
             uint16_t *rid = reinterpret_cast<uint16_t *>(ant_ptr(j, AL.rid));
-            uint8_t *li = ant_ptr(j, AL.li);
             const int size = s_size[j];
-            int last = 0; // position of the last depot before this chunk
             for (int base = 0; base < size; base += 32) {
                 const int p = base + lane;
                 const int v = p < size ? (int)tour[p] : -1;
@@ -371,14 +368,11 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
                         rstart[count + __popc(lt)] = (uint16_t)p;
                     } else {
                         const int r = count + __popc(lt) - 1;     // depots before p, less the first
-                        const int rb = lt ? base + 31 - __clz(lt) : last; // the depot opening p's route
                         pos[v] = (uint16_t)p;
                         rid[v] = (uint16_t)r;
-                        li[v] = (uint8_t)(p - rb < 256 ? p - rb : 0);
                     }
                 }
                 count += __popc(m);
-                if (m) last = base + 31 - __clz(m);
             }
             count -= 1;
         }
@@ -434,7 +428,6 @@ __global__ void __launch_bounds__(1024) local_search_kernel(const LocalSearchArg
         const LocalSearchArgs a = args[s_inst[j]];
         uint16_t *tour = reinterpret_cast<uint16_t *>(ant_ptr(j, AL.tour));
         uint16_t *pos = reinterpret_cast<uint16_t *>(ant_ptr(j, AL.pos));
-        uint8_t *li = ant_ptr(j, AL.li);
         uint16_t *rid = reinterpret_cast<uint16_t *>(ant_ptr(j, AL.rid));
         uint8_t *dlb = ant_ptr(j, AL.dlb);
         const uint16_t *rstart = reinterpret_cast<const uint16_t *>(ant_ptr(j, AL.rstart));
