@@ -68,6 +68,14 @@ __device__ __forceinline__ uint32_t pm_norm(int x)
     return (uint32_t)r;
 }
 
+// The largest demand that fits: demand <= room exactly when load + demand <= capacity.
+// A negative load (negative demands) under a capacity near 2^31 is not subtracted
+// past the type.
+__device__ __forceinline__ int room_left(int capacity, int load)
+{
+    return min(capacity, 0x7fffffff + min(load, 0)) - load;
+}
+
 template <int WPA, bool FIN, bool SMAT>
 __global__ void __launch_bounds__(512) construct_parity_kernel(ConstructArgs a)
 {
@@ -364,7 +372,7 @@ __global__ void __launch_bounds__(512) construct_parity_regs_kernel(ConstructArg
         // the last edge's length joins here: its load is in flight with the row's
         if (FIN) rdist = ext ? __fadd_rn(rdist, __fadd_rn(pend, a.serv_time)) : 0.f;
         // the next step's draws, under the latency of the loads
-        const int room = a.capacity - load;
+        const int room = room_left(a.capacity, load);
         float rc[JM];
         uint32_t open = 0u;
 #pragma unroll
@@ -1026,9 +1034,9 @@ __device__ __forceinline__ bool construct_nn_item(const ConstructArgs &a, int ap
                 // (a global s_perm in the shared call would make its reads generic for every caller)
                 nxt = DRAW || GPERM
                           ? best_of_row<FIN, REGVIS>(row, s_perm, s_dem, s_d0, drow, vis, vism, n, words, lane, glast,
-                                                     cap - load, rdist, a.serv_time, a.max_dist)
+                                                     room_left(cap, load), rdist, a.serv_time, a.max_dist)
                           : fallback_pick<FIN, REGVIS>(row, s_perm, s_dem, s_d0, drow, vis, vism, n, words, lane, glast,
-                                                       cap - load, rdist, a.serv_time, a.max_dist);
+                                                       room_left(cap, load), rdist, a.serv_time, a.max_dist);
                 if (nxt >= 0) {
                     nd = s_dem[nxt];
                     if (FIN) ed = __ldg(drow + s_perm[nxt]);
