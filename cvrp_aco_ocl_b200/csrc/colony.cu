@@ -521,7 +521,7 @@ int Colony::create(const InstanceSpec *specs, int count, const aco_params &pin)
         if (ih.n <= 128) wpa = 1;
         else if (per_sm > 3) wpa = ih.n <= 256 ? 1 : 2;
         else if (per_sm <= 1 && ih.n > 256) wpa = 8;
-        while (wpa < 8 && 32 * wpa * 16 < ih.n) wpa *= 2; // 16 nodes a thread fit its registers
+        while (wpa < 8 && 32 * wpa * 16 < ih.n) wpa *= 2; // 16 nodes a thread: the register kernel's most
         while (p.ants_per_block > 0 && wpa > 1 && p.ants_per_block * wpa > 16) wpa /= 2;
         wpa = std::min(wpa, ih.nloc / 32);
         if (p.warps_per_ant > 0) wpa = p.warps_per_ant;

@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(512) construct_parity_kernel(ConstructArgs a)
 }
 
 // The same step with everything a thread needs about its nodes in registers, for
-// at most JM (16) nodes a thread; the kernel above is left with longer rows.
+// at most JM (16) nodes a thread; the kernel above takes longer rows.  Register
+// use at 16 nodes a thread: 128, with a route limit 25-31 of its values spilled.
 // What bounds it is the latency of one step, so all that does not depend on the
 // step's row is taken off the chain:
 //   * every node keeps its own draw.  The draws of a lane are consecutive powers

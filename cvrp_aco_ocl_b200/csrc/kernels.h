@@ -181,10 +181,11 @@ cudaError_t launch_construct_nn(const ConstructArgs *d_args, const int2 *d_items
                                 int ants_per_cta, size_t smem, int sm_count, bool finite_maxd, cudaStream_t st,
                                 int ls_warps = 0, bool draw = false, bool lens_later = false, bool wide = false,
                                 bool gperm = false);
-// 2-opt: one CTA of `warps` warps per ant; d_ant_inst[g] = instance of global ant g,
-// d_ant_base[b] = first global ant of instance b.
-// Route-level 2-opt over the construct's route list (d_ctr: {entries, next,
-// CTAs done}, rewound by the kernel); a persistent grid of `warps`-warp CTAs.
+// In the 2-opt kernels d_ant_inst[g] = instance of global ant g, d_ant_base[b] =
+// first global ant of instance b.
+// Route-level 2-opt over the construct's route list (d_ctr: the eight ints of
+// ConstructArgs.route_ctr, rewound by the kernel); a persistent grid of
+// `warps`-warp CTAs.
 size_t route_opt_smem(int n_max, int warps);
 cudaError_t launch_route_opt(const LocalSearchArgs *d_args, const int *d_ant_inst, const int *d_ant_base,
                              const int2 *d_desc, int *d_ctr, int cap, int *d_rem, const uint8_t *d_flagged, int n_max,
@@ -274,8 +275,8 @@ struct PrepArgs {
 };
 // Every instance of a batch in one launch per step (global row g: row g -
 // row_base[b] of instance b = row_inst[g]; global ant g: ant g - ant_base[b] of
-// b = ant_inst[g]): distances and demand ranks, then the lists (the reference's
-// quicksort per row) with the candidate and 2-opt tables, then the lane seeds
+// b = ant_inst[g]): distances and demand ranks, then the lists (in the order of the
+// reference's quicksort) with the candidate and 2-opt tables, then the lane seeds
 // (rnd_seed + b).
 cudaError_t launch_prep_batch(const PrepArgs *d_args, const int *d_row_base, const int *d_row_inst, int total_rows,
                               int n_max, const int *d_ant_base, const int *d_ant_inst, int total_ants, int nloc,

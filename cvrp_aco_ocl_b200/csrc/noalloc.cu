@@ -15,11 +15,11 @@
 // One launch.  A CTA owns a block of matrix rows and finds for itself what its
 // rows receive: it selects the elites from the lengths, walks the elite tours (a
 // few times 2n ints, from L2) and keeps the edges that leave its rows in shared
-// memory, then streams the rows.  Before, one CTA wrote deposit lists for a
-// second launch to read.  What bounds it: the instructions of one CTA's phases
+// memory, then streams the rows.  What bounds it: the instructions of one CTA's phases
 // (37 k a CTA at half the issue slots) and the chain of dependent reads between
 // them (lengths, tour sizes, tours; the rows' first part is loaded ahead); 16 MB at
-// the copy bandwidth would take 2.5 us.  n = 1001, 256 ants: 28.7 -> 12.3 us a call.
+// the copy bandwidth would take 2.5 us.  n = 1001, 256 ants: 12.3 us a call, 28.7 with
+// deposit lists written by one CTA for a second launch.
 //
 // The elite tours come from the caller's buffers, so they are checked before
 // they are used as indices: an elite whose tour size lies outside [2, 2n-1] or

@@ -15,8 +15,8 @@
 // before it have none), it is applied, and the scan resumes there.  Distances
 // of tour edges are kept per position, so a candidate costs four independent
 // reads of the matrix, three rows of it when it is symmetric.  What bounds it is
-// the latency of those reads times the rounds: 302 nodes, 128 ants, 1.01 ms with
-// a warp an ant and eight ants a CTA -> 0.28 ms.
+// the latency of those reads times the rounds: 302 nodes, 128 ants, 0.28 ms (1.01
+// with a warp an ant and eight ants a CTA).
 #include <cuda_runtime.h>
 
 #include <cstdint>
